@@ -221,10 +221,13 @@ int alloc_fields(ib3d_ctx* c) {
   }
   if (cudaMalloc(&c->e32, n3 * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMalloc(&c->r32, n3 * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
-  if (c->d.nx % 2 == 0) {   // colour-packed arrays of the FP32 inner solve (even nx)
-    c->packed_lp = packed_row_length(c->d.nx);
-    const size_t np = (size_t)c->packed_lp * (size_t)c->d.NY2 * (size_t)c->d.NZ2;
-    if (np >= ((size_t)1 << 31)) return IB3D_ERR_TOO_LARGE;   // the sweep kernels use 32-bit offsets
+  // colour-packed arrays of the FP32 inner solve; the sweep kernels use 32-bit offsets, and
+  // an odd nx whose packed rows exceed them (a row of few cells is mostly padding) keeps
+  // the padded layout
+  c->packed_lp = packed_row_length(c->d.nx);
+  const size_t np = (size_t)c->packed_lp * (size_t)c->d.NY2 * (size_t)c->d.NZ2;
+  if (np >= ((size_t)1 << 31) && c->d.nx % 2 == 0) return IB3D_ERR_TOO_LARGE;
+  if (np < ((size_t)1 << 31)) {
     for (int q = 0; q < 2; ++q) {
       if (cudaMalloc(&c->ep[q], np * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
       if (cudaMalloc(&c->rp[q], np * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
@@ -281,7 +284,7 @@ int fail(ib3d_ctx* c, int code, const char* msg) {
 using namespace ib3d;
 
 // FP32 copies of the nine Poisson tables (each padded to 8 floats; off32[3*axis+col]
-// is each table's offset) and, for even nx, the x tables regrouped for the
+// is each table's offset) and the x tables regrouped for the
 // colour-packed sweep: hp[((s*3 + col)*nq + g)*4 + e] = Acx(i-1, col) at
 // i = 2 + s + 8g + 2e (0 beyond the row), columns 1 and 3 (col 0, 2) negated: the
 // sweep subtracts their products with fused multiply-adds, fma(-a, x, num).
@@ -294,24 +297,21 @@ static void poisson32_host(const ib3d_ctx* c, std::vector<float>& h32, std::vect
       for (double x : c->hac[ax][q]) h32.push_back((float)x);
       while (h32.size() % 8) h32.push_back(0.0f);
     }
-  const int nx = c->d.nx;
-  if (nx % 2 == 0) {
-    const int nq = ((nx >> 1) + 3) >> 2;
-    hp.assign((size_t)2 * 3 * nq * 4, 0.0f);
-    for (int s = 0; s < 2; ++s)
-      for (int q = 0; q < 3; ++q)
-        for (int g = 0; g < nq; ++g)
-          for (int e = 0; e < 4; ++e) {
-            const long long i = 2 + s + 8ll * g + 2 * e;
-            if (i <= nx + 1) {
-              const float a = (float)c->hac[0][q][i - 1];
-              hp[(((size_t)s * 3 + q) * nq + g) * 4 + e] = q == 1 ? a : -a;
-            }
+  const int nx = c->d.nx, nq = row_groups(nx);
+  hp.assign((size_t)2 * 3 * nq * 4, 0.0f);
+  for (int s = 0; s < 2; ++s)
+    for (int q = 0; q < 3; ++q)
+      for (int g = 0; g < nq; ++g)
+        for (int e = 0; e < 4; ++e) {
+          const long long i = 2 + s + 8ll * g + 2 * e;
+          if (i <= nx + 1) {
+            const float a = (float)c->hac[0][q][i - 1];
+            hp[(((size_t)s * 3 + q) * nq + g) * 4 + e] = q == 1 ? a : -a;
           }
-    // then the three z coefficients of each plane as one float4 (Grid1D::acz4)
-    for (size_t m = 0; m < c->hac[2][0].size(); ++m)
-      for (int q = 0; q < 4; ++q) hp.push_back(q < 3 ? (float)c->hac[2][q][m] : 0.0f);
-  }
+        }
+  // then the three z coefficients of each plane as one float4 (Grid1D::acz4)
+  for (size_t m = 0; m < c->hac[2][0].size(); ++m)
+    for (int q = 0; q < 4; ++q) hp.push_back(q < 3 ? (float)c->hac[2][q][m] : 0.0f);
 }
 
 static int upload_poisson32(ib3d_ctx* c, const std::vector<float>& h32, const std::vector<float>& hp) {
@@ -390,6 +390,7 @@ int ib3d_create(ib3d_ctx** out, const ib3d_params* prm, int64_t nx, int64_t ny, 
   ib3d_ctx* c = new ib3d_ctx();
   c->prm = *prm;
   cudaGetDevice(&c->device);
+  cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
   c->d.nx = (int)nx; c->d.ny = (int)ny; c->d.nz = (int)nz;
   c->d.NX2 = (int)nx + 2; c->d.NY2 = (int)ny + 2; c->d.NZ2 = (int)nz + 2;
   c->d.n3 = (long long)c->d.NX2 * c->d.NY2 * c->d.NZ2;
@@ -469,7 +470,7 @@ int ib3d_create(ib3d_ctx** out, const ib3d_params* prm, int64_t nx, int64_t ny, 
           *slot = c->d_tables32 + off32[3 * ax + q];
         }
       if (!hp.empty()) {
-        const int nq = (int)(((nx >> 1) + 3) >> 2);
+        const int nq = row_groups((int)nx);
         for (int s = 0; s < 2; ++s)
           for (int q = 0; q < 3; ++q)
             c->g.axp[s][q] = reinterpret_cast<const float4*>(c->d_axp) + ((size_t)s * 3 + q) * nq;

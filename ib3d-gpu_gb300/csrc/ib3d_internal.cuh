@@ -34,6 +34,10 @@ struct Dims {
   }
 };
 
+// float4 groups of one colour's cells in a row of nx cells (the colour-packed layout of
+// k_sor32.cu: (nx+1)/2 entries a row and colour, rounded up to whole groups).
+__host__ __device__ __forceinline__ int row_groups(int nx) { return (((nx + 1) >> 1) + 3) >> 2; }
+
 // 1-D device tables; every pointer is 1-based (element 0 unused) unless noted.
 struct Grid1D {
   const double *x1, *y1, *z1, *dx, *dy, *dz;
@@ -125,6 +129,7 @@ struct ib3d_ctx {
   cudaEvent_t xfer_done[3] = {nullptr, nullptr, nullptr};
   bool async_pending = false;
   int device = 0;
+  int nsm = 148;               // multiprocessors of the device (set at creation)
   std::string err;
 
   // host copies of the 1-D tables (1-based std::vectors)

@@ -480,7 +480,7 @@ int run_sor_fp32dc(ib3d_ctx* c, ib3d_solve_stats* st) {
   const bool fused = P.sweep_kernel == 2;
   const bool packed = P.sweep_kernel != 1 && c->ep[0] != nullptr;
   if (fused) {
-    if (!packed || !fused_sweep_fits(d.nx)) {
+    if (!packed || d.nx % 2 != 0 || !fused_sweep_fits(d.nx)) {
       c->err = "sweep_kernel 2 (fused sweep) needs an even nx whose packed rows fit its blocks (nx <= 512)";
       return IB3D_ERR_ARG;
     }

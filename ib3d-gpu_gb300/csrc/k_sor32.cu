@@ -27,7 +27,7 @@ namespace ib3d {
 
 // Row length of a packed colour array: the row's cells rounded up to whole float4
 // groups, plus 4 entries of left padding (ghost at 3) and 4 of right padding.
-int packed_row_length(int nx) { return 4 * (((nx >> 1) + 3) >> 2) + 8; }
+int packed_row_length(int nx) { return 4 * row_groups(nx) + 8; }
 
 // Two FP32 values in one 64-bit register for the packed FP32 instructions of
 // sm_100 and later (fma/add/mul.rn.f32x2): each lane is rounded as the scalar
@@ -119,7 +119,7 @@ __device__ __forceinline__ void update4(const float (&rv)[4], float (&ev)[4], co
 // earlier, which costs registers (a few spill at the 64-register cap) but keeps more
 // bytes in flight: 5 % faster on arrays larger than L2 (384x256x256: 81.9 against 86.0
 // us per sweep), 6 % slower where they sit in L2 (256x192x192: 24.4 against 23.0), so
-// the launcher picks it by the arrays' size. Both forms give the same bits.
+// sweep_kernel 3 and 4 select between them. Both forms give the same bits.
 constexpr int kPlanes = 8;
 constexpr int kRows = 4;
 
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
   // launched with programmatic dependent launch: the blocks may start while the
   // previous pass drains; wait for it (and its writes) before touching memory
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int nq = ((d.nx >> 1) + 3) >> 2;
+  const int nq = row_groups(d.nx);
   const int lane = threadIdx.x;
   const int q = blockIdx.x * 32 + lane;
   const int j = blockIdx.y * kRows + threadIdx.y + 2;
@@ -190,42 +190,64 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// One colour pass with two rows per thread. A warp owns rows a = j (even) and
-// b = j + 1 over kPlanes2 planes from an even plane k0, so the row phase of each
-// row at each plane is fixed by the colour: row a starts with the updated colour
-// at even planes exactly when COLOR is 1, row b at odd planes. The thread keeps
-// the x coefficients of both phases in registers for all its planes instead of
+// One colour pass with two rows per thread. A lane owns one float4 group of rows a = j
+// (even) and b = j + 1 over P planes (P even) of a slab that starts at an even plane, so
+// the row phase of each row at each plane is fixed by the colour: row a starts with the
+// updated colour at even planes exactly when COLOR is 1, row b at odd planes. The thread
+// keeps the x coefficients of both phases in registers for all its planes instead of
 // loading them per plane, and each row's other-colour centre values serve as the
 // other row's y neighbour, so a plane of two rows loads eight float4 groups
 // (r and e of both rows, the other colour at row a-1, row b+1 and both rows of
-// plane k+1) against ten plus six coefficient groups for two rows of k_sor32p.
-// Row b may be the top ghost row (odd ny): its other-colour values (zero) are
-// read as row a's neighbours, and its own update is neither loaded nor stored.
-// Per cell the arithmetic is update4's, so the bits are those of k_sor32p.
+// the next plane) against ten plus six coefficient groups for two rows of k_sor32p.
+// Lanes run through the groups of all row pairs without a break at a row's end, so no
+// lane idles whatever nx is (a warp per 32 groups of one row left 25 % of the lanes idle
+// at nx = 384 and 41 % at 300: 72.6 against 82.8 us per sweep at 384x256x256); at a row's
+// end the x neighbour is the ghost entry, 0. Row b may be the top ghost row (odd ny): its
+// other-colour values (zero) are read as row a's neighbours, and its own update is
+// neither loaded nor stored. Per cell the arithmetic is update4's, so the bits are those
+// of k_sor32p.
+//
+// STREAM, for arrays that do not fit in L2: the right-hand side, read once a pass and not
+// again until the pass after next, is loaded past L1 and first to leave L2, so that L2
+// keeps the corrections, which every pass reads. DOWN: the slabs and their planes are
+// taken from the top; with the passes alternating in direction each starts on the planes
+// that the last one left in L2. 384x256x256: 72.6 us per sweep without either, 67.7 with
+// the first, 61.4 with both; 256^3 with one wave of blocks 44.2, 36.3 and 33.4.
 constexpr int kRows2 = 4;
-constexpr int kPlanes2 = 8;
-static_assert(kPlanes2 % 2 == 0, "blocks start at even planes");
+constexpr int kUnroll2 = 8;
+static_assert(kUnroll2 % 2 == 0, "the row phases alternate with the planes");
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ld4_stream(const float* p, unsigned long long pol) {
+  float4 v;
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ unsigned long long evict_first_policy() {
+  unsigned long long pol;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  return pol;
+}
 
-template <int COLOR>
+template <int COLOR, bool STREAM, bool DOWN>
 __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, const float* __restrict__ r_own,
-                                                                    float* __restrict__ e_own,
-                                                                    const float* __restrict__ e_oth, int Lp, float omega,
-                                                                    float om1) {
-  const int nq = ((d.nx >> 1) + 3) >> 2;
-  const int lane = threadIdx.x;
-  const int q = blockIdx.x * 32 + lane;
-  const int ja = blockIdx.y * (2 * kRows2) + 2 * threadIdx.y + 2;
-  const int k0 = blockIdx.z * kPlanes2 + 2;
-  const bool live = ja <= d.ny + 1;   // uniform across the warp, so the shuffles see all lanes
-  const bool lds = live && q < nq;
+                                                            float* __restrict__ e_own, const float* __restrict__ e_oth,
+                                                            int Lp, float omega, float om1, int P) {
+  const int nq = row_groups(d.nx);
+  const int lane = threadIdx.x & 31;
+  const unsigned f = blockIdx.x * (32 * kRows2) + threadIdx.x;   // row pair and group, groups fastest
+  const int pair = (int)(f / (unsigned)nq), q = (int)(f - (unsigned)pair * (unsigned)nq);
+  const int ja = 2 * pair + 2;
+  const int k0 = (DOWN ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * P + 2;
+  const unsigned long long pol = STREAM ? evict_first_policy() : 0ull;
+  const bool lds = ja <= d.ny + 1;
   const bool rowb = ja + 1 <= d.ny + 1;
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
   // the coefficient tables are written by the host before the solve, never by a
   // kernel, so they load before the wait for the previous pass
-  const float ya0 = live ? g.acy32[0][ja - 1] : 0.f, ya1 = live ? g.acy32[1][ja - 1] : 0.f,
-              ya2 = live ? g.acy32[2][ja - 1] : 0.f;
+  const float ya0 = lds ? g.acy32[0][ja - 1] : 0.f, ya1 = lds ? g.acy32[1][ja - 1] : 0.f,
+              ya2 = lds ? g.acy32[2][ja - 1] : 0.f;
   const float yb0 = rowb ? g.acy32[0][ja] : 0.f, yb1 = rowb ? g.acy32[1][ja] : 0.f,
               yb2 = rowb ? g.acy32[2][ja] : 0.f;
   // P: the phase of row a at even planes (and of row b at odd ones); Q the other
@@ -234,66 +256,77 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
   const float4 q0 = lds ? g.axp[COLOR][0][q] : z4, q1 = lds ? g.axp[COLOR][1][q] : z4,
                q2 = lds ? g.axp[COLOR][2][q] : z4;
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (live) {
-    const bool load_left = lane == 0, load_right = lane == 31 || q + 1 >= nq;
+  if (__any_sync(0xffffffffu, lds)) {   // every lane of the warp stays for the shuffles
+    const bool load_left = lane == 0, load_right = lane == 31;
+    const bool first = q == 0, last = q + 1 == nq;
     const int plane = (d.ny + 2) * Lp;
     const int sa = (ja - 1) * Lp + 4 * q + 4;
-    float4 oba = lds ? ld4(e_oth + (k0 - 2) * plane + sa) : z4, obb = lds ? ld4(e_oth + (k0 - 2) * plane + sa + Lp) : z4;
-    float4 oxa = lds ? ld4(e_oth + (k0 - 1) * plane + sa) : z4, oxb = lds ? ld4(e_oth + (k0 - 1) * plane + sa + Lp) : z4;
+    // the march runs up from the slab's first plane, or down from its last; oc: the other
+    // colour at the plane, op at the plane before it on the march
+    const int ks = DOWN ? min(k0 + P - 1, d.nz + 1) : k0;
+    const int step = DOWN ? -plane : plane;
+    const int s1 = (ks - 1) * plane + sa;
+    float4 opa = lds ? ld4(e_oth + s1 - step) : z4, opb = lds ? ld4(e_oth + s1 - step + Lp) : z4;
+    float4 oca = lds ? ld4(e_oth + s1) : z4, ocb = lds ? ld4(e_oth + s1 + Lp) : z4;
+    for (int k2 = 0; k2 < P; k2 += kUnroll2)
 #pragma unroll
-    for (int kk = 0; kk < kPlanes2; ++kk) {
-      const int k = k0 + kk;
-      if (k > d.nz + 1) break;
-      const int s0 = (k - 1) * plane + sa;
-      float4 ra = z4, ea = z4, rb = z4, eb = z4, osa = z4, onb = z4, ota = z4, otb = z4;
-      if (lds) {
-        ra = ld4(r_own + s0);
-        ea = ld4(e_own + s0);
-        osa = ld4(e_oth + s0 - Lp);
-        ota = ld4(e_oth + s0 + plane);
-        otb = ld4(e_oth + s0 + Lp + plane);
-        if (rowb) {
-          rb = ld4(r_own + s0 + Lp);
-          eb = ld4(e_own + s0 + Lp);
-          onb = ld4(e_oth + s0 + 2 * Lp);
+      for (int u = 0; u < kUnroll2; ++u) {
+        const int k = DOWN ? k0 + P - 1 - (k2 + u) : k0 + k2 + u;
+        if (k2 + u >= P || (!DOWN && k > d.nz + 1)) break;
+        if (DOWN && k > d.nz + 1) continue;
+        const int s0 = (k - 1) * plane + sa;
+        float4 ra = z4, ea = z4, rb = z4, eb = z4, osa = z4, onb = z4, ona = z4, onn = z4;
+        if (lds) {
+          ra = STREAM ? ld4_stream(r_own + s0, pol) : ld4(r_own + s0);
+          ea = ld4(e_own + s0);
+          osa = ld4(e_oth + s0 - Lp);
+          ona = ld4(e_oth + s0 + step);
+          onn = ld4(e_oth + s0 + Lp + step);
+          if (rowb) {
+            rb = STREAM ? ld4_stream(r_own + s0 + Lp, pol) : ld4(r_own + s0 + Lp);
+            eb = ld4(e_own + s0 + Lp);
+            onb = ld4(e_oth + s0 + 2 * Lp);
+          }
         }
-      }
-      float la = __shfl_up_sync(0xffffffffu, oxa.w, 1), ra_ = __shfl_down_sync(0xffffffffu, oxa.x, 1);
-      float lb = __shfl_up_sync(0xffffffffu, oxb.w, 1), rb_ = __shfl_down_sync(0xffffffffu, oxb.x, 1);
-      if (lds && load_left) {
-        la = e_oth[s0 - 1];
-        lb = e_oth[s0 + Lp - 1];
-      }
-      if (lds && load_right) {
-        ra_ = e_oth[s0 + 4];
-        rb_ = e_oth[s0 + Lp + 4];
-      }
-      const float4 zc = g.acz4[k - 1];
-      const float z0 = zc.x, z1 = zc.y, z2 = zc.z;
-      if (lds) {
-        const float xa[6] = {la, oxa.x, oxa.y, oxa.z, oxa.w, ra_};
-        const float xb[6] = {lb, oxb.x, oxb.y, oxb.z, oxb.w, rb_};
-        const float rva[4] = {ra.x, ra.y, ra.z, ra.w}, rvb[4] = {rb.x, rb.y, rb.z, rb.w};
-        const float sva[4] = {osa.x, osa.y, osa.z, osa.w}, nva[4] = {oxb.x, oxb.y, oxb.z, oxb.w};
-        const float svb[4] = {oxa.x, oxa.y, oxa.z, oxa.w}, nvb[4] = {onb.x, onb.y, onb.z, onb.w};
-        const float bva[4] = {oba.x, oba.y, oba.z, oba.w}, tva[4] = {ota.x, ota.y, ota.z, ota.w};
-        const float bvb[4] = {obb.x, obb.y, obb.z, obb.w}, tvb[4] = {otb.x, otb.y, otb.z, otb.w};
-        float eva[4] = {ea.x, ea.y, ea.z, ea.w}, evb[4] = {eb.x, eb.y, eb.z, eb.w};
-        if ((kk & 1) == 0) {
-          update4<COLOR != 0>(rva, eva, xa, sva, nva, bva, tva, p0, p1, p2, ya0, ya1, ya2, z0, z1, z2, omega, om1);
-          update4<COLOR == 0>(rvb, evb, xb, svb, nvb, bvb, tvb, q0, q1, q2, yb0, yb1, yb2, z0, z1, z2, omega, om1);
-        } else {
-          update4<COLOR == 0>(rva, eva, xa, sva, nva, bva, tva, q0, q1, q2, ya0, ya1, ya2, z0, z1, z2, omega, om1);
-          update4<COLOR != 0>(rvb, evb, xb, svb, nvb, bvb, tvb, p0, p1, p2, yb0, yb1, yb2, z0, z1, z2, omega, om1);
+        float la = __shfl_up_sync(0xffffffffu, oca.w, 1), ra_ = __shfl_down_sync(0xffffffffu, oca.x, 1);
+        float lb = __shfl_up_sync(0xffffffffu, ocb.w, 1), rb_ = __shfl_down_sync(0xffffffffu, ocb.x, 1);
+        if (lds && load_left) {
+          la = e_oth[s0 - 1];
+          lb = e_oth[s0 + Lp - 1];
         }
-        *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
-        if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
+        if (lds && load_right) {
+          ra_ = e_oth[s0 + 4];
+          rb_ = e_oth[s0 + Lp + 4];
+        }
+        if (first) la = lb = 0.f;    // the row's ghost entries; the neighbouring lane is on another row
+        if (last) ra_ = rb_ = 0.f;
+        const float4 zc = g.acz4[k - 1];
+        const float z0 = zc.x, z1 = zc.y, z2 = zc.z;
+        if (lds) {
+          const float4 ba = DOWN ? ona : opa, ta = DOWN ? opa : ona, bb = DOWN ? onn : opb, tb = DOWN ? opb : onn;
+          const float xa[6] = {la, oca.x, oca.y, oca.z, oca.w, ra_};
+          const float xb[6] = {lb, ocb.x, ocb.y, ocb.z, ocb.w, rb_};
+          const float rva[4] = {ra.x, ra.y, ra.z, ra.w}, rvb[4] = {rb.x, rb.y, rb.z, rb.w};
+          const float sva[4] = {osa.x, osa.y, osa.z, osa.w}, nva[4] = {ocb.x, ocb.y, ocb.z, ocb.w};
+          const float svb[4] = {oca.x, oca.y, oca.z, oca.w}, nvb[4] = {onb.x, onb.y, onb.z, onb.w};
+          const float bva[4] = {ba.x, ba.y, ba.z, ba.w}, tva[4] = {ta.x, ta.y, ta.z, ta.w};
+          const float bvb[4] = {bb.x, bb.y, bb.z, bb.w}, tvb[4] = {tb.x, tb.y, tb.z, tb.w};
+          float eva[4] = {ea.x, ea.y, ea.z, ea.w}, evb[4] = {eb.x, eb.y, eb.z, eb.w};
+          if ((u & 1) == (DOWN ? 1 : 0)) {   // an even plane: slabs start at even planes and hold an even number
+            update4<COLOR != 0>(rva, eva, xa, sva, nva, bva, tva, p0, p1, p2, ya0, ya1, ya2, z0, z1, z2, omega, om1);
+            update4<COLOR == 0>(rvb, evb, xb, svb, nvb, bvb, tvb, q0, q1, q2, yb0, yb1, yb2, z0, z1, z2, omega, om1);
+          } else {
+            update4<COLOR == 0>(rva, eva, xa, sva, nva, bva, tva, q0, q1, q2, ya0, ya1, ya2, z0, z1, z2, omega, om1);
+            update4<COLOR != 0>(rvb, evb, xb, svb, nvb, bvb, tvb, p0, p1, p2, yb0, yb1, yb2, z0, z1, z2, omega, om1);
+          }
+          *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
+          if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
+        }
+        opa = oca;
+        oca = ona;
+        opb = ocb;
+        ocb = onn;
       }
-      oba = oxa;
-      oxa = ota;
-      obb = oxb;
-      oxb = otb;
-    }
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -375,7 +408,7 @@ __global__ void __launch_bounds__(640) k_sor32t(Dims d, Grid1D g, const float* _
   extern __shared__ __align__(128) float smf[];   // [S][(4 FY + 8) Lp] stages, then the ring
   __shared__ __align__(8) unsigned long long bar[kMaxStages];
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int nq = ((d.nx >> 1) + 3) >> 2;
+  const int nq = row_groups(d.nx);
   const int nqp = blockDim.x;
   const int q = threadIdx.x, lane = q & 31;
   const int tr = threadIdx.y;                       // 0 and FY + 1: halo rows
@@ -587,7 +620,7 @@ __global__ void k_accumulate_packed(Dims d, double* __restrict__ pc, float* __re
 
 void launch_sor32_packed(ib3d_ctx* c, int color, float omega, float om1) {
   const Dims& d = c->d;
-  const int nq = ((d.nx >> 1) + 3) >> 2;
+  const int nq = row_groups(d.nx);
   const dim3 grid((unsigned)((nq + 31) / 32), (unsigned)((d.ny + kRows - 1) / kRows),
                   (unsigned)((d.nz + kPlanes - 1) / kPlanes)),
       block(32, kRows);
@@ -606,7 +639,7 @@ void launch_sor32_packed(ib3d_ctx* c, int color, float omega, float om1) {
   const float* r = c->rp[color];
   float* e = c->ep[color];
   const float* o = c->ep[1 - color];
-  // the loads without branches (sweep_kernel 0 beyond L2, and 3) or behind branches (4)
+  // the loads without branches (sweep_kernel 3) or behind branches (4)
   if (c->prm.sweep_kernel != 4) {
     if (color == 0) cudaLaunchKernelEx(&cfg, k_sor32p<0, true>, d, c->g, r, e, o, c->packed_lp, omega, om1);
     else cudaLaunchKernelEx(&cfg, k_sor32p<1, true>, d, c->g, r, e, o, c->packed_lp, omega, om1);
@@ -616,26 +649,37 @@ void launch_sor32_packed(ib3d_ctx* c, int color, float omega, float om1) {
   }
 }
 
-// Where the four packed arrays fit in L2 with room to spare, one colour pass per
-// launch of the two-row kernel; beyond 96 MB the one-row kernel with branch-free
-// loads, which keeps more DRAM requests in flight (at 384x256x256, 213 MB: 79.7 us
-// per sweep against 82.5-85.2 for the two-row kernel; at 256^3, 145 MB, the two are
-// within 2 %).
-constexpr size_t kTwoRowMaxBytes = (size_t)96 << 20;
-static bool two_row_kernel(const ib3d_ctx* c) {
-  const Dims& d = c->d;
-  const size_t packed = 4 * sizeof(float) * (size_t)c->packed_lp * (size_t)d.NY2 * (size_t)d.NZ2;
-  return c->prm.sweep_kernel == 0 && packed <= kTwoRowMaxBytes;
+// Where the four packed arrays exceed 96 MB, L2 no longer holds them with what else a pass
+// touches, and the passes stream the right-hand side and alternate in direction: at
+// 272x192x192 (85 MB) that costs 14 % (22.1 against 19.3 us per sweep), at 288x208x208
+// (106 MB) it gains 5 % (31.7 against 33.4), at 256^3 (145 MB) 18 %.
+constexpr size_t kResidentMaxBytes = (size_t)96 << 20;
+
+// Planes per slab: the fewest that let every block of the pass run at once (four per SM),
+// because a second, partly filled wave costs a whole one (us per sweep at 272x192x192: 8
+// planes 24.6, 10 planes 19.3; at 200x160x160: 4 planes 14.2, 6 planes 11.2, 8 planes 13.4;
+// at 256^3: 8 planes 36.8, 14 planes 33.5), and a thread's planes run one after the other.
+// Beyond 24 planes the slabs of one wave get so long that several waves of 8 planes are
+// as good or better (400x320x300: 96.7 against 106).
+static int slab_planes(const ib3d_ctx* c, unsigned bx) {
+  const unsigned slots = 4u * (unsigned)c->nsm;
+  const int nz = c->d.nz;
+  if (bx == 0 || bx > slots) return 8;
+  int P = (nz + (int)(slots / bx) - 1) / (int)(slots / bx);
+  P += P & 1;
+  return P <= 24 ? std::max(P, 2) : 8;
 }
 
 // One colour pass of the two-row kernel.
 static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1) {
   const Dims& d = c->d;
-  const int nq = ((d.nx >> 1) + 3) >> 2;
+  const unsigned groups = (unsigned)row_groups(d.nx) * (unsigned)((d.ny + 1) >> 1);
+  const unsigned bx = (groups + 32 * kRows2 - 1) / (32 * kRows2);
+  const int P = slab_planes(c, bx);
+  const size_t packed = 4 * sizeof(float) * (size_t)c->packed_lp * (size_t)d.NY2 * (size_t)d.NZ2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((nq + 31) / 32), (unsigned)((d.ny + 2 * kRows2 - 1) / (2 * kRows2)),
-                     (unsigned)((d.nz + kPlanes2 - 1) / kPlanes2));
-  cfg.blockDim = dim3(32, kRows2);
+  cfg.gridDim = dim3(bx, (unsigned)((d.nz + P - 1) / P));
+  cfg.blockDim = dim3(32 * kRows2);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = c->st;
   cudaLaunchAttribute attr[1];
@@ -646,13 +690,19 @@ static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1) {
   const float* r = c->rp[color];
   float* e = c->ep[color];
   const float* o = c->ep[1 - color];
-  if (color == 0) cudaLaunchKernelEx(&cfg, k_sor32p2<0>, d, c->g, r, e, o, c->packed_lp, omega, om1);
-  else cudaLaunchKernelEx(&cfg, k_sor32p2<1>, d, c->g, r, e, o, c->packed_lp, omega, om1);
+  const int Lp = c->packed_lp;
+  if (packed > kResidentMaxBytes) {
+    if (color == 0) cudaLaunchKernelEx(&cfg, k_sor32p2<0, true, false>, d, c->g, r, e, o, Lp, omega, om1, P);
+    else cudaLaunchKernelEx(&cfg, k_sor32p2<1, true, true>, d, c->g, r, e, o, Lp, omega, om1, P);
+  } else {
+    if (color == 0) cudaLaunchKernelEx(&cfg, k_sor32p2<0, false, false>, d, c->g, r, e, o, Lp, omega, om1, P);
+    else cudaLaunchKernelEx(&cfg, k_sor32p2<1, false, false>, d, c->g, r, e, o, Lp, omega, om1, P);
+  }
 }
 
 // One red-black sweep with the colour-packed two-pass kernels.
 void launch_sor32_sweep(ib3d_ctx* c, float omega, float om1) {
-  if (two_row_kernel(c)) {
+  if (c->prm.sweep_kernel == 0) {
     launch_pass2(c, 0, omega, om1);
     launch_pass2(c, 1, omega, om1);
   } else {
@@ -723,7 +773,7 @@ static size_t staged_smem(int fy, int S, int Lp, int wx) {
   return (size_t)S * (4 * fy + 8) * Lp * sizeof(float) + (size_t)3 * (fy + 2) * 32 * wx * sizeof(float4);
 }
 static bool staged_shape(int nx, StagedShape& out) {
-  const int nq = ((nx >> 1) + 3) >> 2, wx = (nq + 31) / 32, Lp = packed_row_length(nx);
+  const int nq = row_groups(nx), wx = (nq + 31) / 32, Lp = packed_row_length(nx);
   const size_t cap = 227 * 1024 - 256;   // shared memory per block, less the static barriers
   // one block per SM with the deepest staging that fits: tried at 256x192x192, two
   // blocks of 8 rows and 4 stages per SM ran 35.6 us per sweep against 28.5 us for one
