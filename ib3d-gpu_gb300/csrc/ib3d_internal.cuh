@@ -109,6 +109,16 @@ struct ForceSched {
   int nfinal;
 };
 
+// How a grid's rows are split over the blocks of a resident kernel: gy x gz blocks of at
+// most by x bz rows (full x extent), nt threads (zl: FP32, planes a thread marches
+// through; ni: FP64, cells of a colour per thread), smem bytes of shared memory, and the
+// exchange buffer's size in 64-bit words. ok is false where the grid does not fit.
+struct ResidentPlan {
+  bool ok = false;
+  int gy = 0, gz = 0, by = 0, bz = 0, nt = 0, zl = 0, ni = 0;
+  size_t smem = 0, xch_words = 0;
+};
+
 }  // namespace ib3d
 
 struct ib3d_net;
@@ -168,6 +178,14 @@ struct ib3d_ctx {
   int sweep_kern = -1;
   bool sweep_graph_failed = false;   // capture refused once: the sweeps launch one by one
   int packed_lp = 0;
+  // on-chip sweeps (k_resident.cu): the split of this grid, planned on first use, the
+  // exchange buffer between blocks (both forms use it, one launch at a time), and the
+  // passes run on it so far
+  ib3d::ResidentPlan res32;
+  bool res32_planned = false;
+  unsigned long long* xch = nullptr;
+  size_t xch_words = 0;
+  unsigned xch_seq = 0;
   unsigned char* cell = nullptr;
   int* ibmap = nullptr;
   ib3d::SolveCtl* ctl = nullptr;
@@ -264,6 +282,8 @@ void run_sor32_sweeps(ib3d_ctx* c, int n, float omega, float om1);
 void launch_accumulate_packed(ib3d_ctx* c);
 void launch_sor32_fused(ib3d_ctx* c, float omega, float om1);
 bool fused_sweep_fits(int nx);
+// k_resident.cu
+bool run_resident32(ib3d_ctx* c, int n, int nsmooth, int nramp, double wi, float om, float om1);
 // k_ib.cu
 int run_surface_norm(ib3d_ctx* c);
 int run_search(ib3d_ctx* c);

@@ -507,7 +507,7 @@ int run_sor_fp32dc(ib3d_ctx* c, ib3d_solve_stats* st) {
     rc = read_ctl(c);
     if (rc) return rc;
     if (c->h_ctl->stage_err) {
-      c->err = "fused FP32 sweep: a shared-memory stage never arrived (bounded wait gave up)";
+      c->err = "FP32 sweep: a bounded wait gave up (a shared-memory stage or a neighbouring block's rows never arrived)";
       return IB3D_ERR_CUDA;
     }
     const double res = c->h_ctl->last_res;
@@ -534,7 +534,17 @@ int run_sor_fp32dc(ib3d_ctx* c, ib3d_solve_stats* st) {
     if (sweeps + batch > P.max_sweeps) batch = (int)std::max(1ll, P.max_sweeps - sweeps);
     prev_batch = batch;
     prev_res = res;
-    {
+    // grids that fit run the whole pass in one launch, the correction on chip
+    bool on_chip = false;
+    if (P.sweep_kernel == 0 && packed) {
+      PhaseScope ps(c, PH_SOR32);
+      on_chip = run_resident32(c, batch, outer == 0 ? P.smooth_sweeps : 0, outer == 0 ? P.ramp_sweeps : 0, wi, om, om1);
+      if (on_chip) {
+        c->launches += 1;
+        c->t_launches32 += 1;
+      }
+    }
+    if (!on_chip) {
       PhaseScope ps(c, PH_SOR32);
       c->launches += fused ? batch : 2 * batch;
       c->t_launches32 += fused ? batch : 2 * batch;
@@ -563,7 +573,7 @@ int run_sor_fp32dc(ib3d_ctx* c, ib3d_solve_stats* st) {
       }
       if (direct < batch) run_sor32_sweeps(c, batch - direct, om, om1);
     }
-    {
+    if (!on_chip) {
       PhaseScope ps(c, PH_RESIDUAL);
       c->launches += 1;
       if (packed) launch_accumulate_packed(c);

@@ -24,10 +24,12 @@ def _capped(ib3d, grids, shape, sweeps, b, **kw):
     return st["sweeps"], pc
 
 
-# odd nx (the second colour's rows end in the ghost cell), odd ny (a row pair's second row is
+# sizes whose sweeps run on chip (blocks split both ways, along one axis, with several planes
+# a thread) and beyond; odd nx (the second colour's rows end in the ghost cell), odd ny (a row pair's second row is
 # the ghost row), nz no multiple of a slab; the last two exceed what the blocks hold on chip,
 # and the last one streams its right-hand side and alternates the direction of its passes
-@pytest.mark.parametrize("kernel,shape", [(0, (129, 21, 19)), (0, (37, 18, 45)), (0, (5, 4, 4)), (3, (129, 21, 19)),
+@pytest.mark.parametrize("kernel,shape", [(0, (129, 21, 19)), (0, (37, 18, 45)), (0, (5, 4, 4)), (0, (7, 5, 301)),
+                                          (0, (9, 203, 6)), (0, (126, 130, 97)), (3, (129, 21, 19)),
                                           (4, (67, 9, 11)), (0, (1201, 41, 78)), (0, (271, 225, 202))])
 def test_packed_sweeps_match_the_padded_layout(ib3d, grids, kernel, shape):
     b = np.zeros(tuple(n + 2 for n in shape), order="F")
