@@ -13,11 +13,14 @@
 //
 // The solve is the library's mixed-precision pressure solve: FP64 defect
 // correction around FP32 red-black sweeps, stopped at an FP64 residual L-inf
-// tolerance, with the same arithmetic as ib3d_poisson_solver's IB3D_PREC_FP32DC
-// mode (two-launch sweep form).
+// tolerance, with the same arithmetic as ib3d_poisson_solver's IB3D_PREC_FP32DC mode.
+// Grids that the on-chip sweeps take (k_resident.cu: all but those of very long rows) run
+// each pass in one launch from FP32 tables of the caller's coefficients; before, every
+// sweep was two launches that converted nine FP64 coefficients per cell: 14.4 us a sweep
+// at 96x64x64 against 2.9.
 #include <mutex>
 
-#include "ib3d_internal.cuh"
+#include "resident.cuh"
 
 namespace ib3d {
 namespace {
@@ -27,7 +30,10 @@ namespace {
 constexpr long long kMaxCells = 1ll << 21;
 constexpr size_t kArrayBytes = (size_t)kMaxCells * sizeof(float);
 constexpr size_t kCtlOffset = 2 * kArrayBytes;
-constexpr size_t kScratchBytes = kCtlOffset + 256;
+// FP32 coefficient tables of the on-chip form, behind the control block
+constexpr size_t kTabOffset = kCtlOffset + 256;
+constexpr size_t kTabBytes = 128 * 1024;
+constexpr size_t kScratchBytes = kTabOffset + kTabBytes;
 
 // The scratch itself. Every GPU that loads the library holds it until the process
 // exits. In host code this name is only a host-side stand-in for the device
@@ -90,10 +96,12 @@ __device__ __forceinline__ void decide(SolveCtl* ctl, long long sweeps, double e
   }
 }
 
-// r = b/dt - A pc on fluid cells (FP64), its maximum, and r rounded to FP32.
+// r = b/dt - A pc on fluid cells (FP64), its maximum, and r rounded to FP32: in the padded
+// layout (r32, 0 off the fluid cells), or colour-packed without padding rows (rp: [2][nz][ny]
+// rows of 4 row_groups(nx) entries, NaN off the fluid cells).
 __global__ void k_na_residual(Dims d, Coefs A, const double* __restrict__ b, double deltat,
                               const double* __restrict__ pc, const unsigned char* __restrict__ cell,
-                              float* __restrict__ r32, SolveCtl* ctl, long long sweeps, double eps,
+                              float* __restrict__ r32, float* __restrict__ rp, SolveCtl* ctl, long long sweeps, double eps,
                               long long max_sweeps) {
   const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
   double m = 0.0;
@@ -102,7 +110,7 @@ __global__ void k_na_residual(Dims d, Coefs A, const double* __restrict__ b, dou
     const unsigned t = tid / (unsigned)d.nx;
     const int j = (int)(t % (unsigned)d.ny) + 2, k = (int)(t / (unsigned)d.ny) + 2;
     const long long idx = d.at(i, j, k);
-    float rr = 0.0f;
+    float rr = rp ? __int_as_float(0x7fc00000) : 0.0f;
     if (cell[idx] == 0) {
       const long long sy = d.NX2, sz = (long long)d.NX2 * d.NY2;
       const double bdt = b[idx] / deltat;
@@ -114,10 +122,37 @@ __global__ void k_na_residual(Dims d, Coefs A, const double* __restrict__ b, dou
       m = fabs(r);
       rr = (float)r;
     }
-    r32[idx] = rr;
+    if (rp) {
+      const int L = 4 * row_groups(d.nx);
+      const size_t half = (size_t)d.nz * d.ny * L;
+      rp[(((i + j + k) & 1) ? 0 : half) + ((size_t)(k - 2) * d.ny + (j - 2)) * L + ((i - 2) >> 1)] = rr;
+    } else {
+      r32[idx] = rr;
+    }
   }
   block_max_atomic(m, &ctl->res);
   decide(ctl, sweeps, eps, max_sweeps);
+}
+
+// The FP32 tables of the on-chip sweeps: the x coefficients grouped by four cells of one
+// colour (Grid1D::axp: columns 1 and 3 negated, 0 beyond the row), then the y and the z
+// columns, 1-based.
+__global__ void k_na_tables(Coefs A, float* __restrict__ tab) {
+  const int nq = row_groups(A.nx), nx4 = 24 * nq, ny3 = 3 * (A.ny + 1), nz3 = 3 * (A.nz + 1);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nx4 + ny3 + nz3; t += gridDim.x * blockDim.x) {
+    float v = 0.f;
+    if (t < nx4) {
+      const int s = t / (12 * nq), c = (t / (4 * nq)) % 3, m = t % (4 * nq), i = 2 + s + 2 * m;
+      if (i <= A.nx + 1) v = (float)A.x(c, i - 1) * (c == 1 ? 1.f : -1.f);
+    } else if (t < nx4 + ny3) {
+      const int c = (t - nx4) / (A.ny + 1), m = (t - nx4) % (A.ny + 1);
+      if (m >= 1) v = (float)A.y(c, m);
+    } else {
+      const int c = (t - nx4 - ny3) / (A.nz + 1), m = (t - nx4 - ny3) % (A.nz + 1);
+      if (m >= 1) v = (float)A.z(c, m);
+    }
+    tab[t] = v;
+  }
 }
 
 // One colour of the FP32 red-black sweep on A e = r, in place.
@@ -157,8 +192,26 @@ __global__ void k_na_accumulate(long long n3, double* __restrict__ pc, float* __
   }
 }
 
+// The on-chip form's exchange buffer follows its right-hand side (two halves).
+size_t exchange_offset(size_t half) { return (2 * half * sizeof(float) + 255) / 256 * 256; }
 
-int run_noalloc(int64_t nx, int64_t ny, int64_t nz, const double* acx, const double* acy, const double* acz,
+// The split of the on-chip sweeps where the grid, the exchange buffer and the tables fit.
+bool plan_noalloc(int64_t nx, int64_t ny, int64_t nz, ResidentPlan& plan) {
+  int dev = 0, nsm = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+    return false;
+  const size_t nq = (size_t)row_groups((int)nx);
+  if ((24 * nq + 3 * (size_t)(ny + 1) + 3 * (size_t)(nz + 1)) * sizeof(float) > kTabBytes) return false;
+  plan = plan_resident32((int)nx, (int)ny, (int)nz, nsm);
+  return plan.ok && exchange_offset((size_t)ny * nz * 4 * nq) + plan.xch_words * 8 <= kCtlOffset;
+}
+
+constexpr int kNotResident = 1;   // the cooperative launch was refused before anything ran
+
+// plan: the split of the on-chip sweeps, or null for one launch per colour pass.
+int run_noalloc(const ResidentPlan* plan, int64_t nx, int64_t ny, int64_t nz, const double* acx, const double* acy, const double* acz,
                 const unsigned char* cell, const double* b, double deltat, double* pc, double omega, double eps,
                 int64_t max_sweeps, int32_t inner_sweeps, cudaStream_t st, unsigned char* base,
                 int64_t* sweeps_out, double* residual_out) {
@@ -173,8 +226,35 @@ int run_noalloc(int64_t nx, int64_t ny, int64_t nz, const double* acx, const dou
   const Coefs A{acx, acy, acz, d.nx, d.ny, d.nz};
   // the scratch keeps the previous call's contents: the correction must start at
   // zero and the control block must be cleared
-  if (cudaMemsetAsync(e32, 0, (size_t)n3 * sizeof(float), st) != cudaSuccess) return IB3D_ERR_CUDA;
+  if (!plan && cudaMemsetAsync(e32, 0, (size_t)n3 * sizeof(float), st) != cudaSuccess) return IB3D_ERR_CUDA;
   if (cudaMemsetAsync(ctl, 0, sizeof(SolveCtl), st) != cudaSuccess) return IB3D_ERR_CUDA;
+  Resident32 res{};
+  if (plan) {
+    const int nq = row_groups(d.nx);
+    const size_t rows = (size_t)ny * nz, half = rows * 4 * nq;
+    float* tab = reinterpret_cast<float*>(base + kTabOffset);
+    for (int s = 0; s < 2; ++s)
+      for (int c = 0; c < 3; ++c) res.axp[s][c] = reinterpret_cast<const float4*>(tab) + (3 * s + c) * nq;
+    for (int c = 0; c < 3; ++c) {
+      res.ay[c] = tab + 24 * nq + c * (ny + 1);
+      res.az[c] = tab + 24 * nq + 3 * (ny + 1) + c * (nz + 1);
+    }
+    res.d = d;
+    res.r[0] = r32;
+    res.r[1] = r32 + half;
+    res.rs = 4 * nq;
+    res.ps = d.ny * 4 * nq;
+    res.pc = pc;
+    res.xch = reinterpret_cast<unsigned long long*>(base + exchange_offset(half));
+    res.nsweeps = inner_sweeps;
+    res.om = (float)omega;
+    res.om1 = (float)(1.0 - omega);
+    res.err = &ctl->stage_err;
+    // the rows' entries past their last cell stay NaN; the pass numbers start over
+    if (cudaMemsetAsync(r32, 0xff, 2 * half * sizeof(float), st) != cudaSuccess) return IB3D_ERR_CUDA;
+    if (cudaMemsetAsync(res.xch, 0, plan->xch_words * 8, st) != cudaSuccess) return IB3D_ERR_CUDA;
+    k_na_tables<<<16, kBlock, 0, st>>>(A, tab);
+  }
   const long long ncell = (long long)nx * ny * nz;
   const unsigned gres = (unsigned)((ncell + kBlock - 1) / kBlock);
   const unsigned gcol = (unsigned)((((nx + 1) / 2) * ny * nz + kBlock - 1) / kBlock);
@@ -183,11 +263,22 @@ int run_noalloc(int64_t nx, int64_t ny, int64_t nz, const double* acx, const dou
   SolveCtl h{};
   long long sweeps = 0;
   for (;;) {
-    k_na_residual<<<gres, kBlock, 0, st>>>(d, A, b, deltat, pc, cell, r32, ctl, sweeps, eps, max_sweeps);
+    k_na_residual<<<gres, kBlock, 0, st>>>(d, A, b, deltat, pc, cell, r32, plan ? r32 : nullptr, ctl, sweeps,
+                                              eps, max_sweeps);
     if (cudaGetLastError() != cudaSuccess) return IB3D_ERR_CUDA;
     if (cudaMemcpyAsync(&h, ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, st) != cudaSuccess) return IB3D_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return IB3D_ERR_CUDA;
+    if (h.stage_err) return IB3D_ERR_CUDA;   // a bounded wait of the on-chip sweeps gave up
     if (h.done) break;
+    if (plan) {
+      if (launch_resident32(*plan, res, st) != cudaSuccess) {
+        cudaGetLastError();
+        return sweeps == 0 ? kNotResident : IB3D_ERR_CUDA;
+      }
+      res.seq0 += 2u * (unsigned)inner_sweeps;
+      sweeps += inner_sweeps;
+      continue;
+    }
     for (int q = 0; q < inner_sweeps; ++q) {
       k_na_sor32<0><<<gcol, kBlock, 0, st>>>(d, A, r32, e32, cell, om, om1);
       k_na_sor32<1><<<gcol, kBlock, 0, st>>>(d, A, r32, e32, cell, om, om1);
@@ -223,8 +314,15 @@ extern "C" int ib3d_pressure_solve_noalloc(int64_t nx, int64_t ny, int64_t nz, c
     forget_scratch_address();
     return IB3D_ERR_CUDA;
   }
-  const int rc = run_noalloc(nx, ny, nz, acx, acy, acz, cell, b, deltat, pc, omega, eps, max_sweeps, inner_sweeps,
-                             static_cast<cudaStream_t>(stream), base, sweeps_out, residual_out);
+  ResidentPlan plan;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int rc = kNotResident;
+  if (plan_noalloc(nx, ny, nz, plan))
+    rc = run_noalloc(&plan, nx, ny, nz, acx, acy, acz, cell, b, deltat, pc, omega, eps, max_sweeps, inner_sweeps, st,
+                     base, sweeps_out, residual_out);
+  if (rc == kNotResident)
+    rc = run_noalloc(nullptr, nx, ny, nz, acx, acy, acz, cell, b, deltat, pc, omega, eps, max_sweeps, inner_sweeps, st,
+                     base, sweeps_out, residual_out);
   if (rc == IB3D_ERR_CUDA) forget_scratch_address();
   return rc;
 }

@@ -47,3 +47,59 @@ def test_fused_sweep_still_needs_an_even_nx(ib3d, grids):
     with pytest.raises(ib3d.IB3DError) as e:
         _capped(ib3d, grids, (21, 8, 8), 10, b, sweep_kernel=2)
     assert e.value.code == ib3d.ERR_ARG
+
+
+def _rhs(shape, seed=5):
+    b = np.zeros(tuple(n + 2 for n in shape), order="F")
+    b[1:-1, 1:-1, 1:-1] = np.random.default_rng(seed).standard_normal(shape)
+    return b
+
+
+def test_noalloc_solve_on_rows_too_long_for_a_block(ib3d, grids, oracle_mod):
+    """Launch per colour pass, capped, against the context's one-array kernel on the same sweeps
+    (the two round b/dt - A pc differently)."""
+    import torch
+    shape = (4200, 9, 7)
+    b = _rhs(shape)
+    n, want = _capped(ib3d, grids, shape, 48, b, sweep_kernel=1, inner_sweeps=24)
+    o = oracle_mod.Oracle(*(grids.tanh_axis(n) for n in shape), 100.0, 1.0)
+    dev = lambda v: torch.from_numpy(np.ascontiguousarray(v.ravel(order="F"))).cuda()
+    A, bd, cd = [dev(np.asarray(o.acoef(q))) for q in range(3)], dev(b), dev(np.zeros(b.shape, np.uint8))
+    pc = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+    rc = ib3d.lib().ib3d_pressure_solve_noalloc(*shape, *(v.data_ptr() for v in A), cd.data_ptr(), bd.data_ptr(), 1.0,
+                                                pc.data_ptr(), 1.85, 1e-30, 48, 24, None, None, None)
+    assert (rc, n) == (ib3d.ERR_NOCONV, 48)
+    got = pc.cpu().numpy().reshape(b.shape, order="F")
+    assert np.max(np.abs(got - want)) <= 1e-6 * np.max(np.abs(want))
+
+
+# even and odd rows of the on-chip sweeps
+@pytest.mark.parametrize("shape", [(21, 10, 13), (64, 33, 31)])
+def test_noalloc_solve_meets_the_residual(ib3d, grids, oracle_mod, shape):
+    import ctypes as C
+    import torch
+    x, y, z = (grids.tanh_axis(n) for n in shape)
+    o = oracle_mod.Oracle(x, y, z, 100.0, 1.0)
+    a = [np.asfortranarray(o.acoef(q)) for q in range(3)]
+    b = _rhs(shape)
+    cell = np.zeros(b.shape, np.uint8, order="F")
+    cell[shape[0] // 3:shape[0] // 3 + 3, 3:5, 3:5] = 1
+    dev = lambda v: torch.from_numpy(np.ascontiguousarray(v.ravel(order="F"))).cuda()
+    A, bd, cd = [dev(v) for v in a], dev(b), dev(cell)
+    pc = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+    sweeps, res = np.zeros(1, np.int64), np.zeros(1)
+    rc = ib3d.lib().ib3d_pressure_solve_noalloc(
+        *shape, A[0].data_ptr(), A[1].data_ptr(), A[2].data_ptr(), cd.data_ptr(), bd.data_ptr(), 1.0, pc.data_ptr(), 1.6,
+        1e-6, 2000000, 24, None, sweeps.ctypes.data_as(C.POINTER(C.c_int64)), res.ctypes.data_as(C.POINTER(C.c_double)))
+    assert rc == ib3d.OK and res[0] < 1e-6 and sweeps[0] % 24 == 0
+    q = pc.cpu().numpy().reshape(b.shape, order="F")
+    i = np.s_[1:-1]
+    Ap = (a[0][:, 0][:, None, None] * q[:-2, i, i] + a[0][:, 2][:, None, None] * q[2:, i, i]
+          + a[1][:, 0][None, :, None] * q[i, :-2, i] + a[1][:, 2][None, :, None] * q[i, 2:, i]
+          + a[2][:, 0][None, None, :] * q[i, i, :-2] + a[2][:, 2][None, None, :] * q[i, i, 2:]
+          + (a[0][:, 1][:, None, None] + a[1][:, 1][None, :, None] + a[2][:, 1][None, None, :]) * q[i, i, i])
+    fluid = cell[i, i, i] == 0
+    # the kernel's own residual and this one differ by the rounding of their sums
+    scale = np.abs(a[0]).max() + np.abs(a[1]).max() + np.abs(a[2]).max()
+    assert np.max(np.abs(b[i, i, i] - Ap)[fluid]) < 1e-6 + 1e-14 * scale * np.max(np.abs(q))
+    assert np.all(q[cell != 0] == 0.0)
