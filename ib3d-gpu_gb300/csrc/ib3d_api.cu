@@ -512,10 +512,11 @@ void ib3d_destroy(ib3d_ctx* c) {
                   c->e32, c->r32, c->ep[0], c->ep[1], c->rp[0], c->rp[1], c->cell, c->ibmap, c->ctl, c->d_nodes, c->d_tri, c->d_surf, c->d_iblist,
                   c->d_nelp, c->d_nd, c->d_minel, c->d_scache, c->d_contrib, c->d_coef, c->d_flag, c->d_scan,
                   c->hist[0], c->hist[1], c->r_hist, c->d_norm, c->d_norm_part, c->resi[0], c->resi[1], c->resi[2],
-                  c->wdiag, c->xch, c->epn[0], c->epn[1], c->d_retag_mask, c->d_retag_list};
+                  c->wdiag, c->xch, c->pc2, c->d_errs, c->epn[0], c->epn[1], c->d_retag_mask, c->d_retag_list};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_ctl) cudaFreeHost(c->h_ctl);
+  if (c->h_errs) cudaFreeHost(c->h_errs);
   if (c->sweep_exec) cudaGraphExecDestroy(c->sweep_exec);
   for (cudaStream_t x : c->xfer)
     if (x) {

@@ -111,11 +111,11 @@ struct ForceSched {
 
 // How a grid's rows are split over the blocks of a resident kernel: gy x gz blocks of at
 // most by x bz rows (full x extent), nt threads (zl: FP32, planes a thread marches
-// through; ni: FP64, cells of a colour per thread), smem bytes of shared memory, and the
+// through), smem bytes of shared memory, and the
 // exchange buffer's size in 64-bit words. ok is false where the grid does not fit.
 struct ResidentPlan {
   bool ok = false;
-  int gy = 0, gz = 0, by = 0, bz = 0, nt = 0, zl = 0, ni = 0;
+  int gy = 0, gz = 0, by = 0, bz = 0, nt = 0, zl = 0;
   size_t smem = 0, xch_words = 0;
 };
 
@@ -183,6 +183,10 @@ struct ib3d_ctx {
   // passes run on it so far
   ib3d::ResidentPlan res32;
   bool res32_planned = false;
+  ib3d::ResidentPlan res64, res64f;   // FP64 sweeps, reference arithmetic and fast form
+  bool res64_planned = false, res64f_planned = false;
+  double* pc2 = nullptr;              // the other array of the FP64 batches
+  unsigned long long *d_errs = nullptr, *h_errs = nullptr;   // their per-sweep stopping measures
   unsigned long long* xch = nullptr;
   size_t xch_words = 0;
   unsigned xch_seq = 0;
@@ -284,6 +288,7 @@ void launch_sor32_fused(ib3d_ctx* c, float omega, float om1);
 bool fused_sweep_fits(int nx);
 // k_resident.cu
 bool run_resident32(ib3d_ctx* c, int n, int nsmooth, int nramp, double wi, float om, float om1);
+bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc);
 // k_ib.cu
 int run_surface_norm(ib3d_ctx* c);
 int run_search(ib3d_ctx* c);

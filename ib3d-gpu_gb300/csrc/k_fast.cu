@@ -323,6 +323,10 @@ int run_sor_fp64_fast(ib3d_ctx* c, ib3d_solve_stats* st) {
   const long long ncell = (long long)d.nx * d.ny * d.nz;
   const bool resid = P.criterion == IB3D_CRIT_RESIDUAL;
   const int every = P.check_every < 1 ? 1 : P.check_every;
+  {
+    int rc = IB3D_OK;
+    if (run_resident64(c, st, false, rc)) return rc;   // grids that fit run on chip
+  }
   if (!c->wdiag) IB3D_CUDA(c, cudaMalloc(&c->wdiag, (size_t)d.n3 * sizeof(double)));
   c->launches += 1;
   k_wdiag<<<nblk(d.n3), kBlock, 0, c->st>>>(d, c->g, c->cell, P.omega, c->wdiag);

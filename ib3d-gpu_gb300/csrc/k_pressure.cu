@@ -431,6 +431,7 @@ int run_sor_fp64(ib3d_ctx* c, ib3d_solve_stats* st) {
   const int every = P.check_every < 1 ? 1 : P.check_every;
   int rc = reset_ctl(c);
   if (rc) return rc;
+  if (run_resident64(c, st, true, rc)) return rc;   // grids that fit run on chip, same bits
   long long sweep = 0;
   long long batch = 4;
   for (;;) {

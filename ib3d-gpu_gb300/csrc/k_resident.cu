@@ -25,6 +25,8 @@
 //
 // Compiled with -fmad=false: the FP64 kernel keeps the reference's rounding.
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 
 #include "resident.cuh"
 #include "sor32_update.cuh"
@@ -52,6 +54,22 @@ __device__ __forceinline__ int ld_flag(const int* p) {
   return v;
 }
 __device__ __forceinline__ float4 ld4s(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// a / b, correctly rounded, for a divisor known in advance: zh = 1/b rounded, zl the rest
+// of 1/b. a (zh + zl) is within half an ulp and 2^-100 of the quotient, so its remainder
+// is exact and one more fused step rounds correctly (Markstein, IBM J. Res. Dev. 34, 1990;
+// known divisors: Brisebarre, Muller and Raina, IEEE Trans. Comput. 53, 2004). Numerators
+// so small or large that a step could leave the normal range, zeros, infinities and NaN
+// take the division itself; |b| lies within 2^+-200 (plain_diagonal).
+__device__ __forceinline__ double div_known(double a, double b, double zh, double zl) {
+  const unsigned ex = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
+  if (ex - 323u < 1400u) {
+    const double q = fma(a, zh, a * zl);
+    return fma(fma(-b, q, a), zh, q);
+  }
+  return a / b;
+}
+
 __device__ __forceinline__ u64 tagged(unsigned bits, unsigned seq) { return ((u64)seq << 32) | bits; }
 
 // The rows of this block: [j0, j0 + nyb) x [k0, k0 + nzb).
@@ -296,6 +314,225 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident32(Resident32 A) {
     }
 }
 
+// FP64 sweeps of the plain path (REDBLACKSOR, subPcorVcor.f90:148-212), one cell of a
+// colour per item; both colours' pc of the block's rows, the ghost rows and the x ghost
+// cells in shared memory, and b/dt and what the division needs per cell beside them (in
+// registers they spilled).
+//
+// EXACT: the reference's arithmetic. The kernel is bound by the FP64 pipe (1.65 operations
+// per clock and SM), and the division by the diagonal was the largest single item of
+// k_sor64 (about 8.6 of its 27 operations a cell). The diagonal of a cell never changes
+// within a solve, so the division runs as four fused operations from its precomputed
+// reciprocal (div_known) with the same rounded quotient.
+// Otherwise the fast plain form (IB3D_PREC_FP64_FAST), k_sor64_fast's operations.
+//
+// check == 0: every sweep's largest |pc_new - pc_old| goes to errs[sweep]; else every
+// check-th sweep's largest |b/dt - A pc| (k_residual64's or k_residual_fast's operations).
+// The host applies the stopping test afterwards and, when it stops inside the batch, runs
+// the batch again from its unchanged input up to the stopping sweep.
+template <bool EXACT>
+__global__ void __launch_bounds__(kMaxThreads, 1) k_resident64(Resident64 A) {
+  extern __shared__ __align__(16) double smd[];
+  const Dims& d = A.d;
+  const int nh = (d.nx + 1) >> 1, Ld = nh + 2;         // entry m of a row at m + 1, m = -1 .. nh
+  const int plane = (A.by + 2) * Ld, all = (A.bz + 2) * plane, allB = A.by * A.bz * nh;
+  const Span s = block_span(d, A.gy, A.gz);
+  const int nt = blockDim.x, t = threadIdx.x;
+  double* E = smd;                    // [2][all]
+  double* B = E + 2 * all;            // [2][allB]
+  double* X = B + 2 * allB;           // [3][nx + 1]
+  double* Y = X + 3 * (d.nx + 1);     // [3][by]
+  double* Z = Y + 3 * A.by;           // [3][bz]
+  double* zh = Z + 3 * A.bz;          // [2][allB] EXACT: the diagonal's reciprocal, else omega / diagonal
+  double* zl = zh + 2 * allB;         // [2][allB] EXACT: the rest of the reciprocal
+  double* dg = zl + 2 * allB;         // [2][allB] EXACT: the diagonal
+  // per item: kk << 22 | jj << 12 | m, and bits 30 + c where its cell of colour c is fluid
+  unsigned* pos = reinterpret_cast<unsigned*>(EXACT ? dg + 2 * allB : zl);
+  for (int e = t; e < 3 * d.nx; e += nt) X[(e / d.nx) * (d.nx + 1) + e % d.nx + 1] = A.ax[e / d.nx][e % d.nx + 1];
+  for (int e = t; e < 3 * s.nyb; e += nt) Y[(e / s.nyb) * A.by + e % s.nyb] = A.ay[e / s.nyb][s.j0 + e % s.nyb - 1];
+  for (int e = t; e < 3 * s.nzb; e += nt) Z[(e / s.nzb) * A.bz + e % s.nzb] = A.az[e / s.nzb][s.k0 + e % s.nzb - 1];
+  // pc of the rows j0-1 .. j0+nyb, planes k0-1 .. k0+nzb, ghost cells included
+  const int rows = (s.nyb + 2) * (s.nzb + 2);
+  for (int e = t; e < rows * d.NX2; e += nt) {
+    const int row = e / d.NX2, i = e - row * d.NX2 + 1, kk = row / (s.nyb + 2) - 1, jj = row % (s.nyb + 2) - 1;
+    const int j = s.j0 + jj, k = s.k0 + kk;
+    const int c = ((i + j + k) & 1) ? 0 : 1;
+    const int m = (i & 1) ? (i - 3) / 2 : (i - 2) / 2;   // rows start with even i in one colour, odd i in the other
+    E[c * all + (kk + 1) * plane + (jj + 1) * Ld + m + 1] = A.pc_in[d.at(i, j, k)];
+  }
+  const int items = s.nyb * s.nzb * nh;
+  const int ER = 2 * (A.by + A.bz), cstride = ER * 2 * nh;   // a value takes two words
+  u64* mine = A.xch + (size_t)blockIdx.x * 2 * cstride;
+  for (int it = t; it < items; it += nt) {
+    const int row = it / nh, m = it - row * nh, kk = row / s.nyb, jj = row - kk * s.nyb;
+    const int j = s.j0 + jj, k = s.k0 + kk;
+    unsigned p = (unsigned)(kk << 22 | jj << 12 | m);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int i = ((c == 0) == (((j + k) & 1) == 1) ? 2 : 3) + 2 * m;
+      if (i > d.nx + 1) continue;
+      const long long o = d.at(i, j, k);
+      if (A.cell[o] != 0) continue;
+      const int q = c * allB + it;
+      B[q] = A.bdt[o];
+      const double diag = A.ax[1][i - 1] + A.ay[1][j - 1] + A.az[1][k - 1];
+      const double r = (EXACT ? 1.0 : A.omega) / diag;
+      zh[q] = r;
+      if (EXACT) {
+        dg[q] = diag;
+        zl[q] = fma(-r, diag, 1.0) / diag;
+      }
+      if (EXACT || r != 0.0) p |= 1u << (30 + c);
+    }
+    pos[it] = p;
+  }
+  const u64* hsrc[kHalo];
+  int hdst[kHalo];
+  const int ghosts = 2 * (s.nyb + s.nzb) * nh;
+#pragma unroll
+  for (int n = 0; n < kHalo; ++n) {
+    hdst[n] = -1;
+    hsrc[n] = nullptr;
+    const int h = nt - 1 - t + n * nt;
+    if (h < ghosts) {
+      const int row = h / nh, m = h - row * nh;
+      int kk, jj, nb, er;
+      if (ghost_row(s, A.gy, A.gz, A.by, A.bz, row, kk, jj, nb, er)) {
+        hdst[n] = (kk + 1) * plane + (jj + 1) * Ld + m + 1;
+        hsrc[n] = A.xch + (size_t)nb * 2 * cstride + (size_t)(er * nh + m) * 2;
+      }
+    }
+  }
+  __syncthreads();
+  bool fail = false;
+  u64 big = 0;                                         // largest update of the sweep
+  for (int sweep = 0; sweep < A.nsweeps; ++sweep) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const double* Eo = E + (1 - c) * all;
+      double* Ec = E + c * all;
+      const unsigned seq = A.seq0 + 2u * (unsigned)sweep + (unsigned)c + 1u;
+      for (int it = t; it < items; it += nt) {
+        const unsigned ps = pos[it];
+        const int m = ps & 4095u, jj = ps >> 12 & 1023u, kk = ps >> 22 & 255u;
+        const int off = (kk + 1) * plane + (jj + 1) * Ld + m + 1;
+        const bool first = (c == 0) == (((s.j0 + jj + s.k0 + kk) & 1) == 1);
+        double nw = Ec[off];
+        if (ps >> (30 + c) & 1) {
+          const double* o = Eo + off;
+          const int i = (first ? 2 : 3) + 2 * m, q = c * allB + it;
+          const double old = nw, bd = B[q];
+          const double W = first ? o[-1] : o[0], Ea = first ? o[0] : o[1];
+          const double a0 = X[i - 1], a2 = X[2 * (d.nx + 1) + i - 1];
+          const double y0 = Y[jj], y2 = Y[2 * A.by + jj], z0 = Z[kk], z2 = Z[2 * A.bz + kk];
+          if (EXACT) {
+            const double num = bd - a0 * W - a2 * Ea - y0 * o[-Ld] - y2 * o[Ld] - z0 * o[-plane] - z2 * o[plane];
+            const double gs = div_known(num, dg[q], zh[q], zl[q]);
+            nw = A.om1 * old + A.omega * gs;
+          } else {
+            double num = fma(-a0, W, bd);
+            num = fma(-a2, Ea, num);
+            num = fma(-y0, o[-Ld], num);
+            num = fma(-y2, o[Ld], num);
+            num = fma(-z0, o[-plane], num);
+            num = fma(-z2, o[plane], num);
+            nw = fma(zh[q], num, A.om1 * old);
+          }
+          Ec[off] = nw;
+          if (A.check == 0) {
+            const u64 b = (u64)__double_as_longlong(fabs(nw - old));
+            big = b > big ? b : big;
+          }
+        }
+        const int ye = jj == 0 && s.jb > 0 ? edge_ylo(kk) : jj == s.nyb - 1 && s.jb + 1 < A.gy ? edge_yhi(A.bz, kk) : -1;
+        const int ze = kk == 0 && s.kb > 0 ? edge_zlo(A.bz, jj)
+                       : kk == s.nzb - 1 && s.kb + 1 < A.gz ? edge_zhi(A.by, A.bz, jj) : -1;
+        if (ye >= 0 || ze >= 0) {
+          const u64 v = (u64)__double_as_longlong(nw);
+          const u64 lo = tagged((unsigned)v, seq), hi = tagged((unsigned)(v >> 32), seq);
+          if (ye >= 0) st_pair(mine + c * cstride + (ye * nh + m) * 2, lo, hi);
+          if (ze >= 0) st_pair(mine + c * cstride + (ze * nh + m) * 2, lo, hi);
+        }
+      }
+      if (c == 1 && A.check == 0) {
+        big = warp_max_bits(big);
+        if ((t & 31) == 0 && big != 0) atomicMax(A.errs + sweep, big);
+        big = 0;
+      }
+      unsigned pend = 0;
+#pragma unroll
+      for (int n = 0; n < kHalo; ++n) pend |= hdst[n] >= 0 ? 1u << n : 0u;
+      for (int it = 0; pend != 0; ++it) {
+        u64 v[kHalo][2];
+#pragma unroll
+        for (int n = 0; n < kHalo; ++n)
+          if (pend >> n & 1) ld_pair(hsrc[n] + c * cstride, v[n][0], v[n][1]);
+#pragma unroll
+        for (int n = 0; n < kHalo; ++n)
+          if ((pend >> n & 1) && (unsigned)(v[n][0] >> 32) == seq && (unsigned)(v[n][1] >> 32) == seq) {
+            Ec[hdst[n]] = __longlong_as_double((long long)((v[n][1] << 32) | (v[n][0] & 0xffffffffull)));
+            pend &= ~(1u << n);
+          }
+        if (pend != 0 && (it & 255) == 255 && (it > kPollLimit || ld_flag(A.err) != 0)) {
+          fail = true;
+          break;
+        }
+      }
+      if (__syncthreads_or(fail)) {
+        if (t == 0) atomicExch(A.err, 1);
+        return;
+      }
+    }
+    if (A.check > 0 && (A.sweep0 + sweep + 1) % A.check == 0) {
+      u64 res = 0;
+      for (int it = t; it < items; it += nt) {
+        const unsigned ps = pos[it];
+        const int m = ps & 4095u, jj = ps >> 12 & 1023u, kk = ps >> 22 & 255u;
+        const int off = (kk + 1) * plane + (jj + 1) * Ld + m + 1;
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          if (ps >> (30 + c) & 1) {
+            const double* o = E + (1 - c) * all + off;
+            const bool first = (c == 0) == (((s.j0 + jj + s.k0 + kk) & 1) == 1);
+            const int i = (first ? 2 : 3) + 2 * m;
+            const double bd = B[c * allB + it], own = E[c * all + off];
+            const double W = first ? o[-1] : o[0], Ea = first ? o[0] : o[1];
+            const double a0 = X[i - 1], a2 = X[2 * (d.nx + 1) + i - 1];
+            const double y0 = Y[jj], y2 = Y[2 * A.by + jj], z0 = Z[kk], z2 = Z[2 * A.bz + kk];
+            double r;
+            if (EXACT) {
+              const double num = bd - a0 * W - a2 * Ea - y0 * o[-Ld] - y2 * o[Ld] - z0 * o[-plane] - z2 * o[plane];
+              r = num - dg[c * allB + it] * own;
+            } else {
+              double q = a0 * W;
+              q = fma(a2, Ea, q);
+              q = fma(y0, o[-Ld], q);
+              q = fma(y2, o[Ld], q);
+              q = fma(z0, o[-plane], q);
+              q = fma(z2, o[plane], q);
+              q = fma(X[d.nx + 1 + i - 1] + Y[A.by + jj] + Z[A.bz + kk], own, q);
+              r = bd - q;
+            }
+            const u64 b = (u64)__double_as_longlong(fabs(r));
+            res = b > res ? b : res;
+          }
+      }
+      res = warp_max_bits(res);
+      if ((t & 31) == 0 && res != 0) atomicMax(A.errs + sweep, res);
+    }
+  }
+  for (int it = t; it < items; it += nt) {
+    const unsigned ps = pos[it];
+    const int m = ps & 4095u, jj = ps >> 12 & 1023u, kk = ps >> 22 & 255u, j = s.j0 + jj, k = s.k0 + kk;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (ps >> (30 + c) & 1) {
+        const int i = ((c == 0) == (((j + k) & 1) == 1) ? 2 : 3) + 2 * m;
+        A.pc_out[d.at(i, j, k)] = E[c * all + (kk + 1) * plane + (jj + 1) * Ld + m + 1];
+      }
+  }
+}
+
 // -------------------------------------------------------------------------- plans
 
 namespace {
@@ -353,6 +590,42 @@ cudaError_t launch_resident32(const ResidentPlan& pl, Resident32 a, cudaStream_t
   a.gy = pl.gy; a.gz = pl.gz; a.by = pl.by; a.bz = pl.bz; a.zl = pl.zl;
   const int nh = (2 * (pl.by + pl.bz) * row_groups(a.d.nx) + pl.nt - 1) / pl.nt;
   return nh <= 1 ? go32<1>(pl, a, st) : nh <= 2 ? go32<2>(pl, a, st) : go32<kHalo>(pl, a, st);
+}
+
+// The split for the FP64 form: bound by the FP64 pipe, so the busiest block's rows count
+// first, then its edge rows.
+ResidentPlan plan_resident64(int nx, int ny, int nz, int nsm, bool exact) {
+  ResidentPlan pl;
+  const int nh = (nx + 1) >> 1;
+  double best = 1e300;
+  for (int gy = 1; gy <= std::min(ny / 2, nsm); ++gy)
+    for (int gz = 1; gz <= std::min(nz / 2, nsm / gy); ++gz) {
+      const int by = (ny + gy - 1) / gy, bz = (nz + gz - 1) / gz;
+      const double cost = (double)by * bz + 0.15 * ((gy > 1 ? 2 * bz : 0) + (gz > 1 ? 2 * by : 0));
+      if (cost < best) {
+        best = cost;
+        pl.gy = gy; pl.gz = gz; pl.by = by; pl.bz = bz;
+      }
+    }
+  if (pl.gy == 0 || nh > 4095 || pl.by > 1023 || pl.bz > 255) return pl;
+  const int items = pl.by * pl.bz * nh, ghosts = 2 * (pl.by + pl.bz) * nh;
+  pl.nt = std::min(kMaxThreads, (items + 31) / 32 * 32);
+  while (pl.nt < kMaxThreads && kHalo * pl.nt < ghosts) pl.nt += 32;
+  const size_t all = (size_t)(pl.bz + 2) * (pl.by + 2) * (nh + 2);
+  pl.smem = (2 * all + (exact ? 8 : 4) * (size_t)items + 3 * (size_t)(nx + 1) + 3 * (size_t)(pl.by + pl.bz)) * sizeof(double) +
+            (size_t)items * sizeof(unsigned);
+  pl.xch_words = (size_t)pl.gy * pl.gz * 2 * 2 * (pl.by + pl.bz) * 2 * nh;
+  pl.ok = kHalo * pl.nt >= ghosts && pl.smem <= kSmemCap;
+  return pl;
+}
+
+cudaError_t launch_resident64(const ResidentPlan& pl, Resident64 a, bool exact, cudaStream_t st) {
+  a.gy = pl.gy; a.gz = pl.gz; a.by = pl.by; a.bz = pl.bz;
+  const void* k = exact ? (const void*)k_resident64<true> : (const void*)k_resident64<false>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&a};
+  return cudaLaunchCooperativeKernel(k, dim3((unsigned)(pl.gy * pl.gz)), dim3((unsigned)pl.nt), args, pl.smem, st);
 }
 
 // The exchange buffer of a context, at least `words` long, zeroed when it is new (pass
@@ -416,6 +689,150 @@ bool run_resident32(ib3d_ctx* c, int n, int nsmooth, int nramp, double wi, float
     return false;
   }
   c->xch_seq += 2u * (unsigned)n;
+  return true;
+}
+
+// Is the diagonal of every cell of one sign and of a size that div_known takes?
+static bool plain_diagonal(const ib3d_ctx* c) {
+  const int n[3] = {c->d.nx, c->d.ny, c->d.nz};
+  double lo = 0.0, hi = 0.0;
+  for (int ax = 0; ax < 3; ++ax) {
+    double l = 1e300, h = 0.0;
+    for (int i = 1; i <= n[ax]; ++i) {
+      const double v = -c->hac[ax][1][i];
+      if (!(v > 0.0)) return false;
+      l = std::min(l, v);
+      h = std::max(h, v);
+    }
+    lo += l;
+    hi += h;
+  }
+  return lo > 0x1p-200 && hi < 0x1p200;
+}
+
+// A whole FP64 solve (REDBLACKSOR) in batches of on-chip sweeps: k_sor64's arithmetic, or
+// k_sor64_fast's. Returns false (and nothing done) where the grid does not fit; rc is the
+// solve's result otherwise. Each batch goes from one array to the other, so a batch in
+// which the stopping test is met runs again from its input up to that sweep; the batches
+// grow to 256 sweeps and shrink as the measured rate says that the end is near.
+bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc) {
+  constexpr int kBatch = 256;
+  ResidentPlan& pl = exact ? c->res64 : c->res64f;
+  bool& planned = exact ? c->res64_planned : c->res64f_planned;
+  if (!planned) {
+    planned = true;
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+    if (coop) pl = plan_resident64(c->d.nx, c->d.ny, c->d.nz, c->nsm, exact);
+    const size_t bytes = (size_t)c->d.n3 * sizeof(double);
+    if (pl.ok && !ensure_exchange(c, pl.xch_words)) pl.ok = false;
+    if (pl.ok && !c->pc2 &&
+        (cudaMalloc(&c->pc2, bytes) != cudaSuccess || cudaMalloc(&c->d_errs, (kBatch + 1) * sizeof(u64)) != cudaSuccess ||
+         cudaMallocHost(&c->h_errs, (kBatch + 1) * sizeof(u64)) != cudaSuccess)) {
+      cudaGetLastError();
+      pl.ok = false;
+    }
+  }
+  if (!pl.ok || (exact && !plain_diagonal(c))) return false;
+  const ib3d_params& P = c->prm;
+  const size_t bytes = (size_t)c->d.n3 * sizeof(double);
+  const bool resid = P.criterion == IB3D_CRIT_RESIDUAL;
+  const int every = P.check_every < 1 ? 1 : P.check_every;
+  Resident64 a{};
+  a.d = c->d;
+  for (int q = 0; q < 3; ++q) {
+    a.ax[q] = c->g.acx[q];
+    a.ay[q] = c->g.acy[q];
+    a.az[q] = c->g.acz[q];
+  }
+  a.bdt = c->bdt;
+  a.cell = c->cell;
+  a.xch = c->xch;
+  a.check = resid ? every : 0;
+  a.omega = P.omega;
+  a.om1 = 1.0 - P.omega;
+  a.errs = c->d_errs;
+  a.err = reinterpret_cast<int*>(c->d_errs + kBatch);
+  rc = IB3D_ERR_CUDA;
+  auto failed = [&](const char* what) {
+    c->err = what;
+    rc = IB3D_ERR_CUDA;
+    return true;
+  };
+  double *in = c->pc, *out = c->pc2;
+  if (cudaMemcpyAsync(c->pc2, c->pc, bytes, cudaMemcpyDeviceToDevice, c->st) != cudaSuccess) return failed("FP64 sweeps: copy of pc");
+  long long sweep = 0, launched = 0;
+  int batch = 16, done = 0;
+  double err = 0.0, last_res = 0.0, rate_err = 0.0;   // rate_err: the stopping measure at rate_at sweeps
+  long long rate_at = 0;
+  bool have_rate = false;
+  while (!done) {
+    PhaseScope ps(c, PH_SOR64);
+    int n = (int)std::min<long long>(batch, P.max_sweeps - sweep);
+    a.pc_in = in;
+    a.pc_out = out;
+    a.sweep0 = sweep;
+    a.nsweeps = n;
+    a.seq0 = c->xch_seq;
+    if (cudaMemsetAsync(c->d_errs, 0, (kBatch + 1) * sizeof(u64), c->st) != cudaSuccess) return failed("FP64 sweeps: control words");
+    const cudaError_t le = launch_resident64(pl, a, exact, c->st);
+    if (le != cudaSuccess) {
+      cudaGetLastError();
+      pl.ok = false;
+      if (launched == 0) return false;
+      return failed("FP64 sweeps: cooperative launch refused");
+    }
+    ++launched;
+    c->launches += 1;
+    c->xch_seq += 2u * (unsigned)n;
+    if (cudaMemcpyAsync(c->h_errs, c->d_errs, (kBatch + 1) * sizeof(u64), cudaMemcpyDeviceToHost, c->st) != cudaSuccess ||
+        cudaStreamSynchronize(c->st) != cudaSuccess)
+      return failed("FP64 sweeps: reading the convergence words");
+    if ((int)c->h_errs[kBatch] != 0) return failed("FP64 sweeps: a neighbouring block's rows never arrived (bounded wait gave up)");
+    int stop = 0;   // sweeps of this batch up to the decision
+    for (int q = 1; q <= n && !done; ++q) {
+      const long long at = sweep + q;
+      const bool tested = !resid || at % every == 0;
+      if (tested) {
+        std::memcpy(&err, &c->h_errs[q - 1], sizeof(double));
+        last_res = err;
+        if (!(err >= P.eps)) done = 1;
+      } else {
+        err = last_res;
+      }
+      if (!done && at >= P.max_sweeps) done = 2;
+      stop = q;
+    }
+    if (done == 1 && stop < n) {   // the test was met inside the batch: up to that sweep, from the same input
+      a.nsweeps = stop;
+      a.seq0 = c->xch_seq;
+      if (launch_resident64(pl, a, exact, c->st) != cudaSuccess) return failed("FP64 sweeps: cooperative launch refused");
+      c->launches += 1;
+      c->xch_seq += 2u * (unsigned)stop;
+      if (cudaMemcpyAsync(c->h_errs, c->d_errs, (kBatch + 1) * sizeof(u64), cudaMemcpyDeviceToHost, c->st) != cudaSuccess ||
+          cudaStreamSynchronize(c->st) != cudaSuccess || (int)c->h_errs[kBatch] != 0)
+        return failed("FP64 sweeps: a neighbouring block's rows never arrived (bounded wait gave up)");
+    }
+    sweep += stop;
+    std::swap(in, out);
+    batch = std::min(2 * batch, kBatch);
+    if (!done && last_res > 0.0) {   // sweeps that the rate since the last batch still asks for
+      if (have_rate && last_res < rate_err) {
+        const double need = std::log(P.eps / last_res) / (std::log(last_res / rate_err) / (double)(sweep - rate_at));
+        batch = std::max(16, (int)std::min((double)batch, 0.9 * need));
+      }
+      rate_err = last_res;
+      rate_at = sweep;
+      have_rate = true;
+    }
+  }
+  if (in != c->pc && cudaMemcpyAsync(c->pc, in, bytes, cudaMemcpyDeviceToDevice, c->st) != cudaSuccess)
+    return failed("FP64 sweeps: copy of pc");
+  st->sweeps = sweep;
+  st->outer = 0;
+  c->t_sweeps64 += sweep;
+  st->final_err = err;
+  rc = err != err ? IB3D_ERR_NONFINITE : done == 2 ? IB3D_ERR_NOCONV : IB3D_OK;
   return true;
 }
 

@@ -26,4 +26,24 @@ struct Resident32 {
 };
 cudaError_t launch_resident32(const ResidentPlan& pl, Resident32 a, cudaStream_t st);
 
+// One launch of FP64 sweeps on A pc = b/dt, from pc_in to pc_out (padded layout; pc_out's
+// cells that are not fluid are left alone).
+struct Resident64 {
+  Dims d;
+  const double *ax[3], *ay[3], *az[3];  // Poisson coefficients, 1-based by i-1, j-1, k-1
+  const double* bdt;
+  const double* pc_in;
+  double* pc_out;
+  const unsigned char* cell;
+  unsigned long long* xch;
+  unsigned seq0;
+  int gy, gz, by, bz;
+  int nsweeps, check;                   // check: sweeps between residuals, 0: update norm of every sweep
+  long long sweep0;                     // sweeps of the solve before this launch
+  double omega, om1;
+  unsigned long long* errs;             // [nsweeps] largest update or residual (bit pattern)
+  int* err;
+};
+cudaError_t launch_resident64(const ResidentPlan& pl, Resident64 a, bool exact, cudaStream_t st);
+
 }  // namespace ib3d

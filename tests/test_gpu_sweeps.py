@@ -55,6 +55,39 @@ def _rhs(shape, seed=5):
     return b
 
 
+# blocks of two rows, of several, split along one axis only; odd extents; the test met inside a
+# batch (of 16, 32, ... sweeps), at its end, and not at all; residuals checked at every sweep
+# and between; a start from a given pc whose ghost and boundary values count
+@pytest.mark.parametrize("shape,criterion,every,eps,cap", [
+    ((21, 9, 8), 0, 1, 1e-7, 100000), ((37, 18, 25), 1, 3, 1e-6, 100000), ((8, 41, 5), 1, 1, 1e-6, 100000),
+    ((7, 5, 61), 0, 1, 1e-30, 77), ((16, 12, 12), 1, 8, 1e-30, 48), ((16, 12, 12), 1, 5, 1e-30, 33),
+    ((130, 40, 31), 0, 1, 1e-30, 40)])
+def test_fp64_sweeps_on_chip_are_bit_exact(ib3d, grids, oracle_mod, shape, criterion, every, eps, cap):
+    x, y, z = (grids.tanh_axis(n) for n in shape)
+    b, pc0 = _rhs(shape), np.asfortranarray(np.random.default_rng(9).standard_normal(tuple(n + 2 for n in shape)))
+    o = oracle_mod.Oracle(x, y, z, 100.0, 1.0, omega=1.7, eps=eps, criterion=criterion, max_sweeps=cap,
+                          check_every=every)
+    o.no_body()
+    o.set_field("b", b)
+    r = o.redblack_sor(allow_noconv=True)
+    p = ib3d.default_params(re=100.0, deltat=1.0, omega=1.7, eps=eps, max_sweeps=cap)
+    p.criterion, p.check_every = criterion, every
+    s = ib3d.Solver(x, y, z, p)
+    s.set_field("b", b)
+    s.set_field("pc", pc0)
+    g = s.redblack_sor(allow_noconv=True)        # a zero start replaces the given pc
+    assert (g["sweeps"], g["final_err"]) == (r["sweeps"], r["final_err"])
+    want = o.get_field("pc")
+    assert np.array_equal(s.get_field("pc"), want)
+    # the fast form: the same method within rounding, amplified by the sweeps
+    s.set_params(precision=ib3d.PREC_FP64_FAST)
+    f = s.redblack_sor(allow_noconv=True)
+    assert abs(f["sweeps"] - r["sweeps"]) <= max(1, every)
+    if f["sweeps"] == r["sweeps"]:
+        assert np.max(np.abs(s.get_field("pc") - want)) <= 1e-13 * r["sweeps"] * np.max(np.abs(want))
+    s.close()
+
+
 def test_noalloc_solve_on_rows_too_long_for_a_block(ib3d, grids, oracle_mod):
     """Launch per colour pass, capped, against the context's one-array kernel on the same sweeps
     (the two round b/dt - A pc differently)."""
