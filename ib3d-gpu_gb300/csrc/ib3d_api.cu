@@ -243,7 +243,8 @@ int alloc_fields(ib3d_ctx* c) {
   cudaMemsetAsync(c->ibmap, 0xff, n3 * sizeof(int), c->st);
   if (cudaMalloc(&c->ctl, sizeof(SolveCtl)) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMallocHost(&c->h_ctl, sizeof(SolveCtl)) != cudaSuccess) return IB3D_ERR_MEMORY;
-  if (cudaMalloc(&c->d_flag, sizeof(int)) != cudaSuccess) return IB3D_ERR_MEMORY;
+  if (cudaMalloc(&c->d_flag, 4 * sizeof(int)) != cudaSuccess) return IB3D_ERR_MEMORY;
+  if (cudaMalloc(&c->d_levels, 128 * sizeof(int)) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMalloc(&c->d_coef, 8 * sizeof(double)) != cudaSuccess) return IB3D_ERR_MEMORY;
   {
     const double uc0 = 1.0;   // uc = 1 (subReadInput.f90:28); d_coef[6] holds the outlet speed
@@ -509,7 +510,7 @@ void ib3d_destroy(ib3d_ctx* c) {
   for (cudaEvent_t e : c->pool) cudaEventDestroy(e);
   free_ib(c);
   void* ptrs[] = {c->d_tables, c->d_tables32, c->d_fast, c->d_axp, c->u, c->v, c->w, c->ut, c->vt, c->wt, c->p, c->pc, c->b, c->bdt,
-                  c->e32, c->r32, c->ep[0], c->ep[1], c->rp[0], c->rp[1], c->cell, c->ibmap, c->ctl, c->d_nodes, c->d_tri, c->d_surf, c->d_iblist,
+                  c->e32, c->r32, c->ep[0], c->ep[1], c->rp[0], c->rp[1], c->cell, c->ibmap, c->ctl, c->d_nodes, c->d_tri, c->d_surf, c->d_c32, c->d_c32_max, c->d_levels, c->d_iblist,
                   c->d_nelp, c->d_nd, c->d_minel, c->d_scache, c->d_contrib, c->d_coef, c->d_flag, c->d_scan,
                   c->hist[0], c->hist[1], c->r_hist, c->d_norm, c->d_norm_part, c->resi[0], c->resi[1], c->resi[2],
                   c->wdiag, c->xch, c->pc2, c->d_errs, c->epn[0], c->epn[1], c->d_retag_mask, c->d_retag_list};
@@ -576,24 +577,33 @@ int ib3d_set_mesh(ib3d_ctx* c, int64_t nnodes, const double* xn, const double* y
     nodes[nnodes + i] = yn[i] + yshift;
     nodes[2 * nnodes + i] = zn[i] + zshift;
   }
-  cudaFree(c->d_nodes); cudaFree(c->d_tri); cudaFree(c->d_surf); cudaFree(c->d_scache); cudaFree(c->d_contrib);
-  c->d_nodes = nullptr; c->d_tri = nullptr; c->d_surf = nullptr; c->d_scache = nullptr; c->d_contrib = nullptr;
+  if (nnodes > c->nodes_cap || nelems > c->elems_cap) {   // room kept: a body may be set again and again
+    cudaFree(c->d_nodes); cudaFree(c->d_tri); cudaFree(c->d_surf); cudaFree(c->d_scache); cudaFree(c->d_contrib);
+    cudaFree(c->d_c32); cudaFree(c->d_c32_max);
+    c->d_c32 = nullptr; c->d_c32_max = nullptr;
+    c->d_nodes = nullptr; c->d_tri = nullptr; c->d_surf = nullptr; c->d_scache = nullptr; c->d_contrib = nullptr;
+    c->nodes_cap = c->elems_cap = 0;
+    c->nnodes = c->nelems = 0;
+    IB3D_CUDA(c, cudaMalloc(&c->d_nodes, (size_t)3 * nnodes * sizeof(double)));
+    IB3D_CUDA(c, cudaMalloc(&c->d_tri, (size_t)3 * nelems * sizeof(int)));
+    IB3D_CUDA(c, cudaMalloc(&c->d_scache, (size_t)15 * nelems * sizeof(int)));
+    IB3D_CUDA(c, cudaMalloc(&c->d_contrib, (size_t)7 * nelems * sizeof(double)));
+    IB3D_CUDA(c, cudaMalloc(&c->d_c32, ((size_t)nelems + 256) * sizeof(float4)));
+    IB3D_CUDA(c, cudaMalloc(&c->d_c32_max, sizeof(unsigned)));
+    IB3D_CUDA(c, cudaMalloc(&c->d_surf, (size_t)9 * nelems * sizeof(double)));
+    c->nodes_cap = nnodes;
+    c->elems_cap = nelems;
+  }
   c->nnodes = nnodes; c->nelems = nelems; c->inor = inor;
-  IB3D_CUDA(c, cudaMalloc(&c->d_nodes, nodes.size() * sizeof(double)));
-  IB3D_CUDA(c, cudaMalloc(&c->d_tri, tri.size() * sizeof(int)));
-  IB3D_CUDA(c, cudaMalloc(&c->d_surf, (size_t)9 * nelems * sizeof(double)));
-  IB3D_CUDA(c, cudaMalloc(&c->d_scache, (size_t)15 * nelems * sizeof(int)));
-  IB3D_CUDA(c, cudaMalloc(&c->d_contrib, (size_t)7 * nelems * sizeof(double)));
-  IB3D_CUDA(c, cudaMemcpy(c->d_nodes, nodes.data(), nodes.size() * sizeof(double), cudaMemcpyHostToDevice));
-  IB3D_CUDA(c, cudaMemcpy(c->d_tri, tri.data(), tri.size() * sizeof(int), cudaMemcpyHostToDevice));
-  int rc = run_surface_norm(c);
+  int bad = 0;
+  IB3D_CUDA(c, cudaMemcpyAsync(c->d_nodes, nodes.data(), nodes.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
+  IB3D_CUDA(c, cudaMemcpyAsync(c->d_tri, tri.data(), tri.size() * sizeof(int), cudaMemcpyHostToDevice, c->st));
+  IB3D_CUDA(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
+  int rc = run_surface_norm(c, c->d_flag);
   if (rc) return rc;
-  std::vector<double> cosv((size_t)3 * nelems);
-  IB3D_CUDA(c, cudaMemcpyAsync(cosv.data(), c->d_surf + 3 * nelems, cosv.size() * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->st));
+  IB3D_CUDA(c, cudaMemcpyAsync(&bad, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   IB3D_CUDA(c, cudaStreamSynchronize(c->st));
-  for (double x : cosv)
-    if (!std::isfinite(x)) return fail(c, IB3D_ERR_MESH, "ib3d_set_mesh: degenerate triangle (zero area)");
+  if (bad) return fail(c, IB3D_ERR_MESH, "ib3d_set_mesh: degenerate triangle (zero area)");
   c->searched = false;
   c->retag_ok = false;
   c->have_scache = false;

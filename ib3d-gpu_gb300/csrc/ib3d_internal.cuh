@@ -98,6 +98,7 @@ struct ForceSched {
   int nops;
   int nlevels;
   int* order;        // op ids sorted by level (device)
+  int* lvl;          // level of each op (device)
   std::vector<int> level_off;  // host: start of each level in `order`, size nlevels+1
   int* rd_idx;       // 8 linear read indices per op (device)
   int* rd_src;       // 8 sources per op: op id that wrote it earlier, or -1 (device)
@@ -105,8 +106,8 @@ struct ForceSched {
   int* brk;          // 3 bracket indices per op (device)
   unsigned char* fin;// 1 if the op is the last writer of its target (device)
   double* out;       // ghost value per op (device)
-  int* final_ops;    // ops with fin = 1 (device)
-  int nfinal;
+  int cap;           // ops that the arrays have room for
+  bool ordered;      // false: no op reads another's value, and one level holds them all
 };
 
 // How a grid's rows are split over the blocks of a resident kernel: gy x gz blocks of at
@@ -197,8 +198,11 @@ struct ib3d_ctx {
 
   // surface mesh
   long long nnodes = 0, nelems = 0, inor = 1;
+  long long nodes_cap = 0, elems_cap = 0;   // sizes that the arrays below have room for
   double* d_nodes = nullptr;  // 3*nnodes shifted node coordinates (x block, y block, z block)
   int* d_tri = nullptr;       // 3*nelems 1-based node ids
+  float4* d_c32 = nullptr;    // nelems FP32 centroids and 256 spheres around groups of them (k_ib.cu)
+  unsigned* d_c32_max = nullptr;
   double* d_surf = nullptr;   // 9*nelems: xc,yc,zc,cosA,cosB,cosG,alpha3,beta3,gamma3
   ib3d::Motion motion{};      // prescribed body motion (ib3d_move_body)
   double bprev[3] = {0, 0, 0};
@@ -216,6 +220,8 @@ struct ib3d_ctx {
   int* d_nelp = nullptr;      // nib, 1-based element ids
   double* d_nd = nullptr;     // 7*nib normal distances (p,u1,u2,v1,v2,w1,w2)
   int* d_minel = nullptr;     // box-sized nearest element
+  int* d_levels = nullptr;    // control words of the level search (k_ib.cu)
+  size_t minel_cap = 0, ib_cap = 0;   // cells that d_minel, and the IB arrays above, have room for
   long long box[6] = {0, 0, 0, 0, 0, 0};
 
   ib3d::ForceSched fv{};  // velocity ghost points
@@ -226,7 +232,7 @@ struct ib3d_ctx {
   int* d_scache = nullptr;     // 15*nelems: cell, u, v, w, p brackets (3 each)
   double* d_contrib = nullptr; // 7*nelems per-element terms
   double* d_coef = nullptr;    // 4 coefficients
-  int* d_flag = nullptr;       // device error flag (probe out of grid)
+  int* d_flag = nullptr;       // device flags: [0] error (probe out of grid), [1], [2] see finish_search
 
   // reduction / scan scratch
   long long* d_scan = nullptr;
@@ -290,7 +296,7 @@ bool fused_sweep_fits(int nx);
 bool run_resident32(ib3d_ctx* c, int n, int nsmooth, int nramp, double wi, float om, float om1);
 bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc);
 // k_ib.cu
-int run_surface_norm(ib3d_ctx* c);
+int run_surface_norm(ib3d_ctx* c, int* flag);
 int run_search(ib3d_ctx* c);
 int run_selective_retag(ib3d_ctx* c);
 int run_velocity_forcing(ib3d_ctx* c);

@@ -129,8 +129,9 @@ __device__ __forceinline__ OpGeom vel_geom(const Grid1D& g, const int* iblist, c
 // ------------------------------------------------------------- surface and search
 
 // computeSurfaceNorm (subSearch.f90:95-125).
+// flag (may be null) is set where a normal is not finite (a triangle without area).
 __global__ void k_surface_norm(const double* __restrict__ nodes, const int* __restrict__ tri, int nn, int ne,
-                               double inor, double* __restrict__ surf) {
+                               double inor, double* __restrict__ surf, int* flag) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   const int a = tri[e] - 1, b = tri[ne + e] - 1, c = tri[2 * ne + e] - 1;
@@ -145,9 +146,11 @@ __global__ void k_surface_norm(const double* __restrict__ nodes, const int* __re
   const double cg = (p2x - p1x) * (p3y - p1y) - (p3x - p1x) * (p2y - p1y);
   surf[6 * ne + e] = ca; surf[7 * ne + e] = cb; surf[8 * ne + e] = cg;
   const double len = sqrt((ca * ca + cb * cb) + cg * cg);
-  surf[3 * ne + e] = (ca / len) * inor;
-  surf[4 * ne + e] = (cb / len) * inor;
-  surf[5 * ne + e] = (cg / len) * inor;
+  const double na = (ca / len) * inor, nb = (cb / len) * inor, ng = (cg / len) * inor;
+  surf[3 * ne + e] = na;
+  surf[4 * ne + e] = nb;
+  surf[5 * ne + e] = ng;
+  if (flag && !(isfinite(na) && isfinite(nb) && isfinite(ng))) atomicExch(flag, 1);
 }
 
 __device__ __forceinline__ double corner_dot(const double* surf, int ne, int e, double x, double y, double z) {
@@ -161,76 +164,217 @@ __device__ __forceinline__ double corner_dot(const double* surf, int ne, int e, 
 // element whose squared distance is not below the current best's squared distance
 // cannot have a strictly smaller rounded root, so the root is only taken for
 // candidates that improve the squared distance: the same argmin, bit for bit.
-// Centroids are staged through shared memory in tiles. The cells tagged are the
-// box's (list == nullptr), or the nlist cells of a list inside the box (the
-// neighbourhoods of selectiveRetagging); minel is indexed by the cell's position in
-// the box either way.
-constexpr int kTagTile = 512;
+// The result is the lowest index among the elements of smallest rounded distance, whatever
+// the order, so elements that cannot attain it need no FP64 arithmetic, which this part
+// runs at 1/64 of the FP32 rate (the FP64 scan of every element took 9.6 of 11.3 ms of the
+// search at 256x192x192 with 5,120 triangles, an FP32 scan of every element 0.9).
+// k_centroid_groups gives the centroids in FP32 relative to the first one, and a sphere
+// around each of up to 256 groups of consecutive elements. Per cell: the group with the
+// nearest centre is scanned in FP32 for the smallest distance so far, then every group
+// whose sphere comes as near as that; elements within the error of the smallest distance
+// are queued, and those still within it at the end are evaluated in FP64. Four threads
+// share a cell, because the cells near the body's centre, whose distances to all groups
+// are alike, would keep single threads busy long after the rest.
+// Errors: with L the largest relative coordinate, an FP32 difference is off by at most
+// 2^-22 L (two conversions and a subtraction), so a distance by at most 3.5 x 2^-22 L with
+// its own rounding, and the nearest element lies within 7 x 2^-22 L of the FP32 minimum;
+// the bound used is 16 x 2^-22 L, for the spheres 64 x 2^-22 L, plus 1e-20 for squares that
+// underflow. Overflow and NaN pass the filters.
+// The cells tagged are the box's (list == nullptr), or the nlist cells of a list inside the
+// box (the neighbourhoods of selectiveRetagging); minel is indexed by the cell's position
+// in the box either way.
+constexpr int kGroups = 256;
+// elements per group: at least 32, a multiple of 32, at most kGroups groups
+__host__ __device__ __forceinline__ int group_size(int ne) { return ((ne + kGroups - 1) / kGroups + 31) / 32 * 32; }
+
+__device__ __forceinline__ float dist32(const float4 a, float x, float y, float z) {
+  const float dx = x - a.x, dy = y - a.y, dz = z - a.z;
+  return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+
+// Relative FP32 centroids c32[0..ne), a sphere per group (centre of the group's bounding
+// box, w its radius) behind them, and the largest |coordinate| (bit pattern, reset before).
+// One warp per group.
+__global__ void k_centroid_groups(const double* __restrict__ surf, int ne, float4* __restrict__ c32,
+                                  unsigned* __restrict__ big) {
+  const int gs = group_size(ne), lane = threadIdx.x & 31;
+  const int gr = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int e0 = gr * gs, e1 = min(ne, e0 + gs);
+  if (e0 >= ne) return;
+  const double ox = surf[0], oy = surf[ne], oz = surf[2 * ne];
+  const float inf = __int_as_float(0x7f800000);
+  float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+  for (int e = e0 + lane; e < e1; e += 32) {
+    const float v[3] = {(float)(surf[e] - ox), (float)(surf[ne + e] - oy), (float)(surf[2 * ne + e] - oz)};
+    c32[e] = make_float4(v[0], v[1], v[2], 0.f);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = fminf(lo[a], v[a]);
+      hi[a] = fmaxf(hi[a], v[a]);
+    }
+  }
+  float m = 0.f, c[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+      hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+    }
+    m = fmaxf(m, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
+    c[a] = 0.5f * lo[a] + 0.5f * hi[a];
+  }
+  float r = 0.f;
+  for (int e = e0 + lane; e < e1; e += 32) {
+    const float d = sqrtf(dist32(c32[e], c[0], c[1], c[2]));
+    r = d > r || d != d ? d : r;    // a NaN stays, and keeps the group in
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const float x = __shfl_xor_sync(0xffffffffu, r, o);
+    r = x > r || x != x ? x : r;
+  }
+  if (lane == 0) {
+    c32[ne + gr] = make_float4(c[0], c[1], c[2], r);
+    atomicMax(big, __float_as_uint(m));   // non-negative: the bit patterns order as the numbers
+  }
+}
+
 __global__ void __launch_bounds__(kBlock) k_tagging(Dims d, Grid1D g, const double* __restrict__ surf, int ne,
+                                                    const float4* __restrict__ c32, const unsigned* __restrict__ bigp,
                                                     int bi0, int bj0, int bk0, int bni, int bnj, int bnk,
                                                     const int* __restrict__ list, int nlist,
                                                     unsigned char* __restrict__ cell, int* __restrict__ minel) {
-  __shared__ double sx[kTagTile], sy[kTagTile], sz[kTagTile];
-  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int kQueue = 12;
+  __shared__ int qe[kQueue][kBlock];     // queued elements, per thread, and their FP32 squared distances
+  __shared__ float qd[kQueue][kBlock];
+  const int t = threadIdx.x, s = t & 3;  // four threads per cell, thread s its elements s, s + 4, ...
+  const unsigned quad = (t & 31) & ~3u;
+  const unsigned tid = (blockIdx.x * blockDim.x + t) >> 2;
   const unsigned ncell = list ? (unsigned)nlist : (unsigned)bni * (unsigned)bnj * (unsigned)bnk;
   const bool active = tid < ncell;
-  int i = 0, j = 0, k = 0;
-  double n1x = 0, n1y = 0, n1z = 0;
-  if (active) {
-    if (list) {
-      i = list[tid];
-      j = list[nlist + tid];
-      k = list[2 * nlist + tid];
-    } else {
-      i = bi0 + (int)(tid % (unsigned)bni);
-      const unsigned t = tid / (unsigned)bni;
-      j = bj0 + (int)(t % (unsigned)bnj);
-      k = bk0 + (int)(t / (unsigned)bnj);
-    }
-    n1x = g.xp[i]; n1y = g.yp[j]; n1z = g.zp[k];
+  const unsigned cid = active ? tid : 0;   // idle threads follow along on cell 0 and store nothing
+  int i, j, k;
+  if (list) {
+    i = list[cid];
+    j = list[nlist + cid];
+    k = list[2 * nlist + cid];
+  } else {
+    i = bi0 + (int)(cid % (unsigned)bni);
+    const unsigned r = cid / (unsigned)bni;
+    j = bj0 + (int)(r % (unsigned)bnj);
+    k = bk0 + (int)(r / (unsigned)bnj);
   }
-  double best = 1e14, best2 = 1e300;
-  int nel = 0;
-  for (int base = 0; base < ne; base += kTagTile) {
-    const int cnt = min(kTagTile, ne - base);
-    __syncthreads();
-    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-      sx[q] = surf[base + q]; sy[q] = surf[ne + base + q]; sz[q] = surf[2 * ne + base + q];
+  const double n1x = g.xp[i], n1y = g.yp[j], n1z = g.zp[k];
+  const float cx = (float)(n1x - surf[0]), cy = (float)(n1y - surf[ne]), cz = (float)(n1z - surf[2 * ne]);
+  const float L = fmaxf(__uint_as_float(*bigp), fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))));
+  const float slack = 0x1p-18f * L + 1e-20f, slack_group = 0x1p-16f * L + 1e-20f, up = 1.0f + 0x1p-20f;
+  const int gs = group_size(ne), ng = (ne + gs - 1) / gs;
+  const float4* sph = c32 + ne;
+  const float inf = __int_as_float(0x7f800000);
+  float m32 = inf, near2 = inf;          // smallest squared distance so far, and the queue's bound
+  double best = 1e14;
+  int nel = 0, nq = 0;
+  // the queued elements in FP64; together over the warp at the end (one by one each cost the
+  // warp a pass of the FP64 pipe)
+  auto evaluate = [&]() {
+    for (int u = 0; u < nq; ++u) {
+      if (qd[u][t] > near2) continue;
+      const int e = qe[u][t];
+      const double ay = n1y - surf[ne + e], ax = n1x - surf[e], az = n1z - surf[2 * ne + e];
+      const double dis = sqrt((ay * ay + ax * ax) + az * az);
+      if (dis < best || (dis == best && e + 1 < nel)) { best = dis; nel = e + 1; }
     }
-    __syncthreads();
-    if (active) {
-      for (int q = 0; q < cnt; ++q) {
-        const double ay = n1y - sy[q], ax = n1x - sx[q], az = n1z - sz[q];
-        const double d2 = (ay * ay + ax * ax) + az * az;
-        if (d2 < best2) {
-          const double dis = sqrt(d2);
-          if (dis < best) { best = dis; best2 = d2; nel = base + q + 1; }
-        }
+    nq = 0;
+  };
+  auto scan = [&](int q) {
+    const int e1 = min(ne, (q + 1) * gs);
+    for (int e0 = q * gs + s; e0 < e1; e0 += 32) {
+      float d2[8];
+      unsigned cand = 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int e = min(e0 + 4 * u, ne - 1);
+        d2[u] = dist32(c32[e], cx, cy, cz);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (e0 + 4 * u < e1 && !(d2[u] > near2)) cand |= 1u << u;
+      if (cand) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (cand >> u & 1) {
+            if (d2[u] < m32) {
+              m32 = d2[u];
+              const float T = sqrtf(m32) + slack;
+              near2 = T * T * up;
+            }
+            if (nq == kQueue) {            // drop what the bound has left behind
+              int n = 0;
+              for (int v = 0; v < kQueue; ++v)
+                if (!(qd[v][t] > near2)) {
+                  qe[n][t] = qe[v][t];
+                  qd[n][t] = qd[v][t];
+                  ++n;
+                }
+              nq = n;
+              if (nq == kQueue) evaluate();
+            }
+            qe[nq][t] = e0 + 4 * u;
+            qd[nq][t] = d2[u];
+            ++nq;
+          }
       }
     }
+    // the four threads share the smallest distance
+    m32 = fminf(m32, __shfl_xor_sync(0xfu << quad, m32, 1));
+    m32 = fminf(m32, __shfl_xor_sync(0xfu << quad, m32, 2));
+    const float T = sqrtf(m32) + slack;
+    near2 = T * T * up;
+  };
+  float c2 = inf;
+  int g0 = 0;
+#pragma unroll 4
+  for (int q = s; q < ng; q += 4) {
+    const float d2 = dist32(sph[q], cx, cy, cz);
+    if (d2 < c2) { c2 = d2; g0 = q; }
   }
-  if (!active) return;
-  const double n2x = g.x1[i], n3x = g.x1[i + 1], n2y = g.y1[j], n3y = g.y1[j + 1];
-  const double n2z = g.z1[k], n3z = g.z1[k + 1];
-  const int e = nel - 1;
-  const double thr = -1e-16;
-  double dd[8];
-  dd[0] = corner_dot(surf, ne, e, n2x, n2y, n2z);
-  dd[1] = corner_dot(surf, ne, e, n2x, n3y, n2z);
-  dd[2] = corner_dot(surf, ne, e, n3x, n2y, n2z);
-  dd[3] = corner_dot(surf, ne, e, n3x, n3y, n2z);
-  dd[4] = corner_dot(surf, ne, e, n2x, n2y, n3z);
-  dd[5] = corner_dot(surf, ne, e, n2x, n3y, n3z);
-  dd[6] = corner_dot(surf, ne, e, n3x, n2y, n3z);
-  dd[7] = corner_dot(surf, ne, e, n3x, n3y, n3z);
-  bool all_in = true, all_out = true;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    if (!(dd[q] <= thr)) all_in = false;
-    if (!(dd[q] > thr)) all_out = false;
+  for (int o = 1; o < 4; o <<= 1) {
+    const float x = __shfl_xor_sync(0xffffffffu, c2, o);
+    const int y = __shfl_xor_sync(0xffffffffu, g0, o);
+    if (x < c2 || (x == c2 && y < g0)) { c2 = x; g0 = y; }
   }
-  cell[d.at(i, j, k)] = all_in ? 1 : (all_out ? 0 : 2);
-  minel[(i - bi0) + bni * ((j - bj0) + bnj * (k - bk0))] = nel;
+  scan(g0);
+  for (int q0 = 0; q0 < ng; q0 += 4) {
+    const int q = q0 + s;
+    bool in = false;
+    if (q < ng && q != g0) {
+      const float4 sp = sph[q];
+      const float tr = sqrtf(m32) + slack_group + sp.w;
+      in = !(dist32(sp, cx, cy, cz) > tr * tr * up);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, in) >> quad;
+#pragma unroll 1
+    for (int u = 0; u < 4; ++u)
+      if (m >> u & 1) scan(q0 + u);
+  }
+  evaluate();
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    const double x = __shfl_xor_sync(0xffffffffu, best, o);
+    const int y = __shfl_xor_sync(0xffffffffu, nel, o);
+    if (y != 0 && (nel == 0 || x < best || (x == best && y < nel))) { best = x; nel = y; }
+  }
+  if (nel == 0) nel = 1;   // no element within 1e14
+  // the signs of the eight corners' distances to the element's plane, two per thread
+  const double x = s & 1 ? g.x1[i + 1] : g.x1[i], z = s & 2 ? g.z1[k + 1] : g.z1[k];
+  const double d0 = corner_dot(surf, ne, nel - 1, x, g.y1[j], z), d1 = corner_dot(surf, ne, nel - 1, x, g.y1[j + 1], z);
+  const double thr = -1e-16;
+  const bool all_in = (__ballot_sync(0xffffffffu, d0 <= thr && d1 <= thr) >> quad & 15u) == 15u;
+  const bool all_out = (__ballot_sync(0xffffffffu, d0 > thr && d1 > thr) >> quad & 15u) == 15u;
+  if (active && s == 0) {
+    cell[d.at(i, j, k)] = all_in ? 1 : (all_out ? 0 : 2);
+    minel[(i - bi0) + bni * ((j - bj0) + bnj * (k - bk0))] = nel;
+  }
 }
 
 // Bounding box of the IB list: {min i, max i, min j, max j, min k, max k}, out[] set
@@ -310,24 +454,28 @@ __global__ void k_mask_scatter(const unsigned char* __restrict__ mask, unsigned 
 
 // Cell counts over the interior (subSearch.f90:259-270) and the red/black split of
 // the fluid cells (subSearch.f90:557-567): {fluid, solid, ib, red, black}.
-__global__ void k_count(Dims d, const unsigned char* __restrict__ cell, unsigned long long* counts) {
+__global__ void __launch_bounds__(kBlock) k_count(Dims d, const unsigned char* __restrict__ cell,
+                                                  unsigned long long* counts) {
   __shared__ unsigned int sc[5];
   if (threadIdx.x < 5) sc[threadIdx.x] = 0;
   __syncthreads();
-  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid < (unsigned)d.nx * (unsigned)d.ny * (unsigned)d.nz) {
+  unsigned n[5] = {0, 0, 0, 0, 0};
+  const unsigned total = (unsigned)d.nx * (unsigned)d.ny * (unsigned)d.nz;
+  for (unsigned tid = blockIdx.x * blockDim.x + threadIdx.x; tid < total; tid += gridDim.x * blockDim.x) {
     const int i = (int)(tid % (unsigned)d.nx) + 2;
     const unsigned t = tid / (unsigned)d.nx;
     const int j = (int)(t % (unsigned)d.ny) + 2, k = (int)(t / (unsigned)d.ny) + 2;
     const unsigned char c = cell[d.at(i, j, k)];
-    if (c == 0) {
-      atomicAdd(&sc[0], 1u);
-      atomicAdd(&sc[((i + j + k) & 1) ? 3 : 4], 1u);
-    } else if (c == 1) {
-      atomicAdd(&sc[1], 1u);
-    } else if (c == 2) {
-      atomicAdd(&sc[2], 1u);
-    }
+    n[0] += c == 0;
+    n[1] += c == 1;
+    n[2] += c == 2;
+    n[3] += c == 0 && ((i + j + k) & 1);
+    n[4] += c == 0 && !((i + j + k) & 1);
+  }
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const unsigned s = __reduce_add_sync(0xffffffffu, n[q]);
+    if ((threadIdx.x & 31) == 0 && s) atomicAdd(&sc[q], s);
   }
   __syncthreads();
   if (threadIdx.x < 5 && sc[threadIdx.x]) atomicAdd(&counts[threadIdx.x], (unsigned long long)sc[threadIdx.x]);
@@ -447,7 +595,7 @@ __global__ void k_sched_vel(Dims d, Grid1D g, const int* __restrict__ iblist, co
                             const double* __restrict__ nd, const double* __restrict__ surf, int nib, int ne,
                             const int* __restrict__ ibmap, int* __restrict__ brk, int* __restrict__ rd_idx,
                             int* __restrict__ rd_src, int* __restrict__ tgt, unsigned char* __restrict__ fin,
-                            int* err) {
+                            int* err, int* deps) {
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= 6ll * nib) return;
   const int n = (int)(q / 6), blk = (int)(q % 6);
@@ -478,6 +626,7 @@ __global__ void k_sched_vel(Dims d, Grid1D g, const int* __restrict__ iblist, co
     for (int s = 0; s < 2; ++s)
       if (w[s] >= 0 && w[s] < q && w[s] > src) src = w[s];
     rd_src[8 * q + r] = (int)src;
+    if (src >= 0) *deps = 1;
   }
   const int ta = o.i + gb.tgt[0], tb = o.j + gb.tgt[1], tc = o.k + gb.tgt[2];
   tgt[q] = (int)d.at(ta, tb, tc);
@@ -492,7 +641,7 @@ __global__ void k_sched_p(Dims d, Grid1D g, const int* __restrict__ iblist, cons
                           const double* __restrict__ nd, const double* __restrict__ surf, int nib, int ne,
                           const int* __restrict__ ibmap, int* __restrict__ brk, int* __restrict__ rd_idx,
                           int* __restrict__ rd_src, int* __restrict__ tgt, unsigned char* __restrict__ fin,
-                          int* err) {
+                          int* err, int* deps) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nib) return;
   const int i = iblist[n], j = iblist[nib + n], k = iblist[2 * nib + n];
@@ -519,6 +668,7 @@ __global__ void k_sched_p(Dims d, Grid1D g, const int* __restrict__ iblist, cons
       if (m >= 0 && m < n) src = m;
     }
     rd_src[8 * n + r] = src;
+    if (src >= 0) *deps = 1;
   }
   tgt[n] = (int)d.at(i, j, k);
   fin[n] = 1;
@@ -536,7 +686,7 @@ __global__ void k_force_vel(Grid1D g, const int* __restrict__ order, int off, in
                             double* out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
-  const int q = order[off + t];
+  const int q = order ? order[off + t] : t;   // null: one level holds every op
   const int n = q / 6, blk = q % 6;
   const GhostBlock& gb = c_ghost[blk];
   const OpGeom o = vel_geom(g, iblist, nelp, nd, surf, nib, ne, n, blk);
@@ -569,7 +719,7 @@ __global__ void k_force_p(Grid1D g, const int* __restrict__ order, int off, int 
                           const double* __restrict__ p, Motion mo, double* out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
-  const int n = order[off + t];
+  const int n = order ? order[off + t] : t;
   const int i = iblist[n], j = iblist[nib + n], k = iblist[2 * nib + n];
   const int e = nelp[n] - 1;
   const double sd = nd[n];
@@ -597,11 +747,10 @@ __global__ void k_force_p(Grid1D g, const int* __restrict__ order, int off, int 
 }
 
 // Stores each face's last-writer value (after every level has run).
-__global__ void k_force_scatter(const int* __restrict__ final_ops, int nfinal, const int* __restrict__ tgt,
+__global__ void k_force_scatter(const unsigned char* __restrict__ fin, int nops, const int* __restrict__ tgt,
                                 const double* __restrict__ out, int vel, double* f0, double* f1, double* f2) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nfinal) return;
-  const int q = final_ops[t];
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nops || !fin[q]) return;
   double* F = f0;
   if (vel) {
     const int field = (q % 6) >> 1;
@@ -717,34 +866,83 @@ int run_move_body(ib3d_ctx* c, double dx, double dy, double dz) {
   k_shift_nodes<<<nblk(c->nnodes), kBlock, 0, c->st>>>(c->d_nodes, (int)c->nnodes, dx, dy, dz);
   IB3D_CUDA(c, cudaGetLastError());
   c->launches += 2;
-  return run_surface_norm(c);
+  return run_surface_norm(c, nullptr);
 }
 
-int run_surface_norm(ib3d_ctx* c) {
+int run_surface_norm(ib3d_ctx* c, int* flag) {
   k_surface_norm<<<nblk(c->nelems), kBlock, 0, c->st>>>(c->d_nodes, c->d_tri, (int)c->nnodes, (int)c->nelems,
-                                                        (double)c->inor, c->d_surf);
+                                                        (double)c->inor, c->d_surf, flag);
   IB3D_CUDA(c, cudaGetLastError());
   return IB3D_OK;
 }
 
+// One round of the level search: l = 1 + max level of the sources. Levels only grow, so a
+// round that reads another op's newer level is as good. ctl[0] becomes r + 1 when the round
+// changed something.
+__global__ void k_level_round(int n, const int* __restrict__ src, int* lvl, int r, int* ctl) {
+  if (*ctl < r) return;   // the last round changed nothing
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  int l = 0;
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const int e = src[8 * (size_t)q + s];
+    if (e >= 0) l = max(l, ((volatile int*)lvl)[e] + 1);
+  }
+  if (l != lvl[q]) {
+    lvl[q] = l;
+    atomicMax(ctl, r + 1);
+  }
+}
+// Ops per level; the last of `most` counts also takes what lies beyond. Counted per block
+// first: nearly all ops are of one level, and one counter for all of them took 31 us.
+__global__ void __launch_bounds__(kBlock) k_level_count(int n, const int* __restrict__ lvl, int most, int* cnt) {
+  __shared__ int s[32];
+  if (threadIdx.x < 32) s[threadIdx.x] = 0;
+  __syncthreads();
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < n) atomicAdd(&s[min(lvl[q], most - 1)], 1);
+  __syncthreads();
+  if (threadIdx.x < (unsigned)most && s[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], s[threadIdx.x]);
+}
+struct LevelStart {
+  int at[32];
+};
+// The ops of each level together, in no particular order: those of one level do not depend
+// on one another.
+__global__ void __launch_bounds__(kBlock) k_level_scatter(int n, const int* __restrict__ lvl, LevelStart start,
+                                                          int* __restrict__ used, int* __restrict__ order) {
+  __shared__ int s[32], at[32];
+  if (threadIdx.x < 32) s[threadIdx.x] = 0;
+  __syncthreads();
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int l = q < n ? lvl[q] : 0;
+  const int mine = q < n ? atomicAdd(&s[l], 1) : 0;
+  __syncthreads();
+  if (threadIdx.x < 32 && s[threadIdx.x]) at[threadIdx.x] = start.at[threadIdx.x] + atomicAdd(&used[threadIdx.x], s[threadIdx.x]);
+  __syncthreads();
+  if (q < n) order[at[l] + mine] = q;
+}
+
 namespace {
 void free_sched(ForceSched& s) {
+  cudaFree(s.lvl);
   cudaFree(s.order); cudaFree(s.rd_idx); cudaFree(s.rd_src); cudaFree(s.tgt); cudaFree(s.brk);
-  cudaFree(s.fin); cudaFree(s.out); cudaFree(s.final_ops);
+  cudaFree(s.fin); cudaFree(s.out);
   s = ForceSched{};
 }
 
 // Dependency levels (level = 1 + max level of the sources; sources precede the op in
-// serial order) and the level-sorted op list.
-int build_levels(ib3d_ctx* c, ForceSched& s) {
+// serial order) and the level-sorted op list, for a schedule in which some op reads
+// another's value. The levels settle on the device in as many rounds as there are levels
+// (a handful); a schedule that is still moving after kRounds, or has more than kMaxLevels,
+// is sorted on the host (the copies and loops of that took 0.35 ms at 45,000 ops).
+constexpr int kRounds = 8, kMaxLevels = 32;   // k_level_count and k_level_scatter hold 32
+int build_levels_host(ib3d_ctx* c, ForceSched& s) {
   const int n = s.nops;
   std::vector<int> src((size_t)8 * n), lvl(n, 0);
-  std::vector<unsigned char> fin(n);
-  if (n > 0) {
-    IB3D_CUDA(c, cudaMemcpyAsync(src.data(), s.rd_src, sizeof(int) * 8 * (size_t)n, cudaMemcpyDeviceToHost, c->st));
-    IB3D_CUDA(c, cudaMemcpyAsync(fin.data(), s.fin, (size_t)n, cudaMemcpyDeviceToHost, c->st));
-    IB3D_CUDA(c, cudaStreamSynchronize(c->st));
-  }
+  IB3D_CUDA(c, cudaMemcpyAsync(src.data(), s.rd_src, sizeof(int) * 8 * (size_t)n, cudaMemcpyDeviceToHost, c->st));
+  IB3D_CUDA(c, cudaStreamSynchronize(c->st));
   int maxl = -1;
   for (int q = 0; q < n; ++q) {
     int l = 0;
@@ -759,32 +957,61 @@ int build_levels(ib3d_ctx* c, ForceSched& s) {
   s.level_off.assign((size_t)s.nlevels + 1, 0);
   for (int q = 0; q < n; ++q) s.level_off[lvl[q] + 1]++;
   for (int l = 0; l < s.nlevels; ++l) s.level_off[l + 1] += s.level_off[l];
-  std::vector<int> order(n), pos(s.level_off.begin(), s.level_off.end() - 1), finals;
+  std::vector<int> order(n), pos(s.level_off.begin(), s.level_off.end() - 1);
   for (int q = 0; q < n; ++q) order[pos[lvl[q]]++] = q;
-  for (int q = 0; q < n; ++q)
-    if (fin[q]) finals.push_back(q);
-  s.nfinal = (int)finals.size();
-  IB3D_CUDA(c, cudaMalloc(&s.order, sizeof(int) * (size_t)std::max(n, 1)));
-  IB3D_CUDA(c, cudaMalloc(&s.final_ops, sizeof(int) * (size_t)std::max(s.nfinal, 1)));
-  if (n > 0)
-    IB3D_CUDA(c, cudaMemcpyAsync(s.order, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->st));
-  if (s.nfinal > 0)
-    IB3D_CUDA(c, cudaMemcpyAsync(s.final_ops, finals.data(), sizeof(int) * (size_t)s.nfinal,
-                                 cudaMemcpyHostToDevice, c->st));
+  IB3D_CUDA(c, cudaMemcpyAsync(s.order, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->st));
   IB3D_CUDA(c, cudaStreamSynchronize(c->st));
+  s.ordered = true;
   return IB3D_OK;
 }
 
+// ctl: [0] rounds that changed a level, [1..kMaxLevels] ops per level (the last one also
+// counts what lies beyond)
+int build_levels(ib3d_ctx* c, ForceSched& s) {
+  const int n = s.nops;
+  int* ctl = c->d_levels;
+  IB3D_CUDA(c, cudaMemsetAsync(s.lvl, 0, sizeof(int) * (size_t)n, c->st));
+  IB3D_CUDA(c, cudaMemsetAsync(ctl, 0, sizeof(int) * (2 * kMaxLevels + 1), c->st));
+  for (int r = 0; r < kRounds; ++r) k_level_round<<<nblk(n), kBlock, 0, c->st>>>(n, s.rd_src, s.lvl, r, ctl);
+  k_level_count<<<nblk(n), kBlock, 0, c->st>>>(n, s.lvl, kMaxLevels, ctl + 1);
+  int h[kMaxLevels + 1];
+  IB3D_CUDA(c, cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, c->st));
+  IB3D_CUDA(c, cudaStreamSynchronize(c->st));
+  if (h[0] >= kRounds || h[kMaxLevels] != 0) return build_levels_host(c, s);
+  s.nlevels = 0;
+  s.level_off.assign(1, 0);
+  for (int l = 0; l < kMaxLevels && h[1 + l] > 0; ++l) {
+    s.level_off.push_back(s.level_off.back() + h[1 + l]);
+    ++s.nlevels;
+  }
+  LevelStart start{};
+  for (int l = 0; l < s.nlevels; ++l) start.at[l] = s.level_off[l];
+  k_level_scatter<<<nblk(n), kBlock, 0, c->st>>>(n, s.lvl, start, ctl + 1 + kMaxLevels, s.order);
+  IB3D_CUDA(c, cudaGetLastError());
+  s.ordered = true;
+  return IB3D_OK;
+}
+
+// Room for nops ops, kept for the next search (a moving body searches every step), and a
+// schedule of one level until build_levels finds more.
 int alloc_sched(ib3d_ctx* c, ForceSched& s, int nops) {
-  free_sched(s);
+  if (nops > s.cap || s.cap == 0) {
+    const size_t n = (size_t)nops + (size_t)nops / 8 + 64;
+    free_sched(s);
+    IB3D_CUDA(c, cudaMalloc(&s.order, sizeof(int) * n));
+    IB3D_CUDA(c, cudaMalloc(&s.lvl, sizeof(int) * n));
+    IB3D_CUDA(c, cudaMalloc(&s.rd_idx, sizeof(int) * 8 * n));
+    IB3D_CUDA(c, cudaMalloc(&s.rd_src, sizeof(int) * 8 * n));
+    IB3D_CUDA(c, cudaMalloc(&s.tgt, sizeof(int) * n));
+    IB3D_CUDA(c, cudaMalloc(&s.brk, sizeof(int) * 3 * n));
+    IB3D_CUDA(c, cudaMalloc(&s.fin, n));
+    IB3D_CUDA(c, cudaMalloc(&s.out, sizeof(double) * n));
+    s.cap = (int)n;
+  }
   s.nops = nops;
-  const size_t n = (size_t)std::max(nops, 1);
-  IB3D_CUDA(c, cudaMalloc(&s.rd_idx, sizeof(int) * 8 * n));
-  IB3D_CUDA(c, cudaMalloc(&s.rd_src, sizeof(int) * 8 * n));
-  IB3D_CUDA(c, cudaMalloc(&s.tgt, sizeof(int) * n));
-  IB3D_CUDA(c, cudaMalloc(&s.brk, sizeof(int) * 3 * n));
-  IB3D_CUDA(c, cudaMalloc(&s.fin, n));
-  IB3D_CUDA(c, cudaMalloc(&s.out, sizeof(double) * n));
+  s.ordered = false;
+  s.nlevels = nops > 0 ? 1 : 0;
+  s.level_off.assign({0, nops});
   return IB3D_OK;
 }
 }  // namespace
@@ -805,6 +1032,40 @@ int ensure_scan(ib3d_ctx* c, size_t n) {
   }
   return IB3D_OK;
 }
+// Nearest elements of the box's cells, room kept for the next search.
+int ensure_minel(ib3d_ctx* c, size_t nbox) {
+  if (nbox > c->minel_cap) {
+    cudaFree(c->d_minel);
+    c->d_minel = nullptr;
+    c->minel_cap = 0;
+    const size_t n = nbox + nbox / 4;
+    IB3D_CUDA(c, cudaMalloc(&c->d_minel, sizeof(int) * n));
+    c->minel_cap = n;
+  }
+  return IB3D_OK;
+}
+// The IB list with its elements and distances, room kept for the next search.
+int ensure_ib(ib3d_ctx* c, size_t nib) {
+  if (nib > c->ib_cap || c->ib_cap == 0) {
+    cudaFree(c->d_iblist); cudaFree(c->d_nelp); cudaFree(c->d_nd);
+    c->d_iblist = nullptr; c->d_nelp = nullptr; c->d_nd = nullptr;
+    c->ib_cap = 0;
+    const size_t n = nib + nib / 8 + 64;
+    IB3D_CUDA(c, cudaMalloc(&c->d_iblist, sizeof(int) * 3 * n));
+    IB3D_CUDA(c, cudaMalloc(&c->d_nelp, sizeof(int) * n));
+    IB3D_CUDA(c, cudaMalloc(&c->d_nd, sizeof(double) * 7 * n));
+    c->ib_cap = n;
+  }
+  return IB3D_OK;
+}
+// The FP32 centroids and their groups for k_tagging, from the surface as it is now.
+int group_centroids(ib3d_ctx* c) {
+  const int ne = (int)c->nelems, gs = group_size(ne), ng = (ne + gs - 1) / gs;
+  IB3D_CUDA(c, cudaMemsetAsync(c->d_c32_max, 0, sizeof(unsigned), c->st));
+  k_centroid_groups<<<(ng + 7) / 8, 256, 0, c->st>>>(c->d_surf, ne, c->d_c32, c->d_c32_max);
+  IB3D_CUDA(c, cudaGetLastError());
+  return IB3D_OK;
+}
 int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int bnk);
 }  // namespace
 
@@ -817,10 +1078,9 @@ int run_search(ib3d_ctx* c) {
   const int ne = (int)c->nelems;
   // fresh flags and maps
   IB3D_CUDA(c, cudaMemsetAsync(c->cell, 0, (size_t)d.n3, c->st));
-  cudaFree(c->d_minel);
-  c->d_minel = nullptr;
-  IB3D_CUDA(c, cudaMalloc(&c->d_minel, sizeof(int) * (size_t)nbox));
-  k_tagging<<<nblk(nbox), kBlock, 0, c->st>>>(d, c->g, c->d_surf, ne, bi0, bj0, bk0, bni, bnj, bnk, nullptr, 0,
+  if (int rc = ensure_minel(c, nbox)) return rc;
+  if (int rc = group_centroids(c)) return rc;
+  k_tagging<<<nblk(4ll * nbox), kBlock, 0, c->st>>>(d, c->g, c->d_surf, ne, c->d_c32, c->d_c32_max, bi0, bj0, bk0, bni, bnj, bnk, nullptr, 0,
                                                c->cell, c->d_minel);
   IB3D_CUDA(c, cudaGetLastError());
   return finish_search(c, bi0, bj0, bk0, bni, bnj, bnk);
@@ -847,9 +1107,7 @@ int run_selective_retag(ib3d_ctx* c) {
   const int bk0 = std::max(hb[4] - 2, 2), bk1 = std::min(hb[5] + 3, d.nz + 1);
   const int bni = bi1 - bi0 + 1, bnj = bj1 - bj0 + 1, bnk = bk1 - bk0 + 1;
   const unsigned nbox = (unsigned)bni * bnj * bnk;
-  cudaFree(c->d_minel);
-  c->d_minel = nullptr;
-  IB3D_CUDA(c, cudaMalloc(&c->d_minel, sizeof(int) * (size_t)nbox));
+  if (int rc = ensure_minel(c, nbox)) return rc;
   IB3D_CUDA(c, cudaMemsetAsync(c->d_minel, 0, sizeof(int) * (size_t)nbox, c->st));
   if ((size_t)nbox > c->retag_cap) {
     cudaFree(c->d_retag_mask);
@@ -874,8 +1132,9 @@ int run_selective_retag(ib3d_ctx* c) {
   // the list is sized for the whole box: the three index blocks start nlist apart
   k_mask_scatter<<<nb, kBlock, 0, c->st>>>(c->d_retag_mask, nbox, bi0, bj0, bk0, bni, bnj, boff, (int)nlist,
                                            c->d_retag_list);
+  if (int rc = group_centroids(c)) return rc;
   if (nlist > 0)
-    k_tagging<<<nblk(nlist), kBlock, 0, c->st>>>(d, c->g, c->d_surf, ne, bi0, bj0, bk0, bni, bnj, bnk,
+    k_tagging<<<nblk(4ll * nlist), kBlock, 0, c->st>>>(d, c->g, c->d_surf, ne, c->d_c32, c->d_c32_max, bi0, bj0, bk0, bni, bnj, bnk,
                                                  c->d_retag_list, (int)nlist, c->cell, c->d_minel);
   IB3D_CUDA(c, cudaGetLastError());
   c->retagged = nlist;
@@ -894,7 +1153,7 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
   // counts
   unsigned long long* dcount = reinterpret_cast<unsigned long long*>(c->d_scan);
   IB3D_CUDA(c, cudaMemsetAsync(dcount, 0, 5 * sizeof(unsigned long long), c->st));
-  k_count<<<nblk((long long)d.nx * d.ny * d.nz), kBlock, 0, c->st>>>(d, c->cell, dcount);
+  k_count<<<std::min(nblk((long long)d.nx * d.ny * d.nz), 8u * (unsigned)c->nsm), kBlock, 0, c->st>>>(d, c->cell, dcount);
   unsigned long long hc[5];
   IB3D_CUDA(c, cudaMemcpyAsync(hc, dcount, sizeof(hc), cudaMemcpyDeviceToHost, c->st));
   IB3D_CUDA(c, cudaStreamSynchronize(c->st));
@@ -902,11 +1161,7 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
   c->nib = (int)hc[2];
   const int nib = c->nib;
   // compaction of the IB cells
-  cudaFree(c->d_iblist); cudaFree(c->d_nelp); cudaFree(c->d_nd);
-  c->d_iblist = nullptr; c->d_nelp = nullptr; c->d_nd = nullptr;
-  IB3D_CUDA(c, cudaMalloc(&c->d_iblist, sizeof(int) * 3 * (size_t)std::max(nib, 1)));
-  IB3D_CUDA(c, cudaMalloc(&c->d_nelp, sizeof(int) * (size_t)std::max(nib, 1)));
-  IB3D_CUDA(c, cudaMalloc(&c->d_nd, sizeof(double) * 7 * (size_t)std::max(nib, 1)));
+  if (int rc = ensure_ib(c, (size_t)nib)) return rc;
   const unsigned nb = nblk(nbox);
   if (int rc = ensure_scan(c, nb)) return rc;
   long long* boff = c->d_scan + 8;
@@ -918,7 +1173,7 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
                                                 bk0, bni, bnj, c->d_nelp, c->d_nd, c->ibmap);
   IB3D_CUDA(c, cudaGetLastError());
   // ghost-point schedules
-  IB3D_CUDA(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
+  IB3D_CUDA(c, cudaMemsetAsync(c->d_flag, 0, 3 * sizeof(int), c->st));
   int rc = alloc_sched(c, c->fv, 6 * nib);
   if (rc) return rc;
   rc = alloc_sched(c, c->fp, nib);
@@ -926,20 +1181,19 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
   if (nib > 0) {
     k_sched_vel<<<nblk(6ll * nib), kBlock, 0, c->st>>>(d, c->g, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf, nib, ne,
                                                        c->ibmap, c->fv.brk, c->fv.rd_idx, c->fv.rd_src, c->fv.tgt,
-                                                       c->fv.fin, c->d_flag);
+                                                       c->fv.fin, c->d_flag, c->d_flag + 1);
     k_sched_p<<<nblk(nib), kBlock, 0, c->st>>>(d, c->g, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf, nib, ne,
                                                c->ibmap, c->fp.brk, c->fp.rd_idx, c->fp.rd_src, c->fp.tgt, c->fp.fin,
-                                               c->d_flag);
+                                               c->d_flag, c->d_flag + 2);
     IB3D_CUDA(c, cudaGetLastError());
   }
-  rc = build_levels(c, c->fv);
-  if (rc) return rc;
-  rc = build_levels(c, c->fp);
-  if (rc) return rc;
-  int flag = 0;
-  IB3D_CUDA(c, cudaMemcpy(&flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
+  int flag[3] = {0, 0, 0};   // a probe off the grid; ops of the velocity, of the pressure depend on one another
+  IB3D_CUDA(c, cudaMemcpyAsync(flag, c->d_flag, sizeof(flag), cudaMemcpyDeviceToHost, c->st));
+  IB3D_CUDA(c, cudaStreamSynchronize(c->st));
+  if (flag[1] && (rc = build_levels(c, c->fv))) return rc;
+  if (flag[2] && (rc = build_levels(c, c->fp))) return rc;
   c->have_scache = false;
-  if (flag) {
+  if (flag[0]) {
     c->err = "ib3d_search: a ghost-point probe fell outside the grid";
     return IB3D_ERR_PROBE;
   }
@@ -950,16 +1204,16 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
 int run_velocity_forcing(ib3d_ctx* c) {
   PhaseScope ps(c, PH_FORCING);
   ForceSched& s = c->fv;
-  c->launches += s.nlevels + (s.nfinal > 0 ? 1 : 0);
+  c->launches += s.nlevels + (s.nops > 0 ? 1 : 0);
   for (int l = 0; l < s.nlevels; ++l) {
     const int off = s.level_off[l], cnt = s.level_off[l + 1] - off;
     if (cnt <= 0) continue;
-    k_force_vel<<<nblk(cnt), kBlock, 0, c->st>>>(c->g, s.order, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
+    k_force_vel<<<nblk(cnt), kBlock, 0, c->st>>>(c->g, s.ordered ? s.order : nullptr, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
                                                  c->nib, (int)c->nelems, s.brk, s.rd_idx, s.rd_src, c->ut, c->vt,
                                                  c->wt, c->motion, s.out);
   }
-  if (s.nfinal > 0)
-    k_force_scatter<<<nblk(s.nfinal), kBlock, 0, c->st>>>(s.final_ops, s.nfinal, s.tgt, s.out, 1, c->ut, c->vt,
+  if (s.nops > 0)
+    k_force_scatter<<<nblk(s.nops), kBlock, 0, c->st>>>(s.fin, s.nops, s.tgt, s.out, 1, c->ut, c->vt,
                                                           c->wt);
   IB3D_CUDA(c, cudaGetLastError());
   return IB3D_OK;
@@ -969,16 +1223,16 @@ int run_pressure_forcing(ib3d_ctx* c) {
   PhaseScope ps(c, PH_FORCING);
   ForceSched& s = c->fp;
   for (int q = 0; q < 3; ++q) c->motion.acc[q] = -(c->motion.vel[q] - c->bprev[q]) / c->prm.deltat;   // :20
-  c->launches += s.nlevels + (s.nfinal > 0 ? 1 : 0);
+  c->launches += s.nlevels + (s.nops > 0 ? 1 : 0);
   for (int l = 0; l < s.nlevels; ++l) {
     const int off = s.level_off[l], cnt = s.level_off[l + 1] - off;
     if (cnt <= 0) continue;
-    k_force_p<<<nblk(cnt), kBlock, 0, c->st>>>(c->g, s.order, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
+    k_force_p<<<nblk(cnt), kBlock, 0, c->st>>>(c->g, s.ordered ? s.order : nullptr, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
                                                c->nib, (int)c->nelems, s.brk, s.rd_idx, s.rd_src, c->p, c->motion,
                                                s.out);
   }
-  if (s.nfinal > 0)
-    k_force_scatter<<<nblk(s.nfinal), kBlock, 0, c->st>>>(s.final_ops, s.nfinal, s.tgt, s.out, 0, c->p, nullptr,
+  if (s.nops > 0)
+    k_force_scatter<<<nblk(s.nops), kBlock, 0, c->st>>>(s.fin, s.nops, s.tgt, s.out, 0, c->p, nullptr,
                                                           nullptr);
   IB3D_CUDA(c, cudaGetLastError());
   return IB3D_OK;
