@@ -764,89 +764,148 @@ __global__ void k_force_scatter(const unsigned char* __restrict__ fin, int nops,
 // Per-element terms of stressCal1/2 (subStressCal1.f90:85-434): viscous traction and
 // pressure force from the probe at one cell diagonal along the normal. Probe cells
 // are found on the first call and cached (stressCal2 reuses them, :81-83 etc.).
-__global__ void k_stress_elem(Dims d, Grid1D g, const double* __restrict__ surf, int ne, int first,
-                              int* __restrict__ scache, const double* __restrict__ ut,
-                              const double* __restrict__ vt, const double* __restrict__ wt,
-                              const double* __restrict__ p, double inv_re, double* __restrict__ contrib, int* err) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
+// Four threads per element, one per probed field: each probe is a chain of some 20 FP64
+// divisions, and 5,120 elements of one thread each filled 20 of the SMs (with the sum below
+// 0.35 ms; now 0.1).
+__global__ void __launch_bounds__(64) k_stress_elem(Dims d, Grid1D g, const double* __restrict__ surf, int ne, int first,
+                                                    int* __restrict__ scache, const double* __restrict__ ut,
+                                                    const double* __restrict__ vt, const double* __restrict__ wt,
+                                                    const double* __restrict__ p, double inv_re,
+                                                    double* __restrict__ contrib, int* err) {
+  const int e0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, c = threadIdx.x & 3;
+  const bool active = e0 < ne;
+  const int e = active ? e0 : ne - 1;   // idle threads follow along on the last element and store nothing
+  const int lead = (threadIdx.x & 31) & ~3;
   const int nn[3] = {d.nx, d.ny, d.nz};
   const double xs = surf[e], ys = surf[ne + e], zs = surf[2 * ne + e];
   const double ca = surf[3 * ne + e], cb = surf[4 * ne + e], cg = surf[5 * ne + e];
-  if (first) {
-    const double cpos[3] = {xs, ys, zs};
-    const double* A1[3] = {g.x1, g.y1, g.z1};
-    for (int a = 0; a < 3; ++a) {
-      int b = bracket(A1[a], 2, nn[a] + 1, cpos[a]);                   // :89-105
-      if (!b) { atomicExch(err, 1); b = 2; }
-      scache[15 * e + a] = b;
+  int cell = 0;   // thread c < 3: the element's cell along axis c
+  if (c < 3) {
+    if (first) {
+      cell = bracket(c == 0 ? g.x1 : c == 1 ? g.y1 : g.z1, 2, c == 0 ? d.nx + 1 : c == 1 ? d.ny + 1 : d.nz + 1,
+                     c == 0 ? xs : c == 1 ? ys : zs);                  // :89-105
+      if (!cell) { if (active) atomicExch(err, 1); cell = 2; }
+      if (active) scache[15 * e + c] = cell;
+    } else {
+      cell = scache[15 * e + c];
     }
   }
-  const int ic = scache[15 * e], jc = scache[15 * e + 1], kc = scache[15 * e + 2];
+  const int ic = __shfl_sync(0xffffffffu, cell, lead), jc = __shfl_sync(0xffffffffu, cell, lead + 1),
+            kc = __shfl_sync(0xffffffffu, cell, lead + 2);
   const double dX = g.x1[ic + 1] - g.x1[ic], dY = g.y1[jc + 1] - g.y1[jc], dZ = g.z1[kc + 1] - g.z1[kc];
   const double diagdis = sqrt((dX * dX + dY * dY) + dZ * dZ);           // :119
   const double px = xs + diagdis * ca, py = ys + diagdis * cb, pz = zs + diagdis * cg;
-  const double ppos[3] = {px, py, pz};
-  double dnds[3];
-  for (int c = 0; c < 4; ++c) {
-    const StagCoords sc = stag(g, c);
+  const StagCoords sc = stag(g, c);
+  int br[3];
+  if (first) {
+    const double ppos[3] = {px, py, pz};
     const double* A[3] = {sc.X, sc.Y, sc.Z};
-    if (first) {
-      for (int a = 0; a < 3; ++a) {
-        int b = bracket(A[a], 2, nn[a] + 1, ppos[a]);                  // e.g. :135-145
-        if (!b) { atomicExch(err, 1); b = 2; }
-        scache[15 * e + 3 + 3 * c + a] = b;
-      }
-    }
-    const int ix = scache[15 * e + 3 + 3 * c], iy = scache[15 * e + 4 + 3 * c], iz = scache[15 * e + 5 + 3 * c];
-    const double* F = c == 0 ? ut : c == 1 ? vt : c == 2 ? wt : p;
-    const int a0 = ix - (c == 0), b0 = iy - (c == 1), c0 = iz - (c == 2);
-    double f[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) f[r] = F[d.at(a0 + (r & 1), b0 + ((r >> 1) & 1), c0 + (r >> 2))];
-    double pe[4];
-    probe_eval(f, sc.X, sc.Y, sc.Z, ix, iy, iz, px, py, pz, pe);
-    const double dn_e = pe[1] * ca + pe[2] * cb + pe[3] * cg;
-    if (c < 3) {
-      dnds[c] = (2.0 / diagdis) * (pe[0] - 0.0) - dn_e;                // :195, :260, :324
-    } else {
-      const double a3 = surf[6 * ne + e], b3 = surf[7 * ne + e], g3 = surf[8 * ne + e];
-      const double alen = sqrt((a3 * a3 + b3 * b3) + g3 * g3);         // :327-331
-      const double area = alen / 2.0;
-      const double dot = dnds[0] * ca + dnds[1] * cb + dnds[2] * cg;
-      const double stx1 = dnds[0] - dot * ca;                         // :335-337
-      const double sty1 = dnds[1] - dot * cb;
-      const double dpdn = 0.0;
-      const double cval = pe[0] - (dn_e + dpdn) * diagdis * 0.5;      // :415
-      const double f_surf = cval * area;
-      contrib[0 * ne + e] = inv_re * stx1 * area;                     // shear_x_force :341
-      contrib[1 * ne + e] = -f_surf * ca;                             // f_surf_x :421
-      contrib[2 * ne + e] = inv_re * sty1 * area;                     // shear_y_force :343
-      contrib[3 * ne + e] = -f_surf * cb;                             // f_surf_y :423
-      contrib[4 * ne + e] = area;
-      contrib[5 * ne + e] = 0.5 * fabs(b3);                           // area_xz :330
-      contrib[6 * ne + e] = 0.5 * fabs(a3);                           // area_yz :329
+    for (int a = 0; a < 3; ++a) {
+      br[a] = bracket(A[a], 2, nn[a] + 1, ppos[a]);                     // e.g. :135-145
+      if (!br[a]) { if (active) atomicExch(err, 1); br[a] = 2; }
+      if (active) scache[15 * e + 3 + 3 * c + a] = br[a];
     }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) br[a] = scache[15 * e + 3 + 3 * c + a];
+  }
+  const double* F = c == 0 ? ut : c == 1 ? vt : c == 2 ? wt : p;
+  const int a0 = br[0] - (c == 0), b0 = br[1] - (c == 1), c0 = br[2] - (c == 2);
+  double f[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) f[r] = F[d.at(a0 + (r & 1), b0 + ((r >> 1) & 1), c0 + (r >> 2))];
+  double pe[4];
+  probe_eval(f, sc.X, sc.Y, sc.Z, br[0], br[1], br[2], px, py, pz, pe);
+  const double dn_e = pe[1] * ca + pe[2] * cb + pe[3] * cg;
+  const double dn = (2.0 / diagdis) * (pe[0] - 0.0) - dn_e;             // :195, :260, :324 (threads 0..2)
+  const double dnds[3] = {__shfl_sync(0xffffffffu, dn, lead), __shfl_sync(0xffffffffu, dn, lead + 1),
+                          __shfl_sync(0xffffffffu, dn, lead + 2)};
+  if (active && c == 3) {
+    const double a3 = surf[6 * ne + e], b3 = surf[7 * ne + e], g3 = surf[8 * ne + e];
+    const double alen = sqrt((a3 * a3 + b3 * b3) + g3 * g3);           // :327-331
+    const double area = alen / 2.0;
+    const double dot = dnds[0] * ca + dnds[1] * cb + dnds[2] * cg;
+    const double stx1 = dnds[0] - dot * ca;                           // :335-337
+    const double sty1 = dnds[1] - dot * cb;
+    const double dpdn = 0.0;
+    const double cval = pe[0] - (dn_e + dpdn) * diagdis * 0.5;        // :415
+    const double f_surf = cval * area;
+    contrib[0 * ne + e] = inv_re * stx1 * area;                       // shear_x_force :341
+    contrib[1 * ne + e] = -f_surf * ca;                               // f_surf_x :421
+    contrib[2 * ne + e] = inv_re * sty1 * area;                       // shear_y_force :343
+    contrib[3 * ne + e] = -f_surf * cb;                               // f_surf_y :423
+    contrib[4 * ne + e] = area;
+    contrib[5 * ne + e] = 0.5 * fabs(b3);                             // area_xz :330
+    contrib[6 * ne + e] = 0.5 * fabs(a3);                             // area_yz :329
   }
 }
 
+__device__ __forceinline__ void stress_coefficients(const double* s, double* coef) {
+  const double area_Sx = 0.5 * s[5], area_Sy = 0.5 * s[6];
+  coef[0] = 2.0 * (s[0] / area_Sx);
+  coef[1] = 2.0 * (s[1] / area_Sy);
+  coef[2] = 2.0 * (s[2] / area_Sy);
+  coef[3] = 2.0 * (s[3] / area_Sx);
+}
+
 // Element-order sums (the serial order of the reference's loop, so the sums are
-// bit-identical to the oracle) and the coefficients (subStressCal1.f90:428-450).
-__global__ void k_stress_sum(const double* __restrict__ contrib, int ne, double* coef) {
+// bit-identical to the oracle) and the coefficients (subStressCal1.f90:428-450). A sum is
+// one chain of FP64 additions, about 85 cycles each on this part: 0.21 ms for 5,120
+// elements; the block brings the terms into shared memory ahead of the seven adding threads.
+constexpr int kSumTile = 256, kSumThreads = 256;
+__global__ void __launch_bounds__(kSumThreads) k_stress_sum(const double* __restrict__ contrib, int ne, double* coef) {
+  __shared__ double tile[2][7][kSumTile + 1];   // the seven rows in different banks
   __shared__ double s[7];
-  if (threadIdx.x < 7) {
-    const double* c = contrib + (long long)threadIdx.x * ne;
-    double acc = 0.0;
-    for (int e = 0; e < ne; ++e) acc = acc + c[e];
-    s[threadIdx.x] = acc;
+  const int t = threadIdx.x;
+  auto fetch = [&](int base, double (&v)[7]) {
+#pragma unroll
+    for (int q = 0; q < 7; ++q) v[q] = base + t < ne ? contrib[(long long)q * ne + base + t] : 0.0;
+  };
+  double v[7], acc = 0.0;
+  fetch(0, v);
+  int buf = 0;
+  for (int base = 0; base < ne; base += kSumTile, buf ^= 1) {
+#pragma unroll
+    for (int q = 0; q < 7; ++q) tile[buf][q][t] = v[q];
+    __syncthreads();
+    if (base + kSumTile < ne) fetch(base + kSumTile, v);
+    if (t < 7) {
+      const double* c = tile[buf][t];
+      const int cnt = min(kSumTile, ne - base);
+#pragma unroll 16
+      for (int e = 0; e < cnt; ++e) acc = acc + c[e];
+    }
+  }
+  if (t < 7) s[t] = acc;
+  __syncthreads();
+  if (t == 0) stress_coefficients(s, coef);
+}
+
+// The same sums in a fixed tree order, for the forms whose results may differ from the
+// reference's arithmetic by rounding (IB3D_PREC_FP32DC, IB3D_PREC_FP64_FAST).
+constexpr int kTreeThreads = 512;
+__global__ void __launch_bounds__(kTreeThreads) k_stress_sum_tree(const double* __restrict__ contrib, int ne, double* coef) {
+  __shared__ double w[7][kTreeThreads / 32], s[7];
+  const int t = threadIdx.x;
+  double a[7] = {};
+  for (int e = t; e < ne; e += kTreeThreads)
+#pragma unroll
+    for (int q = 0; q < 7; ++q) a[q] += contrib[(long long)q * ne + e];
+#pragma unroll
+  for (int q = 0; q < 7; ++q) {
+    for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
+    if ((t & 31) == 0) w[q][t >> 5] = a[q];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double area_Sx = 0.5 * s[5], area_Sy = 0.5 * s[6];
-    coef[0] = 2.0 * (s[0] / area_Sx);
-    coef[1] = 2.0 * (s[1] / area_Sy);
-    coef[2] = 2.0 * (s[2] / area_Sy);
-    coef[3] = 2.0 * (s[3] / area_Sx);
+  if (t < 32) {
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      double x = t < kTreeThreads / 32 ? w[q][t] : 0.0;
+      for (int o = kTreeThreads / 64; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (t == 0) s[q] = x;
+    }
+    if (t == 0) stress_coefficients(s, coef);
   }
 }
 
@@ -1208,7 +1267,7 @@ int run_velocity_forcing(ib3d_ctx* c) {
   for (int l = 0; l < s.nlevels; ++l) {
     const int off = s.level_off[l], cnt = s.level_off[l + 1] - off;
     if (cnt <= 0) continue;
-    k_force_vel<<<nblk(cnt), kBlock, 0, c->st>>>(c->g, s.ordered ? s.order : nullptr, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
+    k_force_vel<<<nblk(cnt, 64), 64, 0, c->st>>>(c->g, s.ordered ? s.order : nullptr, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
                                                  c->nib, (int)c->nelems, s.brk, s.rd_idx, s.rd_src, c->ut, c->vt,
                                                  c->wt, c->motion, s.out);
   }
@@ -1227,7 +1286,7 @@ int run_pressure_forcing(ib3d_ctx* c) {
   for (int l = 0; l < s.nlevels; ++l) {
     const int off = s.level_off[l], cnt = s.level_off[l + 1] - off;
     if (cnt <= 0) continue;
-    k_force_p<<<nblk(cnt), kBlock, 0, c->st>>>(c->g, s.ordered ? s.order : nullptr, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
+    k_force_p<<<nblk(cnt, 64), 64, 0, c->st>>>(c->g, s.ordered ? s.order : nullptr, off, cnt, c->d_iblist, c->d_nelp, c->d_nd, c->d_surf,
                                                c->nib, (int)c->nelems, s.brk, s.rd_idx, s.rd_src, c->p, c->motion,
                                                s.out);
   }
@@ -1244,9 +1303,10 @@ int run_stress(ib3d_ctx* c, int first, double coef[4]) {
   if (do_first) IB3D_CUDA(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->st));
   PhaseScope ps(c, PH_STRESS);
   c->launches += 2;
-  k_stress_elem<<<nblk(ne), kBlock, 0, c->st>>>(c->d, c->g, c->d_surf, ne, do_first, c->d_scache, c->ut, c->vt,
-                                                c->wt, c->p, 1.0 / c->prm.re, c->d_contrib, c->d_flag);
-  k_stress_sum<<<1, 32, 0, c->st>>>(c->d_contrib, ne, c->d_coef);
+  k_stress_elem<<<nblk(4ll * ne, 64), 64, 0, c->st>>>(c->d, c->g, c->d_surf, ne, do_first, c->d_scache, c->ut, c->vt,
+                                                      c->wt, c->p, 1.0 / c->prm.re, c->d_contrib, c->d_flag);
+  if (c->prm.precision == IB3D_PREC_FP64) k_stress_sum<<<1, kSumThreads, 0, c->st>>>(c->d_contrib, ne, c->d_coef);
+  else k_stress_sum_tree<<<1, kTreeThreads, 0, c->st>>>(c->d_contrib, ne, c->d_coef);
   IB3D_CUDA(c, cudaGetLastError());
   if (do_first) {
     int flag = 0;

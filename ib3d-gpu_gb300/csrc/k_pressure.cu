@@ -205,58 +205,133 @@ __global__ void __launch_bounds__(kBlock) k_correct(Dims d, Grid1D g, const doub
 }
 
 // velocityBC, active branch (subBoundaryConditions.f90:350-406): x faces (inlet
-// u = 1, v/w reflected; outlet zero gradient), then y and z faces (slip).
-__global__ void k_bc_x(Dims d, Grid1D g, double* ut, double* vt, double* wt, const double* __restrict__ u,
-                       const double* __restrict__ v, const double* __restrict__ w, const double* __restrict__ ucp,
-                       double deltat, int convective) {
-  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (unsigned)d.ny * (unsigned)d.nz) return;
-  const int j = (int)(tid % (unsigned)d.ny) + 2, k = (int)(tid / (unsigned)d.ny) + 2;
-  const int nx = d.nx;
-  ut[d.at(1, j, k)] = 1.0;
-  vt[d.at(1, j, k)] = -vt[d.at(2, j, k)];
-  wt[d.at(1, j, k)] = -wt[d.at(2, j, k)];
-  if (convective) {   // Orlanski (the commented :153-155), uc from calculateUc
-    const double uc = *ucp;
-    const long long a = d.at(nx + 1, j, k), b2 = d.at(nx + 2, j, k), a0 = d.at(nx, j, k);
-    ut[a] = u[a] - (deltat / g.dx[nx + 1]) * uc * (u[a] - u[a0]);
-    vt[b2] = -vt[a] + v[b2] + v[a] - (2.0 * deltat / g.dx[nx + 2]) * uc * (v[b2] - v[a]);
-    wt[b2] = -wt[a] + w[b2] + w[a] - (2.0 * deltat / g.dx[nx + 2]) * uc * (w[b2] - w[a]);
-  } else {            // zero gradient (:149-151)
-    ut[d.at(nx + 1, j, k)] = ut[d.at(nx, j, k)];
-    vt[d.at(nx + 2, j, k)] = vt[d.at(nx + 1, j, k)];
-    wt[d.at(nx + 2, j, k)] = wt[d.at(nx + 1, j, k)];
+// u = 1, v/w reflected; outlet zero gradient, or Orlanski, the commented :153-155, with uc
+// from calculateUc), then y and z faces (slip), in one launch of one thread per face cell:
+// the faces are some 10^4 values, so the pass costs its launches (three launches took 18 us
+// at 40x32x32, one takes 7).
+//
+// The reference runs the x faces, then y, then z. Where a later pass reads what an earlier
+// one wrote, the value is taken from its source: u at the outlet face (bc_outlet), v = 0 at
+// the high y face. Where an earlier pass reads what a later one overwrites -- v at the high
+// y face (j = ny+1) and w at the high z face (k = nz+1) -- the reader's thread also does the
+// write: x threads for i = 2 and nx+1, y threads for j = 2 and ny+1, and x threads of the
+// edges (j = 2 or ny+1, k = nz+1) do the y faces' work at i = 2 and nx+1 as well.
+__device__ __forceinline__ double bc_outlet(const Dims& d, const Grid1D& g, const double* ut, const double* u, double uc,
+                                            double deltat, int convective, int j, int k) {
+  if (!convective) return ut[d.at(d.nx, j, k)];
+  const long long a = d.at(d.nx + 1, j, k), a0 = d.at(d.nx, j, k);
+  return u[a] - (deltat / g.dx[d.nx + 1]) * uc * (u[a] - u[a0]);
+}
+
+__global__ void __launch_bounds__(128) k_bc(Dims d, Grid1D g, double* ut, double* vt, double* wt,
+                                            const double* __restrict__ u, const double* __restrict__ v,
+                                            const double* __restrict__ w, const double* __restrict__ ucp, double deltat,
+                                            int convective) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const unsigned nX = (unsigned)ny * (unsigned)nz, nY = (unsigned)nx * (unsigned)nz, nZ = (unsigned)nx * (unsigned)ny;
+  unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const double uc = convective ? *ucp : 0.0;
+  // slip at the low or the high y face of column (i, k)
+  auto y_low = [&](int i, int k) {
+    ut[d.at(i, 1, k)] = i == nx + 1 ? bc_outlet(d, g, ut, u, uc, deltat, convective, 2, k) : ut[d.at(i, 2, k)];
+    wt[d.at(i, 1, k)] = wt[d.at(i, 2, k)];
+    vt[d.at(i, 1, k)] = 0.0;
+  };
+  auto y_high = [&](int i, int k) {
+    ut[d.at(i, ny + 2, k)] = i == nx + 1 ? bc_outlet(d, g, ut, u, uc, deltat, convective, ny + 1, k) : ut[d.at(i, ny + 1, k)];
+    wt[d.at(i, ny + 2, k)] = wt[d.at(i, ny + 1, k)];
+  };
+  if (t < nX) {
+    const int j = (int)(t % (unsigned)ny) + 2, k = (int)(t / (unsigned)ny) + 2;
+    const long long b = d.at(2, j, k), a = d.at(nx + 1, j, k), c = d.at(nx + 2, j, k);
+    ut[d.at(1, j, k)] = 1.0;
+    vt[d.at(1, j, k)] = -vt[b];
+    wt[d.at(1, j, k)] = -wt[b];
+    ut[a] = bc_outlet(d, g, ut, u, uc, deltat, convective, j, k);
+    if (convective) {
+      vt[c] = -vt[a] + v[c] + v[a] - (2.0 * deltat / g.dx[nx + 2]) * uc * (v[c] - v[a]);
+      wt[c] = -wt[a] + w[c] + w[a] - (2.0 * deltat / g.dx[nx + 2]) * uc * (w[c] - w[a]);
+    } else {
+      vt[c] = vt[a];
+      wt[c] = wt[a];
+    }
+    if (k == nz + 1) {
+      if (j == 2) {
+        y_low(2, k);
+        y_low(nx + 1, k);
+      }
+      if (j == ny + 1) {
+        y_high(2, k);
+        y_high(nx + 1, k);
+      }
+      wt[b] = 0.0;
+      wt[a] = 0.0;
+    }
+    if (j == ny + 1) {
+      vt[b] = 0.0;
+      vt[a] = 0.0;
+    }
+  } else if ((t -= nX) < nY) {
+    const int i = (int)(t % (unsigned)nx) + 2, k = (int)(t / (unsigned)nx) + 2;
+    const bool end = i == 2 || i == nx + 1;
+    if (k == nz + 1 && end) return;   // an x thread's
+    y_low(i, k);
+    y_high(i, k);
+    if (k == nz + 1) {
+      wt[d.at(i, 2, k)] = 0.0;
+      wt[d.at(i, ny + 1, k)] = 0.0;
+    }
+    if (!end) vt[d.at(i, ny + 1, k)] = 0.0;
+  } else if ((t -= nY) < nZ) {
+    const int i = (int)(t % (unsigned)nx) + 2, j = (int)(t / (unsigned)nx) + 2;
+    const bool out = i == nx + 1;
+    ut[d.at(i, j, 1)] = out ? bc_outlet(d, g, ut, u, uc, deltat, convective, j, 2) : ut[d.at(i, j, 2)];
+    vt[d.at(i, j, 1)] = j == ny + 1 ? 0.0 : vt[d.at(i, j, 2)];
+    wt[d.at(i, j, 1)] = 0.0;
+    ut[d.at(i, j, nz + 2)] = out ? bc_outlet(d, g, ut, u, uc, deltat, convective, j, nz + 1) : ut[d.at(i, j, nz + 1)];
+    vt[d.at(i, j, nz + 2)] = j == ny + 1 ? 0.0 : vt[d.at(i, j, nz + 1)];
+    if (!(i == 2 || out) && j != 2 && j != ny + 1) wt[d.at(i, j, nz + 1)] = 0.0;
   }
 }
 
 // calculateUc (subCalculateuc.f90:2-38): uc = max(mean of ut(nx-4,j,k) over the
-// plane's fluid cells, 0). One warp; the sum runs in the serial order k outer, j
-// inner (lane 0 adds the warp's 32 loaded values one by one), so it matches a
-// serial build of the reference bit for bit.
-__global__ void k_calculate_uc(Dims d, const double* __restrict__ ut, const unsigned char* __restrict__ cell,
-                               double* ucp) {
-  const int lane = threadIdx.x;
-  const int i = d.nx - 4;
+// plane's fluid cells, 0). The sum runs in the serial order k outer, j inner, so it matches
+// a serial build of the reference bit for bit: one thread adds the values that the block
+// has brought into shared memory (0 for the other cells, which leaves the sum as it is:
+// it starts at +0 and never becomes -0), one chain of additions of about 85 cycles each
+// (0.77 ms became 0.31 at 97 x 75 plane cells). The order holds in every precision: uc
+// enters the velocities, and the FP32 sweeps carry one different rounding to 1e-9 of them.
+constexpr int kUcTile = 1024;
+__global__ void __launch_bounds__(kUcTile) k_calculate_uc(Dims d, const double* __restrict__ ut,
+                                                          const unsigned char* __restrict__ cell, double* ucp) {
+  __shared__ double tile[2][kUcTile];
+  __shared__ int fluid;
+  const int t = threadIdx.x, i = d.nx - 4, total = d.ny * d.nz;
+  if (t == 0) fluid = 0;
+  int mine = 0, buf = 0;
   double sum = 0.0;
-  long long count = 0;
-  for (int k = 2; k <= d.nz + 1; ++k)
-    for (int j0 = 2; j0 <= d.ny + 1; j0 += 32) {
-      const int j = j0 + lane;
-      double x = 0.0;
-      int fl = 0;
-      if (j <= d.ny + 1) {
-        const long long o = d.at(i, j, k);
-        fl = cell[o] == 0;
-        x = fl ? ut[o] : 0.0;
-      }
-      for (int l = 0; l < 32; ++l) {
-        const double xl = __shfl_sync(0xffffffffu, x, l);
-        const int fll = __shfl_sync(0xffffffffu, fl, l);
-        if (fll) { sum = sum + xl; ++count; }
+  for (int base = 0; base < total; base += kUcTile, buf ^= 1) {
+    const int q = base + t;
+    double x = 0.0;
+    if (q < total) {
+      const long long o = d.at(i, q % d.ny + 2, q / d.ny + 2);
+      if (cell[o] == 0) {
+        x = ut[o];
+        ++mine;
       }
     }
-  if (lane == 0) {
-    const double uc1 = sum / (double)count;
+    tile[buf][t] = x;
+    __syncthreads();
+    if (t == 0) {
+      const int cnt = min(kUcTile, total - base);
+#pragma unroll 16
+      for (int e = 0; e < cnt; ++e) sum = sum + tile[buf][e];
+    }
+  }
+  atomicAdd(&fluid, mine);
+  __syncthreads();
+  if (t == 0) {
+    const double uc1 = sum / (double)fluid;
     *ucp = uc1 > 0.0 ? uc1 : 0.0;
   }
 }
@@ -264,43 +339,30 @@ __global__ void k_calculate_uc(Dims d, const double* __restrict__ ut, const unsi
 void launch_calculate_uc(ib3d_ctx* c) {
   PhaseScope ps(c, PH_BC);
   c->launches += 1;
-  k_calculate_uc<<<1, 32, 0, c->st>>>(c->d, c->ut, c->cell, c->d_coef + 6);
+  k_calculate_uc<<<1, kUcTile, 0, c->st>>>(c->d, c->ut, c->cell, c->d_coef + 6);
 }
-__global__ void k_bc_y(Dims d, double* ut, double* vt, double* wt) {
-  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (unsigned)d.nx * (unsigned)d.nz) return;
-  const int i = (int)(tid % (unsigned)d.nx) + 2, k = (int)(tid / (unsigned)d.nx) + 2;
-  const int ny = d.ny;
-  ut[d.at(i, 1, k)] = ut[d.at(i, 2, k)];
-  wt[d.at(i, 1, k)] = wt[d.at(i, 2, k)];
-  vt[d.at(i, 1, k)] = 0.0;
-  ut[d.at(i, ny + 2, k)] = ut[d.at(i, ny + 1, k)];
-  wt[d.at(i, ny + 2, k)] = wt[d.at(i, ny + 1, k)];
-  vt[d.at(i, ny + 1, k)] = 0.0;
-}
-__global__ void k_bc_z(Dims d, double* ut, double* vt, double* wt) {
-  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (unsigned)d.nx * (unsigned)d.ny) return;
-  const int i = (int)(tid % (unsigned)d.nx) + 2, j = (int)(tid / (unsigned)d.nx) + 2;
-  const int nz = d.nz;
-  ut[d.at(i, j, 1)] = ut[d.at(i, j, 2)];
-  vt[d.at(i, j, 1)] = vt[d.at(i, j, 2)];
-  wt[d.at(i, j, 1)] = 0.0;
-  ut[d.at(i, j, nz + 2)] = ut[d.at(i, j, nz + 1)];
-  vt[d.at(i, j, nz + 2)] = vt[d.at(i, j, nz + 1)];
-  wt[d.at(i, j, nz + 1)] = 0.0;
-}
-
 // solidCellBC (subBoundaryConditions.f90:199-217), flag-masked.
-__global__ void k_solid_bc(Dims d, const unsigned char* __restrict__ cell, double* ut, double* vt, double* wt,
-                           double* p) {
-  const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (unsigned)d.n3) return;
-  if (cell[idx] != 1) return;
-  int i, j, k;
-  decode(d, idx, i, j, k);
-  if (!interior(d, i, j, k)) return;
-  ut[idx] = 0.0; vt[idx] = 0.0; wt[idx] = 0.0; p[idx] = 0.0;
+// Four flags per thread: nearly every cell is fluid, so the pass is one read of the flags
+// (a thread per cell with its index decoded took 24 us at 256x192x192).
+__global__ void __launch_bounds__(kBlock) k_solid_bc(Dims d, const unsigned char* __restrict__ cell, double* ut,
+                                                     double* vt, double* wt, double* p) {
+  const long long q = ((long long)blockIdx.x * kBlock + threadIdx.x) * 4;
+  if (q >= d.n3) return;
+  unsigned f = 0;
+  if (q + 4 <= d.n3) {
+    f = *reinterpret_cast<const unsigned*>(cell + q);
+  } else {
+    for (int n = 0; q + n < d.n3; ++n) f |= (unsigned)cell[q + n] << (8 * n);
+  }
+  if (f == 0) return;
+  for (int n = 0; n < 4; ++n) {
+    if ((f >> (8 * n) & 255u) != 1u) continue;
+    const unsigned idx = (unsigned)(q + n);
+    int i, j, k;
+    decode(d, idx, i, j, k);
+    if (!interior(d, i, j, k)) continue;
+    ut[idx] = 0.0; vt[idx] = 0.0; wt[idx] = 0.0; p[idx] = 0.0;
+  }
 }
 
 // Steady-state indicator derrStdSt = max |ut-u|/dt (subPcorVcor.f90:45-58) over fluid
@@ -375,19 +437,17 @@ void launch_correct(ib3d_ctx* c) {
 
 void launch_velocity_bc(ib3d_ctx* c) {
   PhaseScope ps(c, PH_BC);
-  c->launches += 3;
+  c->launches += 1;
   const Dims& d = c->d;
-  k_bc_x<<<nblocks((long long)d.ny * d.nz), kBlock, 0, c->st>>>(d, c->g, c->ut, c->vt, c->wt, c->u, c->v, c->w,
-                                                                 c->d_coef + 6, c->prm.deltat,
-                                                                 c->prm.outlet == IB3D_OUTLET_CONVECTIVE ? 1 : 0);
-  k_bc_y<<<nblocks((long long)d.nx * d.nz), kBlock, 0, c->st>>>(d, c->ut, c->vt, c->wt);
-  k_bc_z<<<nblocks((long long)d.nx * d.ny), kBlock, 0, c->st>>>(d, c->ut, c->vt, c->wt);
+  const long long n = (long long)d.ny * d.nz + (long long)d.nx * d.nz + (long long)d.nx * d.ny;
+  k_bc<<<(unsigned)((n + 127) / 128), 128, 0, c->st>>>(d, c->g, c->ut, c->vt, c->wt, c->u, c->v, c->w, c->d_coef + 6,
+                                                       c->prm.deltat, c->prm.outlet == IB3D_OUTLET_CONVECTIVE ? 1 : 0);
 }
 
 void launch_solid_bc(ib3d_ctx* c) {
   PhaseScope ps(c, PH_BC);
   c->launches += 1;
-  k_solid_bc<<<nblocks(c->d.n3), kBlock, 0, c->st>>>(c->d, c->cell, c->ut, c->vt, c->wt, c->p);
+  k_solid_bc<<<nblocks((c->d.n3 + 3) / 4), kBlock, 0, c->st>>>(c->d, c->cell, c->ut, c->vt, c->wt, c->p);
 }
 
 void launch_dss_copy(ib3d_ctx* c) {
