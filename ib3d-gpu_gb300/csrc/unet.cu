@@ -49,6 +49,7 @@ struct Buffers {
   bf16 *p1, *a2, *cat4, *a4, *d2;
   bf16 *g_p1, *g_a2, *g_cat4, *g_a4, *g_d2;
   // level 3
+  float* work;   // partial sums of the weight gradients
   bf16 *p2, *a3, *b;
   bf16 *g_p2, *g_a3, *g_b;
 };
@@ -71,6 +72,8 @@ struct ib3d_net {
   long long cap = 0, count = 0;
   bf16* ds_in = nullptr;   // [patch][S^3][4]
   float* ds_t = nullptr;   // [patch][S^3]
+  float* x = nullptr;      // inputs of ib3d_net_loss_grad on the device, room for x_cap voxels
+  long long x_cap = 0;
   double* d_loss = nullptr;
   int* d_err = nullptr;    // set by a convolution whose tensor-core wait gave up
   bool wgrad_cuda_cores = false;   // weight gradients on the CUDA cores (the tensor-core form's reference)
@@ -133,6 +136,13 @@ int ensure_buffers(ib3d_net* n, const Vol& v1, bool grads) {
          alloc_bf(&b.g_a2, m2, 32) && alloc_bf(&b.g_cat4, m2, 96) && alloc_bf(&b.g_a4, m2, 32) &&
          alloc_bf(&b.g_d2, m2, 32) && alloc_bf(&b.g_p2, m3, 32) && alloc_bf(&b.g_a3, m3, 64) &&
          alloc_bf(&b.g_b, m3, 64);
+  if (ok && grads) {
+    const int level[kL] = {1, 1, 2, 2, 3, 3, 2, 2, 1, 1};
+    size_t most = 1;
+    for (int l = 0; l < kL; ++l)
+      most = std::max(most, wgrad_workspace(level[l] == 1 ? b.v1 : level[l] == 2 ? b.v2 : b.v3, kN[l], kK[l]));
+    ok = alloc_f(&b.work, (long long)most);
+  }
   if (!ok) {
     free_buffers(b);
     return fail(n, IB3D_ERR_MEMORY, "ib3d_net: activation buffers");
@@ -171,17 +181,16 @@ void forward(ib3d_net* n) {
 void conv_bwd(ib3d_net* n, int l, const Vol& v, Act X, Act Y, Act gY, Act gX) {
   const Layer& ly = n->L[l];
   const long long M = v.voxels();
-  relu_bwd(n->st, M, ly.N, gY, Y);
-  bias_grad(n->st, M, gY, ly.N, n->g + ly.b);
+  relu_bias_bwd(n->st, M, ly.N, gY, Y, n->g + ly.b);
   if (n->wgrad_cuda_cores) wgrad_cuda_cores(n->st, v, gY, ly.N, X, ly.K, n->g + ly.w);
-  else wgrad(n->st, v, gY, ly.N, X, ly.K, n->g + ly.w, n->d_err);
+  else wgrad(n->st, v, gY, ly.N, X, ly.K, n->g + ly.w, n->buf.work, n->d_err);
   if (gX.p) conv(n->st, v, gY, ly.N, wt(n, l), nullptr, 0, -1, gX, ly.K, n->d_err);
 }
 
 void backward(ib3d_net* n) {
   Buffers& b = n->buf;
   cudaStream_t st = n->st;
-  head_bwd(st, b.v1.voxels(), 16, A(b.d1, 16), n->p + n->head, b.gout, A(b.g_d1, 16), n->g + n->head);
+  head_bwd(st, b.v1.voxels(), A(b.d1, 16), n->p + n->head, b.gout, A(b.g_d1, 16), n->g + n->head);
   conv_bwd(n, 9, b.v1, A(b.a5, 16), A(b.d1, 16), A(b.g_d1, 16), A(b.g_a5, 16));
   conv_bwd(n, 8, b.v1, A(b.cat5, 48), A(b.a5, 16), A(b.g_a5, 16), A(b.g_cat5, 48));
   up_bwd(st, b.v2, 32, A(b.g_cat5, 48, 0), A(b.g_d2, 32));
@@ -346,7 +355,10 @@ __global__ void k_gather(long long per, int B, const int* __restrict__ ids, cons
 __global__ void k_set_input(long long M, const float* __restrict__ x, bf16* __restrict__ in0) {
   const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
-  for (int c = 0; c < kInputs; ++c) in0[m * 16 + c] = __float2bfloat16(x[m * kInputs + c]);
+  static_assert(kInputs == 4, "one 16-byte load and one 8-byte store");
+  const float4 v = reinterpret_cast<const float4*>(x)[m];
+  const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+  *reinterpret_cast<uint2*>(in0 + m * 16) = *reinterpret_cast<const uint2*>(h);
 }
 
 }  // namespace
@@ -438,7 +450,7 @@ void ib3d_net_destroy(ib3d_net* n) {
   if (!n) return;
   if (n->st) cudaStreamSynchronize(n->st);
   free_buffers(n->buf);
-  void* ptrs[] = {n->p, n->g, n->m1, n->m2, n->wf, n->wt, n->ds_in, n->ds_t, n->d_loss, n->d_err};
+  void* ptrs[] = {n->p, n->g, n->m1, n->m2, n->wf, n->wt, n->ds_in, n->ds_t, n->x, n->d_loss, n->d_err};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (n->st) cudaStreamDestroy(n->st);
@@ -472,8 +484,14 @@ int ib3d_net_loss_grad(ib3d_net* n, int B, int S, const float* x, const float* t
   int rc = ensure_buffers(n, v, true);
   if (rc) return rc;
   const long long M = v.voxels();
-  float* dx = nullptr;
-  NET_CUDA(n, cudaMalloc(&dx, (size_t)M * kInputs * sizeof(float)));
+  if (M > n->x_cap) {   // room kept for the next batch
+    cudaFree(n->x);
+    n->x = nullptr;
+    n->x_cap = 0;
+    NET_CUDA(n, cudaMalloc(&n->x, (size_t)M * kInputs * sizeof(float)));
+    n->x_cap = M;
+  }
+  float* dx = n->x;
   cudaMemcpyAsync(dx, x, (size_t)M * kInputs * sizeof(float), cudaMemcpyHostToDevice, n->st);
   cudaMemcpyAsync(n->buf.tgt, target, (size_t)M * sizeof(float), cudaMemcpyHostToDevice, n->st);
   k_set_input<<<(unsigned)((M + 255) / 256), 256, 0, n->st>>>(M, dx, n->buf.in0);
@@ -486,7 +504,6 @@ int ib3d_net_loss_grad(ib3d_net* n, int B, int S, const float* x, const float* t
   if (grad) cudaMemcpyAsync(grad, n->g, n->nparam * sizeof(float), cudaMemcpyDeviceToHost, n->st);
   if (out) cudaMemcpyAsync(out, n->buf.out, (size_t)M * sizeof(float), cudaMemcpyDeviceToHost, n->st);
   NET_CUDA(n, cudaStreamSynchronize(n->st));
-  cudaFree(dx);
   NET_CUDA(n, cudaGetLastError());
   return check_conv(n);
 }
