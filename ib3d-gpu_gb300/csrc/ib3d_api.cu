@@ -202,6 +202,47 @@ void fast_tables(const std::vector<double>& d, int n, int axis, const std::vecto
   }
 }
 
+// 1-D tables of the reference-arithmetic predictor (k_momentum.cu lists them): every quotient of
+// nsMomentum in which both terms depend only on the grid, evaluated as the reference does,
+// and the divisors that depend only on the grid with their reciprocals in two parts.
+void exact_tables(const std::vector<double>& d, int n, int axis, const std::vector<double> cc[6][12], int S,
+                  std::vector<double>& out) {
+  auto put = [&](int t, int m, double v) { out[(size_t)(axis * kExactTables + t) * S + m] = v; };
+  auto divisor = [&](int t, int m, double b) {
+    const bool ok = std::isfinite(b) && std::fabs(b) > 0x1p-200 && std::fabs(b) < 0x1p200;
+    const double zh = ok ? 1.0 / b : std::nan("");
+    put(t, m, b);
+    put(t + 1, m, zh);
+    put(t + 2, m, ok ? std::fma(-zh, b, 1.0) / b : 0.0);
+  };
+  for (int m = 2; m <= n + 1; ++m) {
+    const double dm = d[m], dp = d[m + 1], dl = d[m - 1];
+    const double hp = 0.5 * (dm + dp), hl = 0.5 * (dm + dl);
+    put(0, m, dp / (dm + dp));
+    put(1, m, 2.0 / (dm + dp));
+    put(2, m, 2.0 / (0.5 * ((dm + dp) + (dm + dl))));
+    divisor(3, m, dp);
+    divisor(6, m, dm);
+    divisor(9, m, hp);
+    divisor(12, m, hl);
+    divisor(15, m, cc[axis][5][m] * dp);
+    divisor(18, m, 2.0 * cc[axis][11][m] * dm);
+    divisor(21, m, cc[3 + axis][5][m] * hp);
+    divisor(24, m, 2.0 * cc[3 + axis][11][m] * hl);
+    for (int f = 0; f < 2; ++f) {
+      const double r = f == 0 ? dm / dp : hl / hp, dA = f == 0 ? dp : hp;
+      const int b = 27 + 7 * f;
+      put(b + 0, m, -1.0 / (r * (r + 1.0)));
+      put(b + 1, m, 1.0 - 1.0 / r);
+      put(b + 2, m, r / (r + 1.0));
+      put(b + 3, m, 1.0 / (2.0 * dA));
+      put(b + 4, m, 2.0 / (r * (r + 1.0)));
+      put(b + 5, m, 2.0 / r);
+      put(b + 6, m, 2.0 / (r + 1.0));
+    }
+  }
+}
+
 struct Packer {
   std::vector<double> host;
   std::vector<std::pair<const double**, size_t>> fix;
@@ -491,6 +532,16 @@ int ib3d_create(ib3d_ctx** out, const ib3d_params* prm, int64_t nx, int64_t ny, 
     if (!rc && cudaMemcpy(c->d_fast, ft.data(), ft.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
       rc = IB3D_ERR_CUDA;
   }
+  if (!rc) {
+    const int S = c->fast_stride;
+    std::vector<double> et((size_t)3 * kExactTables * S, 0.0);
+    exact_tables(c->hdx, (int)nx, 0, c->hcc, S, et);
+    exact_tables(c->hdy, (int)ny, 1, c->hcc, S, et);
+    exact_tables(c->hdz, (int)nz, 2, c->hcc, S, et);
+    if (cudaMalloc(&c->d_exact, et.size() * sizeof(double)) != cudaSuccess) rc = IB3D_ERR_MEMORY;
+    if (!rc && cudaMemcpy(c->d_exact, et.data(), et.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+      rc = IB3D_ERR_CUDA;
+  }
   if (!rc) rc = alloc_fields(c);
   if (!rc) rc = ensure_resi(c, prm->momentum == IB3D_MOMENTUM_AB2);
   if (!rc) rc = ib3d_set_params(c, prm);
@@ -509,7 +560,7 @@ void ib3d_destroy(ib3d_ctx* c) {
   timer_fold(c);
   for (cudaEvent_t e : c->pool) cudaEventDestroy(e);
   free_ib(c);
-  void* ptrs[] = {c->d_tables, c->d_tables32, c->d_fast, c->d_axp, c->u, c->v, c->w, c->ut, c->vt, c->wt, c->p, c->pc, c->b, c->bdt,
+  void* ptrs[] = {c->d_tables, c->d_tables32, c->d_fast, c->d_exact, c->d_axp, c->u, c->v, c->w, c->ut, c->vt, c->wt, c->p, c->pc, c->b, c->bdt,
                   c->e32, c->r32, c->ep[0], c->ep[1], c->rp[0], c->rp[1], c->cell, c->ibmap, c->ctl, c->d_nodes, c->d_tri, c->d_surf, c->d_c32, c->d_c32_max, c->d_levels, c->d_iblist,
                   c->d_nelp, c->d_nd, c->d_minel, c->d_scache, c->d_contrib, c->d_coef, c->d_flag, c->d_scan,
                   c->hist[0], c->hist[1], c->r_hist, c->d_norm, c->d_norm_part, c->resi[0], c->resi[1], c->resi[2],

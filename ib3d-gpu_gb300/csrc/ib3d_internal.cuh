@@ -22,6 +22,7 @@
 namespace ib3d {
 
 constexpr int kBlock = 256;
+constexpr int kExactTables = 41;  // 1-D tables per axis of the reference-arithmetic predictor (k_momentum.cu)
 constexpr int kFastTables = 46;   // 1-D tables per axis of the fast kernels (k_momentum_fast.cu, k_fast.cu)
 
 // Index helpers: 1-based Fortran (i,j,k) into the padded column-major array.
@@ -153,6 +154,7 @@ struct ib3d_ctx {
   double* d_tables = nullptr;  // all 1-D FP64 tables in one allocation
   double* d_fast = nullptr;    // 3 x kFastTables 1-D tables of the fast momentum kernel
   int fast_stride = 0;
+  double* d_exact = nullptr;   // 3 x kExactTables 1-D tables of the reference-arithmetic predictor
   float* d_tables32 = nullptr;
   float* d_axp = nullptr;      // grouped x coefficients of the colour-packed sweep
   ib3d::Grid1D g{};
@@ -385,6 +387,30 @@ __device__ __forceinline__ void block_max_atomic(double v, unsigned long long* s
   }
 }
 __device__ __forceinline__ double bits_to_double(unsigned long long b) { return __longlong_as_double((long long)b); }
+
+// A divisor known in advance: b, zh = 1/b rounded and zl the rest of 1/b. zh is NaN where b is
+// not of a size that div_known takes (the division itself is used then).
+struct KnownDiv {
+  double b, zh, zl;
+};
+// a / b, correctly rounded: a (zh + zl) is within half an ulp and 2^-100 of the quotient, so
+// its remainder is exact and one more fused step rounds correctly (Markstein, IBM J. Res.
+// Dev. 34, 1990; known divisors: Brisebarre, Muller and Raina, IEEE Trans. Comput. 53, 2004).
+// Four FP64 operations instead of a division's nine. |b| lies within 2^+-200; numerators so
+// small or large that a step could leave the normal range, infinities and NaN take the
+// division itself, and a zero numerator its signed zero.
+__device__ __forceinline__ double div_known(double a, double b, double zh, double zl) {
+  const int ha = __double2hiint(a);
+  const unsigned ex = ((unsigned)ha >> 20) & 0x7ffu;
+  if (ex - 323u < 1400u && (__double2hiint(zh) & 0x7ff00000) != 0x7ff00000) {
+    const double q = fma(a, zh, a * zl);
+    return fma(fma(-b, q, a), zh, q);
+  }
+  if (((ha & 0x7fffffff) | __double2loint(a)) == 0 && (__double2hiint(zh) & 0x7ff00000) != 0x7ff00000)
+    return __hiloint2double((ha ^ __double2hiint(b)) & (int)0x80000000, 0);
+  return a / b;
+}
+__device__ __forceinline__ double div_known(double a, const KnownDiv& d) { return div_known(a, d.b, d.zh, d.zl); }
 
 // The finishing step shared by every kernel that ends a sweep or a check: the
 // last block to retire reads the accumulated maximum, applies the stopping test

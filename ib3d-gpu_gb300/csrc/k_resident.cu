@@ -55,21 +55,6 @@ __device__ __forceinline__ int ld_flag(const int* p) {
 }
 __device__ __forceinline__ float4 ld4s(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// a / b, correctly rounded, for a divisor known in advance: zh = 1/b rounded, zl the rest
-// of 1/b. a (zh + zl) is within half an ulp and 2^-100 of the quotient, so its remainder
-// is exact and one more fused step rounds correctly (Markstein, IBM J. Res. Dev. 34, 1990;
-// known divisors: Brisebarre, Muller and Raina, IEEE Trans. Comput. 53, 2004). Numerators
-// so small or large that a step could leave the normal range, zeros, infinities and NaN
-// take the division itself; |b| lies within 2^+-200 (plain_diagonal).
-__device__ __forceinline__ double div_known(double a, double b, double zh, double zl) {
-  const unsigned ex = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
-  if (ex - 323u < 1400u) {
-    const double q = fma(a, zh, a * zl);
-    return fma(fma(-b, q, a), zh, q);
-  }
-  return a / b;
-}
-
 __device__ __forceinline__ u64 tagged(unsigned bits, unsigned seq) { return ((u64)seq << 32) | bits; }
 
 // The rows of this block: [j0, j0 + nyb) x [k0, k0 + nzb).
