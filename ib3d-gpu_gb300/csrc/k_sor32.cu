@@ -19,6 +19,7 @@
 // in k_pressure.cu), so both give the same bits.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 
 #include "ib3d_internal.cuh"
@@ -29,6 +30,22 @@ namespace ib3d {
 // Row length of a packed colour array: the row's cells rounded up to whole float4
 // groups, plus 4 entries of left padding (ghost at 3) and 4 of right padding.
 int packed_row_length(int nx) { return 4 * row_groups(nx) + 8; }
+
+// Loads that the compiler may move over the kernels' stores: a thread loads an own value
+// before it stores it, and the other arrays are not written by the pass. They must not
+// become .nc loads, as loads through const __restrict__ pointers do: a pass may start while
+// the last one runs, griddepcontrol.wait orders ordinary loads only, and with .nc loads values of
+// an earlier pass came back from L1 (wrong results, depending on the timing).
+__device__ __forceinline__ float4 ld4(const float* p) {
+  float4 v;
+  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld1(const float* p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
 
 // One colour pass. Block (32, kRows): a warp covers 32 float4 groups of one row
 // (j, k), so the row's colour phase is uniform across the warp; grid (ceil(nq/32),
@@ -55,12 +72,12 @@ constexpr int kPlanes = 8;
 constexpr int kRows = 4;
 
 template <int COLOR, bool ALL_LOAD>
-__global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, const float* __restrict__ r_own,
-                                                          float* __restrict__ e_own, const float* __restrict__ e_oth,
+__global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, const float* r_own, float* e_own,
+                                                          const float* e_oth,
                                                           int Lp, float omega, float om1) {
   // launched with programmatic dependent launch: the blocks may start while the
   // previous pass drains; wait for it (and its writes) before touching memory
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" : "+l"(r_own), "+l"(e_own), "+l"(e_oth) : : "memory");
   const int nq = row_groups(d.nx);
   const int lane = threadIdx.x;
   const int q = blockIdx.x * 32 + lane;
@@ -75,8 +92,8 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
     const int sj = (j - 1) * Lp + 4 * qa + 4;
     const float ay0 = g.acy32[0][j - 1], ay1 = g.acy32[1][j - 1], ay2 = g.acy32[2][j - 1];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 ob = lds ? *reinterpret_cast<const float4*>(e_oth + (k0 - 2) * plane + sj) : z4;
-    float4 ox = lds ? *reinterpret_cast<const float4*>(e_oth + (k0 - 1) * plane + sj) : z4;
+    float4 ob = lds ? ld4(e_oth + (k0 - 2) * plane + sj) : z4;
+    float4 ox = lds ? ld4(e_oth + (k0 - 1) * plane + sj) : z4;
 #pragma unroll
     for (int kk = 0; kk < kPlanes; ++kk) {
       const int k = k0 + kk;
@@ -86,16 +103,16 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
       const bool own_first = (COLOR == 0) == (((j + k) & 1) == 1);
       float4 rr = z4, eo = z4, os = z4, on = z4, ot = z4;
       if (lds) {
-        rr = *reinterpret_cast<const float4*>(r_own + s0);
-        eo = *reinterpret_cast<const float4*>(e_own + s0);
-        os = *reinterpret_cast<const float4*>(e_oth + s0 - Lp);
-        on = *reinterpret_cast<const float4*>(e_oth + s0 + Lp);
-        ot = *reinterpret_cast<const float4*>(e_oth + s0 + plane);
+        rr = ld4(r_own + s0);
+        eo = ld4(e_own + s0);
+        os = ld4(e_oth + s0 - Lp);
+        on = ld4(e_oth + s0 + Lp);
+        ot = ld4(e_oth + s0 + plane);
       }
       float left = __shfl_up_sync(0xffffffffu, ox.w, 1);
       float right = __shfl_down_sync(0xffffffffu, ox.x, 1);
-      if (lds && load_left) left = e_oth[s0 - 1];
-      if (lds && load_right) right = e_oth[s0 + 4];
+      if (lds && load_left) left = ld1(e_oth + s0 - 1);
+      if (lds && load_right) right = ld1(e_oth + s0 + 4);
       const float oxa[6] = {left, ox.x, ox.y, ox.z, ox.w, right};
       const float rv[4] = {rr.x, rr.y, rr.z, rr.w};
       const float sv[4] = {os.x, os.y, os.z, os.w};
@@ -133,10 +150,16 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
 // Lanes run through the groups of all row pairs without a break at a row's end, so no
 // lane idles whatever nx is (a warp per 32 groups of one row left 25 % of the lanes idle
 // at nx = 384 and 41 % at 300: 72.6 against 82.8 us per sweep at 384x256x256); at a row's
-// end the x neighbour is the ghost entry, 0. Row b may be the top ghost row (odd ny): its
-// other-colour values (zero) are read as row a's neighbours, and its own update is
-// neither loaded nor stored. Per cell the arithmetic is update4's, so the bits are those
-// of k_sor32p.
+// end the x neighbour is the ghost entry, 0. Per cell the arithmetic is update4's, so the
+// bits are those of k_sor32p.
+//
+// No load depends on a predicate: a lane beyond the rows repeats the last pair, row b may be
+// the top ghost row (odd ny) and a slab's last plane the top ghost plane; what is computed
+// there is dropped. A plane's loads then start together and before the last plane's
+// stores, and eight planes are unrolled: 16.2 -> 15.3 us per sweep at 256x192x192 (with
+// guarded loads the sweep waited on one plane after the other). WHOLE: the pairs fill the
+// blocks and the planes the slabs, which takes the clamps out too: 14.6 us there, 14.3
+// against 15.0 at 256x224x160.
 //
 // STREAM, for arrays that do not fit in L2: the right-hand side, read once a pass and not
 // again until the pass after next, is loaded past L1 and first to leave L2, so that L2
@@ -148,10 +171,9 @@ constexpr int kRows2 = 4;
 constexpr int kUnroll2 = 8;
 static_assert(kUnroll2 % 2 == 0, "the row phases alternate with the planes");
 
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 ld4_stream(const float* p, unsigned long long pol) {
   float4 v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+  asm("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
       : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
   return v;
 }
@@ -161,103 +183,101 @@ __device__ __forceinline__ unsigned long long evict_first_policy() {
   return pol;
 }
 
-template <int COLOR, bool STREAM, bool DOWN>
-__global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, const float* __restrict__ r_own,
-                                                            float* __restrict__ e_own, const float* __restrict__ e_oth,
-                                                            int Lp, float omega, float om1, int P) {
+template <int COLOR, bool STREAM, bool DOWN, bool WHOLE>
+__global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, const float* r_own, float* e_own,
+                                                            const float* e_oth, int Lp, float omega, float om1,
+                                                            int P) {
   const int nq = row_groups(d.nx);
   const int lane = threadIdx.x & 31;
   const unsigned f = blockIdx.x * (32 * kRows2) + threadIdx.x;   // row pair and group, groups fastest
-  const int pair = (int)(f / (unsigned)nq), q = (int)(f - (unsigned)pair * (unsigned)nq);
+  int pair = (int)(f / (unsigned)nq);
+  const int q = (int)(f - (unsigned)pair * (unsigned)nq);
+  const bool mine = WHOLE || 2 * pair + 2 <= d.ny + 1;
+  if (!WHOLE) pair = min(pair, (d.ny - 1) >> 1);   // a lane beyond the rows repeats the last pair and stores nothing
   const int ja = 2 * pair + 2;
+  const bool rowb = WHOLE || ja + 1 <= d.ny + 1;
   const int k0 = (DOWN ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * P + 2;
+  const int np = WHOLE ? P : (min(P, d.nz + 2 - k0) + 1) & ~1;   // planes; the last may be the top ghost plane
   const unsigned long long pol = STREAM ? evict_first_policy() : 0ull;
-  const bool lds = ja <= d.ny + 1;
-  const bool rowb = ja + 1 <= d.ny + 1;
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
   // the coefficient tables are written by the host before the solve, never by a
   // kernel, so they load before the wait for the previous pass
-  const float ya0 = lds ? g.acy32[0][ja - 1] : 0.f, ya1 = lds ? g.acy32[1][ja - 1] : 0.f,
-              ya2 = lds ? g.acy32[2][ja - 1] : 0.f;
-  const float yb0 = rowb ? g.acy32[0][ja] : 0.f, yb1 = rowb ? g.acy32[1][ja] : 0.f,
-              yb2 = rowb ? g.acy32[2][ja] : 0.f;
+  const int jb = WHOLE ? ja : min(ja, d.ny);
+  const float ya0 = g.acy32[0][ja - 1], ya1 = g.acy32[1][ja - 1], ya2 = g.acy32[2][ja - 1];
+  const float yb0 = g.acy32[0][jb], yb1 = g.acy32[1][jb], yb2 = g.acy32[2][jb];
   // P: the phase of row a at even planes (and of row b at odd ones); Q the other
-  const float4 p0 = lds ? g.axp[1 - COLOR][0][q] : z4, p1 = lds ? g.axp[1 - COLOR][1][q] : z4,
-               p2 = lds ? g.axp[1 - COLOR][2][q] : z4;
-  const float4 q0 = lds ? g.axp[COLOR][0][q] : z4, q1 = lds ? g.axp[COLOR][1][q] : z4,
-               q2 = lds ? g.axp[COLOR][2][q] : z4;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (__any_sync(0xffffffffu, lds)) {   // every lane of the warp stays for the shuffles
-    const bool load_left = lane == 0, load_right = lane == 31;
-    const bool first = q == 0, last = q + 1 == nq;
-    const int plane = (d.ny + 2) * Lp;
-    const int sa = (ja - 1) * Lp + 4 * q + 4;
-    // the march runs up from the slab's first plane, or down from its last; oc: the other
-    // colour at the plane, op at the plane before it on the march
-    const int ks = DOWN ? min(k0 + P - 1, d.nz + 1) : k0;
-    const int step = DOWN ? -plane : plane;
-    const int s1 = (ks - 1) * plane + sa;
-    float4 opa = lds ? ld4(e_oth + s1 - step) : z4, opb = lds ? ld4(e_oth + s1 - step + Lp) : z4;
-    float4 oca = lds ? ld4(e_oth + s1) : z4, ocb = lds ? ld4(e_oth + s1 + Lp) : z4;
-    for (int k2 = 0; k2 < P; k2 += kUnroll2)
+  const float4 p0 = g.axp[1 - COLOR][0][q], p1 = g.axp[1 - COLOR][1][q], p2 = g.axp[1 - COLOR][2][q];
+  const float4 q0 = g.axp[COLOR][0][q], q1 = g.axp[COLOR][1][q], q2 = g.axp[COLOR][2][q];
+  // the pointers pass through the wait so that no load can move above it
+  asm volatile("griddepcontrol.wait;" : "+l"(r_own), "+l"(e_own), "+l"(e_oth) : : "memory");
+  const bool first = q == 0, last = q + 1 == nq;
+  const int plane = (d.ny + 2) * Lp;
+  const int sa = (ja - 1) * Lp + 4 * q + 4;
+  const int north = rowb ? 2 * Lp : Lp;   // the row above the pair's (odd ny: row b is the ghost row)
+  // the march runs up from the slab's first plane, or down from its last; oc: the other
+  // colour at the plane, op at the plane before it on the march
+  const int ks = DOWN ? k0 + np - 1 : k0;
+  const int s1 = (ks - 1) * plane + sa, sp = DOWN ? min(ks, d.nz + 1) * plane + sa : s1 - plane;
+  float4 opa = ld4(e_oth + sp), opb = ld4(e_oth + sp + Lp), oca = ld4(e_oth + s1), ocb = ld4(e_oth + s1 + Lp);
+  auto update = [&](int m, auto odd) {
+    const int k = DOWN ? ks - m : ks + m;
+    const bool inside = WHOLE || k <= d.nz + 1;
+    const int s0 = (k - 1) * plane + sa;
+    const int s2 = DOWN ? s0 - plane : inside ? s0 + plane : s0;
+    const float4 ra = STREAM ? ld4_stream(r_own + s0, pol) : ld4(r_own + s0);
+    const float4 rb = STREAM ? ld4_stream(r_own + s0 + Lp, pol) : ld4(r_own + s0 + Lp);
+    const float4 ea = ld4(e_own + s0), eb = ld4(e_own + s0 + Lp);
+    const float4 osa = ld4(e_oth + s0 - Lp), onb = ld4(e_oth + s0 + north);
+    const float4 ona = ld4(e_oth + s2), onn = ld4(e_oth + s2 + Lp);
+    float la = __shfl_up_sync(0xffffffffu, oca.w, 1), ra_ = __shfl_down_sync(0xffffffffu, oca.x, 1);
+    float lb = __shfl_up_sync(0xffffffffu, ocb.w, 1), rb_ = __shfl_down_sync(0xffffffffu, ocb.x, 1);
+    if (lane == 0) {
+      la = ld1(e_oth + s0 - 1);
+      lb = ld1(e_oth + s0 + Lp - 1);
+    }
+    if (lane == 31) {
+      ra_ = ld1(e_oth + s0 + 4);
+      rb_ = ld1(e_oth + s0 + Lp + 4);
+    }
+    if (first) la = lb = 0.f;    // the row's ghost entries; the neighbouring lane is on another row
+    if (last) ra_ = rb_ = 0.f;
+    const float4 z = g.acz4[WHOLE ? k - 1 : min(k, d.nz + 1) - 1];
+    const float4 ba = DOWN ? ona : opa, ta = DOWN ? opa : ona, bb = DOWN ? onn : opb, tb = DOWN ? opb : onn;
+    const float xa[6] = {la, oca.x, oca.y, oca.z, oca.w, ra_};
+    const float xb[6] = {lb, ocb.x, ocb.y, ocb.z, ocb.w, rb_};
+    const float rva[4] = {ra.x, ra.y, ra.z, ra.w}, rvb[4] = {rb.x, rb.y, rb.z, rb.w};
+    const float sva[4] = {osa.x, osa.y, osa.z, osa.w}, nva[4] = {ocb.x, ocb.y, ocb.z, ocb.w};
+    const float svb[4] = {oca.x, oca.y, oca.z, oca.w}, nvb[4] = {onb.x, onb.y, onb.z, onb.w};
+    const float bva[4] = {ba.x, ba.y, ba.z, ba.w}, tva[4] = {ta.x, ta.y, ta.z, ta.w};
+    const float bvb[4] = {bb.x, bb.y, bb.z, bb.w}, tvb[4] = {tb.x, tb.y, tb.z, tb.w};
+    float eva[4] = {ea.x, ea.y, ea.z, ea.w}, evb[4] = {eb.x, eb.y, eb.z, eb.w};
+    if (odd.value == DOWN) {   // an even plane: slabs start at even planes and hold an even number
+      update4<COLOR != 0>(rva, eva, xa, sva, nva, bva, tva, p0, p1, p2, ya0, ya1, ya2, z.x, z.y, z.z, omega, om1);
+      update4<COLOR == 0>(rvb, evb, xb, svb, nvb, bvb, tvb, q0, q1, q2, yb0, yb1, yb2, z.x, z.y, z.z, omega, om1);
+    } else {
+      update4<COLOR == 0>(rva, eva, xa, sva, nva, bva, tva, q0, q1, q2, ya0, ya1, ya2, z.x, z.y, z.z, omega, om1);
+      update4<COLOR != 0>(rvb, evb, xb, svb, nvb, bvb, tvb, p0, p1, p2, yb0, yb1, yb2, z.x, z.y, z.z, omega, om1);
+    }
+    if (mine && inside) {
+      *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
+      if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
+    }
+    opa = oca;
+    oca = ona;
+    opb = ocb;
+    ocb = onn;
+  };
+  int m = 0;
+  for (; m + kUnroll2 <= np; m += kUnroll2) {
 #pragma unroll
-      for (int u = 0; u < kUnroll2; ++u) {
-        const int k = DOWN ? k0 + P - 1 - (k2 + u) : k0 + k2 + u;
-        if (k2 + u >= P || (!DOWN && k > d.nz + 1)) break;
-        if (DOWN && k > d.nz + 1) continue;
-        const int s0 = (k - 1) * plane + sa;
-        float4 ra = z4, ea = z4, rb = z4, eb = z4, osa = z4, onb = z4, ona = z4, onn = z4;
-        if (lds) {
-          ra = STREAM ? ld4_stream(r_own + s0, pol) : ld4(r_own + s0);
-          ea = ld4(e_own + s0);
-          osa = ld4(e_oth + s0 - Lp);
-          ona = ld4(e_oth + s0 + step);
-          onn = ld4(e_oth + s0 + Lp + step);
-          if (rowb) {
-            rb = STREAM ? ld4_stream(r_own + s0 + Lp, pol) : ld4(r_own + s0 + Lp);
-            eb = ld4(e_own + s0 + Lp);
-            onb = ld4(e_oth + s0 + 2 * Lp);
-          }
-        }
-        float la = __shfl_up_sync(0xffffffffu, oca.w, 1), ra_ = __shfl_down_sync(0xffffffffu, oca.x, 1);
-        float lb = __shfl_up_sync(0xffffffffu, ocb.w, 1), rb_ = __shfl_down_sync(0xffffffffu, ocb.x, 1);
-        if (lds && load_left) {
-          la = e_oth[s0 - 1];
-          lb = e_oth[s0 + Lp - 1];
-        }
-        if (lds && load_right) {
-          ra_ = e_oth[s0 + 4];
-          rb_ = e_oth[s0 + Lp + 4];
-        }
-        if (first) la = lb = 0.f;    // the row's ghost entries; the neighbouring lane is on another row
-        if (last) ra_ = rb_ = 0.f;
-        const float4 zc = g.acz4[k - 1];
-        const float z0 = zc.x, z1 = zc.y, z2 = zc.z;
-        if (lds) {
-          const float4 ba = DOWN ? ona : opa, ta = DOWN ? opa : ona, bb = DOWN ? onn : opb, tb = DOWN ? opb : onn;
-          const float xa[6] = {la, oca.x, oca.y, oca.z, oca.w, ra_};
-          const float xb[6] = {lb, ocb.x, ocb.y, ocb.z, ocb.w, rb_};
-          const float rva[4] = {ra.x, ra.y, ra.z, ra.w}, rvb[4] = {rb.x, rb.y, rb.z, rb.w};
-          const float sva[4] = {osa.x, osa.y, osa.z, osa.w}, nva[4] = {ocb.x, ocb.y, ocb.z, ocb.w};
-          const float svb[4] = {oca.x, oca.y, oca.z, oca.w}, nvb[4] = {onb.x, onb.y, onb.z, onb.w};
-          const float bva[4] = {ba.x, ba.y, ba.z, ba.w}, tva[4] = {ta.x, ta.y, ta.z, ta.w};
-          const float bvb[4] = {bb.x, bb.y, bb.z, bb.w}, tvb[4] = {tb.x, tb.y, tb.z, tb.w};
-          float eva[4] = {ea.x, ea.y, ea.z, ea.w}, evb[4] = {eb.x, eb.y, eb.z, eb.w};
-          if ((u & 1) == (DOWN ? 1 : 0)) {   // an even plane: slabs start at even planes and hold an even number
-            update4<COLOR != 0>(rva, eva, xa, sva, nva, bva, tva, p0, p1, p2, ya0, ya1, ya2, z0, z1, z2, omega, om1);
-            update4<COLOR == 0>(rvb, evb, xb, svb, nvb, bvb, tvb, q0, q1, q2, yb0, yb1, yb2, z0, z1, z2, omega, om1);
-          } else {
-            update4<COLOR == 0>(rva, eva, xa, sva, nva, bva, tva, q0, q1, q2, ya0, ya1, ya2, z0, z1, z2, omega, om1);
-            update4<COLOR != 0>(rvb, evb, xb, svb, nvb, bvb, tvb, p0, p1, p2, yb0, yb1, yb2, z0, z1, z2, omega, om1);
-          }
-          *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
-          if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
-        }
-        opa = oca;
-        oca = ona;
-        opb = ocb;
-        ocb = onn;
-      }
+    for (int u = 0; u < kUnroll2; u += 2) {
+      update(m + u, std::integral_constant<bool, false>{});
+      update(m + u + 1, std::integral_constant<bool, true>{});
+    }
+  }
+#pragma unroll 1
+  for (; !WHOLE && m < np; m += 2) {
+    update(m, std::integral_constant<bool, false>{});
+    update(m + 1, std::integral_constant<bool, true>{});
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -622,13 +642,16 @@ static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1) {
   float* e = c->ep[color];
   const float* o = c->ep[1 - color];
   const int Lp = c->packed_lp;
-  if (packed > kResidentMaxBytes) {
-    if (color == 0) cudaLaunchKernelEx(&cfg, k_sor32p2<0, true, false>, d, c->g, r, e, o, Lp, omega, om1, P);
-    else cudaLaunchKernelEx(&cfg, k_sor32p2<1, true, true>, d, c->g, r, e, o, Lp, omega, om1, P);
-  } else {
-    if (color == 0) cudaLaunchKernelEx(&cfg, k_sor32p2<0, false, false>, d, c->g, r, e, o, Lp, omega, om1, P);
-    else cudaLaunchKernelEx(&cfg, k_sor32p2<1, false, false>, d, c->g, r, e, o, Lp, omega, om1, P);
-  }
+  const bool whole = groups % (32 * kRows2) == 0 && d.ny % 2 == 0 && P % kUnroll2 == 0 && d.nz % P == 0;
+  const bool stream = packed > kResidentMaxBytes;
+  decltype(&k_sor32p2<0, false, false, false>) kern;
+  if (color == 0)
+    kern = stream ? (whole ? k_sor32p2<0, true, false, true> : k_sor32p2<0, true, false, false>)
+                  : (whole ? k_sor32p2<0, false, false, true> : k_sor32p2<0, false, false, false>);
+  else
+    kern = stream ? (whole ? k_sor32p2<1, true, true, true> : k_sor32p2<1, true, true, false>)
+                  : (whole ? k_sor32p2<1, false, false, true> : k_sor32p2<1, false, false, false>);
+  cudaLaunchKernelEx(&cfg, kern, d, c->g, r, e, o, Lp, omega, om1, P);
 }
 
 // One red-black sweep with the colour-packed two-pass kernels.

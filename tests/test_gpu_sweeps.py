@@ -136,3 +136,16 @@ def test_noalloc_solve_meets_the_residual(ib3d, grids, oracle_mod, shape):
     scale = np.abs(a[0]).max() + np.abs(a[1]).max() + np.abs(a[2]).max()
     assert np.max(np.abs(b[i, i, i] - Ap)[fluid]) < 1e-6 + 1e-14 * scale * np.max(np.abs(q))
     assert np.all(q[cell != 0] == 0.0)
+
+
+# launch-per-pass sweeps: whole tiles (256 x 192 x 192; streamed: 512 x 128 x 304), odd ny and nz
+# (the march starts or ends on the ghost plane, up and down), enough passes in a row
+# that a value left over from an earlier pass would show
+@pytest.mark.parametrize("shape", [(256, 192, 192), (256, 193, 193), (250, 191, 191), (512, 128, 304), (271, 225, 201)])
+def test_passes_read_the_last_pass_only(ib3d, grids, shape):
+    b = _rhs(shape)
+    want = _capped(ib3d, grids, shape, 75, b, sweep_kernel=1, smooth_sweeps=2, ramp_sweeps=5)
+    for kernel in (0, 0, 3, 4):
+        got = _capped(ib3d, grids, shape, 75, b, sweep_kernel=kernel, smooth_sweeps=2, ramp_sweeps=5)
+        assert got[0] == want[0]
+        assert np.array_equal(got[1], want[1]), kernel
