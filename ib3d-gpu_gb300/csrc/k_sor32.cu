@@ -166,7 +166,12 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
 // keeps the corrections, which every pass reads. DOWN: the slabs and their planes are
 // taken from the top; with the passes alternating in direction each starts on the planes
 // that the last one left in L2. 384x256x256: 72.6 us per sweep without either, 67.7 with
-// the first, 61.4 with both; 256^3 with one wave of blocks 44.2, 36.3 and 33.4.
+// the first, 61.4 with both; 256^3 with one wave of blocks 44.2, 36.3 and 33.4. Even so a
+// pass there read 88 MB from DRAM and wrote 48, all that it updates. So a part of the
+// corrections' lines, chosen by address, is marked to stay (half; an eighth where L2 cannot hold
+// that much) and the rest to go first (unmarked there): 60.1 -> 55.5 us at 384x256x256, 69.6 -> 66.0 at
+// 384x288x256, 32.6 -> 31.7 at 256^3; with an eighth 91.3 -> 88.9 at 448x320x256 and 128.8
+// -> 126.5 at 512x384x256 (with half 94.3 and 138).
 constexpr int kRows2 = 4;
 constexpr int kUnroll2 = 8;
 static_assert(kUnroll2 % 2 == 0, "the row phases alternate with the planes");
@@ -177,16 +182,38 @@ __device__ __forceinline__ float4 ld4_stream(const float* p, unsigned long long 
       : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
   return v;
 }
+__device__ __forceinline__ float4 ld4_keep(const float* p, unsigned long long pol) {
+  float4 v;
+  asm("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ void st4_keep(float* p, float4 v, unsigned long long pol) {
+  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
+      :: "l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(pol) : "memory");
+}
 __device__ __forceinline__ unsigned long long evict_first_policy() {
   unsigned long long pol;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
 
+// Keeps half of the lines (and lets the others go first), or an eighth.
+__device__ __forceinline__ unsigned long long keep_half_policy() {
+  unsigned long long pol;
+  asm("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, 0.5;" : "=l"(pol));
+  return pol;
+}
+__device__ __forceinline__ unsigned long long keep_eighth_policy() {
+  unsigned long long pol;
+  asm("createpolicy.fractional.L2::evict_last.b64 %0, 0.125;" : "=l"(pol));
+  return pol;
+}
+
 template <int COLOR, bool STREAM, bool DOWN, bool WHOLE>
 __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, const float* r_own, float* e_own,
-                                                            const float* e_oth, int Lp, float omega, float om1,
-                                                            int P) {
+                                                            const float* e_oth, int Lp, float omega, float om1, int P,
+                                                            bool half) {
   const int nq = row_groups(d.nx);
   const int lane = threadIdx.x & 31;
   const unsigned f = blockIdx.x * (32 * kRows2) + threadIdx.x;   // row pair and group, groups fastest
@@ -198,7 +225,8 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
   const bool rowb = WHOLE || ja + 1 <= d.ny + 1;
   const int k0 = (DOWN ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * P + 2;
   const int np = WHOLE ? P : (min(P, d.nz + 2 - k0) + 1) & ~1;   // planes; the last may be the top ghost plane
-  const unsigned long long pol = STREAM ? evict_first_policy() : 0ull;
+  const unsigned long long pol = STREAM ? evict_first_policy() : 0ull, 
+                           keep = !STREAM ? 0ull : half ? keep_half_policy() : keep_eighth_policy();
   // the coefficient tables are written by the host before the solve, never by a
   // kernel, so they load before the wait for the previous pass
   const int jb = WHOLE ? ja : min(ja, d.ny);
@@ -217,7 +245,8 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
   // colour at the plane, op at the plane before it on the march
   const int ks = DOWN ? k0 + np - 1 : k0;
   const int s1 = (ks - 1) * plane + sa, sp = DOWN ? min(ks, d.nz + 1) * plane + sa : s1 - plane;
-  float4 opa = ld4(e_oth + sp), opb = ld4(e_oth + sp + Lp), oca = ld4(e_oth + s1), ocb = ld4(e_oth + s1 + Lp);
+  auto lde = [&](const float* p) { return STREAM ? ld4_keep(p, keep) : ld4(p); };
+  float4 opa = lde(e_oth + sp), opb = lde(e_oth + sp + Lp), oca = lde(e_oth + s1), ocb = lde(e_oth + s1 + Lp);
   auto update = [&](int m, auto odd) {
     const int k = DOWN ? ks - m : ks + m;
     const bool inside = WHOLE || k <= d.nz + 1;
@@ -225,9 +254,9 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
     const int s2 = DOWN ? s0 - plane : inside ? s0 + plane : s0;
     const float4 ra = STREAM ? ld4_stream(r_own + s0, pol) : ld4(r_own + s0);
     const float4 rb = STREAM ? ld4_stream(r_own + s0 + Lp, pol) : ld4(r_own + s0 + Lp);
-    const float4 ea = ld4(e_own + s0), eb = ld4(e_own + s0 + Lp);
-    const float4 osa = ld4(e_oth + s0 - Lp), onb = ld4(e_oth + s0 + north);
-    const float4 ona = ld4(e_oth + s2), onn = ld4(e_oth + s2 + Lp);
+    const float4 ea = lde(e_own + s0), eb = lde(e_own + s0 + Lp);
+    const float4 osa = lde(e_oth + s0 - Lp), onb = lde(e_oth + s0 + north);
+    const float4 ona = lde(e_oth + s2), onn = lde(e_oth + s2 + Lp);
     float la = __shfl_up_sync(0xffffffffu, oca.w, 1), ra_ = __shfl_down_sync(0xffffffffu, oca.x, 1);
     float lb = __shfl_up_sync(0xffffffffu, ocb.w, 1), rb_ = __shfl_down_sync(0xffffffffu, ocb.x, 1);
     if (lane == 0) {
@@ -258,8 +287,13 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
       update4<COLOR != 0>(rvb, evb, xb, svb, nvb, bvb, tvb, p0, p1, p2, yb0, yb1, yb2, z.x, z.y, z.z, omega, om1);
     }
     if (mine && inside) {
-      *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
-      if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
+      if (STREAM) {
+        st4_keep(e_own + s0, make_float4(eva[0], eva[1], eva[2], eva[3]), keep);
+        if (rowb) st4_keep(e_own + s0 + Lp, make_float4(evb[0], evb[1], evb[2], evb[3]), keep);
+      } else {
+        *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
+        if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
+      }
     }
     opa = oca;
     oca = ona;
@@ -606,6 +640,10 @@ void launch_sor32_packed(ib3d_ctx* c, int color, float omega, float om1) {
 // (106 MB) it gains 5 % (31.7 against 33.4), at 256^3 (145 MB) 18 %.
 constexpr size_t kResidentMaxBytes = (size_t)96 << 20;
 
+// Up to here the passes keep half of the corrections' lines in L2, beyond an eighth (figures at
+// k_sor32p2: the line lies between 384x288x256, 236 MB, and 448x320x256, 303 MB).
+constexpr size_t kHalfMaxBytes = (size_t)256 << 20;
+
 // Planes per slab: the fewest that let every block of the pass run at once (four per SM),
 // because a second, partly filled wave costs a whole one (us per sweep at 272x192x192: 8
 // planes 24.6, 10 planes 19.3; at 200x160x160: 4 planes 14.2, 6 planes 11.2, 8 planes 13.4;
@@ -651,7 +689,7 @@ static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1) {
   else
     kern = stream ? (whole ? k_sor32p2<1, true, true, true> : k_sor32p2<1, true, true, false>)
                   : (whole ? k_sor32p2<1, false, false, true> : k_sor32p2<1, false, false, false>);
-  cudaLaunchKernelEx(&cfg, kern, d, c->g, r, e, o, Lp, omega, om1, P);
+  cudaLaunchKernelEx(&cfg, kern, d, c->g, r, e, o, Lp, omega, om1, P, packed <= kHalfMaxBytes);
 }
 
 // One red-black sweep with the colour-packed two-pass kernels.
