@@ -286,7 +286,8 @@ int alloc_fields(ib3d_ctx* c) {
   if (cudaMallocHost(&c->h_ctl, sizeof(SolveCtl)) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMalloc(&c->d_flag, 4 * sizeof(int)) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMalloc(&c->d_levels, 128 * sizeof(int)) != cudaSuccess) return IB3D_ERR_MEMORY;
-  if (cudaMalloc(&c->d_coef, 8 * sizeof(double)) != cudaSuccess) return IB3D_ERR_MEMORY;
+  if (cudaMalloc(&c->d_coef, 16 * sizeof(double)) != cudaSuccess) return IB3D_ERR_MEMORY;
+  if (cudaMemset(c->d_coef, 0, 16 * sizeof(double)) != cudaSuccess) return IB3D_ERR_CUDA;
   {
     const double uc0 = 1.0;   // uc = 1 (subReadInput.f90:28); d_coef[6] holds the outlet speed
     if (cudaMemcpy(c->d_coef + 6, &uc0, sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) return IB3D_ERR_CUDA;

@@ -233,7 +233,7 @@ struct ib3d_ctx {
   bool have_scache = false;
   int* d_scache = nullptr;     // 15*nelems: cell, u, v, w, p brackets (3 each)
   double* d_contrib = nullptr; // 7*nelems per-element terms
-  double* d_coef = nullptr;    // 4 coefficients
+  double* d_coef = nullptr;    // 4 coefficients; [4], [5] divergence, [6] outlet speed; [8 .. 14] drag sums, [15] blocks done
   int* d_flag = nullptr;       // device flags: [0] error (probe out of grid), [1], [2] see finish_search
 
   // reduction / scan scratch
@@ -409,6 +409,12 @@ __device__ __forceinline__ double div_known(double a, double b, double zh, doubl
   if (((ha & 0x7fffffff) | __double2loint(a)) == 0 && (__double2hiint(zh) & 0x7ff00000) != 0x7ff00000)
     return __hiloint2double((ha ^ __double2hiint(b)) & (int)0x80000000, 0);
   return a / b;
+}
+// The two parts of 1/b worked out by the thread that will divide by b several times.
+__device__ __forceinline__ KnownDiv known(double b) {
+  const unsigned ex = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
+  const double zh = 1.0 / b;
+  return {b, ex - 824u < 399u ? zh : __longlong_as_double(0x7ff8000000000000ll), zh * fma(-zh, b, 1.0)};
 }
 __device__ __forceinline__ double div_known(double a, const KnownDiv& d) { return div_known(a, d.b, d.zh, d.zl); }
 

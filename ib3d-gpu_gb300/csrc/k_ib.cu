@@ -44,29 +44,35 @@ __device__ __forceinline__ int bracket(const double* A, int lo, int hi, double p
 // Trilinear probe value and one-sided quadratic derivative estimates, the common
 // block of subForcing.f90:175-215 (and its analogues in subStressCal1.f90).
 // f = values at (x0|x1, y0|y1, z0|z1) with x fastest: f[q], q = xbit + 2*ybit + 4*zbit.
+// Bound by the warp's count of FP64 instructions (64 cycles each, whatever its lanes do): the
+// fifteen divisions by the cell's three widths run through their reciprocals, 4 operations
+// each instead of 9, with the same rounded quotients.
 __device__ __forceinline__ void probe_eval(const double f[8], const double* X, const double* Y, const double* Z,
                                            int ix, int iy, int iz, double px, double py, double pz,
                                            double out[4]) {
   const double f000 = f[0], f100 = f[1], f010 = f[2], f110 = f[3];
   const double f001 = f[4], f101 = f[5], f011 = f[6], f111 = f[7];
-  const double tx = px - X[ix], dX = X[ix + 1] - X[ix];
-  const double ty = py - Y[iy], dY = Y[iy + 1] - Y[iy];
-  const double tz = pz - Z[iz], dZ = Z[iz + 1] - Z[iz];
-  const double x1z1 = f000 + (f100 - f000) * tx / dX;
-  const double x2z1 = f010 + (f110 - f010) * tx / dX;
-  const double x1z2 = f001 + (f101 - f001) * tx / dX;
-  const double x2z2 = f011 + (f111 - f011) * tx / dX;
-  const double z1 = x1z1 + (x2z1 - x1z1) * ty / dY;
-  const double z2 = x1z2 + (x2z2 - x1z2) * ty / dY;
-  const double y1 = x1z1 + (x1z2 - x1z1) * tz / dZ;
-  const double y2 = x2z1 + (x2z2 - x2z1) * tz / dZ;
-  const double z1x1 = f000 + (f001 - f000) * tz / dZ;
-  const double z2x1 = f010 + (f011 - f010) * tz / dZ;
-  const double z1x2 = f100 + (f101 - f100) * tz / dZ;
-  const double z2x2 = f110 + (f111 - f110) * tz / dZ;
-  const double x1 = z1x1 + (z2x1 - z1x1) * ty / dY;
-  const double x2 = z1x2 + (z2x2 - z1x2) * ty / dY;
-  const double pos = x1 + (x2 - x1) * tx / dX;
+  const double tx = px - X[ix];
+  const KnownDiv dX = known(X[ix + 1] - X[ix]);
+  const double ty = py - Y[iy];
+  const KnownDiv dY = known(Y[iy + 1] - Y[iy]);
+  const double tz = pz - Z[iz];
+  const KnownDiv dZ = known(Z[iz + 1] - Z[iz]);
+  const double x1z1 = f000 + div_known((f100 - f000) * tx, dX);
+  const double x2z1 = f010 + div_known((f110 - f010) * tx, dX);
+  const double x1z2 = f001 + div_known((f101 - f001) * tx, dX);
+  const double x2z2 = f011 + div_known((f111 - f011) * tx, dX);
+  const double z1 = x1z1 + div_known((x2z1 - x1z1) * ty, dY);
+  const double z2 = x1z2 + div_known((x2z2 - x1z2) * ty, dY);
+  const double y1 = x1z1 + div_known((x1z2 - x1z1) * tz, dZ);
+  const double y2 = x2z1 + div_known((x2z2 - x2z1) * tz, dZ);
+  const double z1x1 = f000 + div_known((f001 - f000) * tz, dZ);
+  const double z2x1 = f010 + div_known((f011 - f010) * tz, dZ);
+  const double z1x2 = f100 + div_known((f101 - f100) * tz, dZ);
+  const double z2x2 = f110 + div_known((f111 - f110) * tz, dZ);
+  const double x1 = z1x1 + div_known((z2x1 - z1x1) * ty, dY);
+  const double x2 = z1x2 + div_known((z2x2 - z1x2) * ty, dY);
+  const double pos = x1 + div_known((x2 - x1) * tx, dX);
   double h2 = fabs(X[ix + 1] - px), h1 = fabs(X[ix] - px);
   out[1] = (h1 * h1 * x2 - h2 * h2 * x1 + (h2 * h2 - h1 * h1) * pos) / (h1 * h2 * (h1 + h2) + 1e-16);
   h2 = fabs(Y[iy + 1] - py); h1 = fabs(Y[iy] - py);
@@ -883,29 +889,35 @@ __global__ void __launch_bounds__(kSumThreads) k_stress_sum(const double* __rest
 }
 
 // The same sums in a fixed tree order, for the forms whose results may differ from the
-// reference's arithmetic by rounding (IB3D_PREC_FP32DC, IB3D_PREC_FP64_FAST).
+// reference's arithmetic by rounding (IB3D_PREC_FP32DC, IB3D_PREC_FP64_FAST). A block per sum
+// (one block for all seven was bound by its SM's FP64 pipe: 14 us for 5,120 elements); the
+// last to finish works out the coefficients. sums: coef[8 .. 14]; coef[15] counts the blocks
+// and is left at 0.
 constexpr int kTreeThreads = 512;
 __global__ void __launch_bounds__(kTreeThreads) k_stress_sum_tree(const double* __restrict__ contrib, int ne, double* coef) {
-  __shared__ double w[7][kTreeThreads / 32], s[7];
-  const int t = threadIdx.x;
-  double a[7] = {};
-  for (int e = t; e < ne; e += kTreeThreads)
-#pragma unroll
-    for (int q = 0; q < 7; ++q) a[q] += contrib[(long long)q * ne + e];
-#pragma unroll
-  for (int q = 0; q < 7; ++q) {
-    for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
-    if ((t & 31) == 0) w[q][t >> 5] = a[q];
-  }
+  __shared__ double w[kTreeThreads / 32];
+  const int t = threadIdx.x, q = blockIdx.x;
+  double a = 0.0;
+  for (int e = t; e < ne; e += kTreeThreads) a += contrib[(long long)q * ne + e];
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+  if ((t & 31) == 0) w[t >> 5] = a;
   __syncthreads();
   if (t < 32) {
+    double x = t < kTreeThreads / 32 ? w[t] : 0.0;
+    for (int o = kTreeThreads / 64; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (t == 0) {
+      int* done = reinterpret_cast<int*>(coef + 15);
+      coef[8 + q] = x;
+      __threadfence();
+      if (atomicAdd(done, 1) == 6) {
+        __threadfence();
+        double s[7];
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      double x = t < kTreeThreads / 32 ? w[q][t] : 0.0;
-      for (int o = kTreeThreads / 64; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (t == 0) s[q] = x;
+        for (int r = 0; r < 7; ++r) s[r] = __ldcg(coef + 8 + r);
+        stress_coefficients(s, coef);
+        *done = 0;
+      }
     }
-    if (t == 0) stress_coefficients(s, coef);
   }
 }
 
@@ -1306,7 +1318,7 @@ int run_stress(ib3d_ctx* c, int first, double coef[4]) {
   k_stress_elem<<<nblk(4ll * ne, 64), 64, 0, c->st>>>(c->d, c->g, c->d_surf, ne, do_first, c->d_scache, c->ut, c->vt,
                                                       c->wt, c->p, 1.0 / c->prm.re, c->d_contrib, c->d_flag);
   if (c->prm.precision == IB3D_PREC_FP64) k_stress_sum<<<1, kSumThreads, 0, c->st>>>(c->d_contrib, ne, c->d_coef);
-  else k_stress_sum_tree<<<1, kTreeThreads, 0, c->st>>>(c->d_contrib, ne, c->d_coef);
+  else k_stress_sum_tree<<<7, kTreeThreads, 0, c->st>>>(c->d_contrib, ne, c->d_coef);
   IB3D_CUDA(c, cudaGetLastError());
   if (do_first) {
     int flag = 0;
