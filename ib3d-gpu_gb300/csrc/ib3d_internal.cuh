@@ -111,6 +111,13 @@ struct ForceSched {
   bool ordered;      // false: no op reads another's value, and one level holds them all
 };
 
+// How the launch-per-pass sweeps of a grid beyond L2 go through it: n parts of planes with
+// boundaries at first, first + planes, ..., `group` sweeps at a time (sweep_group in
+// k_sor32.cu). n is 1 where L2 holds the grid, 0 before the first use.
+struct SweepParts {
+  int n, first, planes, group;
+};
+
 // How a grid's rows are split over the blocks of a resident kernel: gy x gz blocks of at
 // most by x bz rows (full x extent), nt threads (zl: FP32, planes a thread marches
 // through), smem bytes of shared memory, and the
@@ -178,7 +185,8 @@ struct ib3d_ctx {
   cudaGraphExec_t sweep_exec = nullptr;
   ib3d::Grid1D sweep_g{};
   float sweep_w = 0.f, sweep_w1 = 0.f;
-  int sweep_kern = -1;
+  int sweep_kern = -1, sweep_launches = 0;
+  ib3d::SweepParts parts{0, 0, 0, 0};
   bool sweep_graph_failed = false;   // capture refused once: the sweeps launch one by one
   int packed_lp = 0;
   // on-chip sweeps (k_resident.cu): the split of this grid, planned on first use, the
@@ -289,8 +297,8 @@ void launch_momentum_fast(ib3d_ctx* c, bool ab2);
 // k_sor32.cu
 int packed_row_length(int nx);
 void launch_sor32_packed(ib3d_ctx* c, int color, float omega, float om1);
-void launch_sor32_sweep(ib3d_ctx* c, float omega, float om1);
-void run_sor32_sweeps(ib3d_ctx* c, int n, float omega, float om1);
+int launch_sor32_sweeps(ib3d_ctx* c, int n, const float2* w);
+int run_sor32_sweeps(ib3d_ctx* c, int n, float omega, float om1);
 void launch_accumulate_packed(ib3d_ctx* c);
 void launch_sor32_fused(ib3d_ctx* c, float omega, float om1);
 bool fused_sweep_fits(int nx);

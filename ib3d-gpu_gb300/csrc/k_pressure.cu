@@ -13,6 +13,7 @@
 // through int64 index lists.
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "ib3d_internal.cuh"
 
@@ -607,14 +608,14 @@ int run_sor_fp32dc(ib3d_ctx* c, ib3d_solve_stats* st) {
     }
     if (!on_chip) {
       PhaseScope ps(c, PH_SOR32);
-      c->launches += fused ? batch : 2 * batch;
-      c->t_launches32 += fused ? batch : 2 * batch;
       // the solve's first sweeps run at relaxation 1 (smooth_sweeps: Gauss-Seidel damps the
       // high-frequency error that the over-relaxed sweeps barely touch), the next
       // ramp_sweeps with the relaxation rising linearly from 1 to omega_inner; the
       // colour-packed kernels run the sweeps after those through run_sor32_sweeps
       const int special = outer == 0 ? P.smooth_sweeps + P.ramp_sweeps : 0;
       const int direct = packed && !fused ? std::min(batch, special) : batch;
+      long long launched = 0;
+      std::vector<float2> ws;
       for (int q = 0; q < direct; ++q) {
         const bool smooth = outer == 0 && q < P.smooth_sweeps;
         float w = smooth ? 1.0f : om, w1 = smooth ? 0.0f : om1;
@@ -625,14 +626,19 @@ int run_sor_fp32dc(ib3d_ctx* c, ib3d_solve_stats* st) {
         }
         if (fused) {
           launch_sor32_fused(c, w, w1);
+          ++launched;
         } else if (packed) {
-          launch_sor32_sweep(c, w, w1);
+          ws.push_back(make_float2(w, w1));
         } else {
           k_sor32<0><<<gcol, kBlock, 0, c->st>>>(d, c->g, c->r32, c->e32, c->cell, w, w1);
           k_sor32<1><<<gcol, kBlock, 0, c->st>>>(d, c->g, c->r32, c->e32, c->cell, w, w1);
+          launched += 2;
         }
       }
-      if (direct < batch) run_sor32_sweeps(c, batch - direct, om, om1);
+      if (!ws.empty()) launched += launch_sor32_sweeps(c, (int)ws.size(), ws.data());
+      if (direct < batch) launched += run_sor32_sweeps(c, batch - direct, om, om1);
+      c->launches += launched;
+      c->t_launches32 += launched;
     }
     if (!on_chip) {
       PhaseScope ps(c, PH_RESIDUAL);

@@ -161,59 +161,16 @@ __global__ void __launch_bounds__(32 * kRows, 8) k_sor32p(Dims d, Grid1D g, cons
 // blocks and the planes the slabs, which takes the clamps out too: 14.6 us there, 14.3
 // against 15.0 at 256x224x160.
 //
-// STREAM, for arrays that do not fit in L2: the right-hand side, read once a pass and not
-// again until the pass after next, is loaded past L1 and first to leave L2, so that L2
-// keeps the corrections, which every pass reads. DOWN: the slabs and their planes are
-// taken from the top; with the passes alternating in direction each starts on the planes
-// that the last one left in L2. 384x256x256: 72.6 us per sweep without either, 67.7 with
-// the first, 61.4 with both; 256^3 with one wave of blocks 44.2, 36.3 and 33.4. Even so a
-// pass there read 88 MB from DRAM and wrote 48, all that it updates. So a part of the
-// corrections' lines, chosen by address, is marked to stay (half; an eighth where L2 cannot hold
-// that much) and the rest to go first (unmarked there): 60.1 -> 55.5 us at 384x256x256, 69.6 -> 66.0 at
-// 384x288x256, 32.6 -> 31.7 at 256^3; with an eighth 91.3 -> 88.9 at 448x320x256 and 128.8
-// -> 126.5 at 512x384x256 (with half 94.3 and 138).
+// The planes are ka .. kb - 1 (0-based interior planes; ka even, kb even or the last): the
+// whole grid, or a part of it where the sweeps go through L2-sized parts (sweep_group).
 constexpr int kRows2 = 4;
 constexpr int kUnroll2 = 8;
 static_assert(kUnroll2 % 2 == 0, "the row phases alternate with the planes");
 
-__device__ __forceinline__ float4 ld4_stream(const float* p, unsigned long long pol) {
-  float4 v;
-  asm("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ float4 ld4_keep(const float* p, unsigned long long pol) {
-  float4 v;
-  asm("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ void st4_keep(float* p, float4 v, unsigned long long pol) {
-  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
-      :: "l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(pol) : "memory");
-}
-__device__ __forceinline__ unsigned long long evict_first_policy() {
-  unsigned long long pol;
-  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
-}
-
-// Keeps half of the lines (and lets the others go first), or an eighth.
-__device__ __forceinline__ unsigned long long keep_half_policy() {
-  unsigned long long pol;
-  asm("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, 0.5;" : "=l"(pol));
-  return pol;
-}
-__device__ __forceinline__ unsigned long long keep_eighth_policy() {
-  unsigned long long pol;
-  asm("createpolicy.fractional.L2::evict_last.b64 %0, 0.125;" : "=l"(pol));
-  return pol;
-}
-
-template <int COLOR, bool STREAM, bool DOWN, bool WHOLE>
+template <int COLOR, bool WHOLE>
 __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, const float* r_own, float* e_own,
                                                             const float* e_oth, int Lp, float omega, float om1, int P,
-                                                            bool half) {
+                                                            int ka, int kb) {
   const int nq = row_groups(d.nx);
   const int lane = threadIdx.x & 31;
   const unsigned f = blockIdx.x * (32 * kRows2) + threadIdx.x;   // row pair and group, groups fastest
@@ -223,10 +180,8 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
   if (!WHOLE) pair = min(pair, (d.ny - 1) >> 1);   // a lane beyond the rows repeats the last pair and stores nothing
   const int ja = 2 * pair + 2;
   const bool rowb = WHOLE || ja + 1 <= d.ny + 1;
-  const int k0 = (DOWN ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * P + 2;
-  const int np = WHOLE ? P : (min(P, d.nz + 2 - k0) + 1) & ~1;   // planes; the last may be the top ghost plane
-  const unsigned long long pol = STREAM ? evict_first_policy() : 0ull, 
-                           keep = !STREAM ? 0ull : half ? keep_half_policy() : keep_eighth_policy();
+  const int k0 = blockIdx.y * P + ka + 2;
+  const int np = WHOLE ? P : (min(P, kb + 2 - k0) + 1) & ~1;   // planes; the last may be the top ghost plane
   // the coefficient tables are written by the host before the solve, never by a
   // kernel, so they load before the wait for the previous pass
   const int jb = WHOLE ? ja : min(ja, d.ny);
@@ -241,22 +196,19 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
   const int plane = (d.ny + 2) * Lp;
   const int sa = (ja - 1) * Lp + 4 * q + 4;
   const int north = rowb ? 2 * Lp : Lp;   // the row above the pair's (odd ny: row b is the ghost row)
-  // the march runs up from the slab's first plane, or down from its last; oc: the other
-  // colour at the plane, op at the plane before it on the march
-  const int ks = DOWN ? k0 + np - 1 : k0;
-  const int s1 = (ks - 1) * plane + sa, sp = DOWN ? min(ks, d.nz + 1) * plane + sa : s1 - plane;
-  auto lde = [&](const float* p) { return STREAM ? ld4_keep(p, keep) : ld4(p); };
-  float4 opa = lde(e_oth + sp), opb = lde(e_oth + sp + Lp), oca = lde(e_oth + s1), ocb = lde(e_oth + s1 + Lp);
+  // oc: the other colour at the plane, op at the plane below
+  const int s1 = (k0 - 1) * plane + sa;
+  float4 opa = ld4(e_oth + s1 - plane), opb = ld4(e_oth + s1 - plane + Lp), oca = ld4(e_oth + s1),
+         ocb = ld4(e_oth + s1 + Lp);
   auto update = [&](int m, auto odd) {
-    const int k = DOWN ? ks - m : ks + m;
+    const int k = k0 + m;
     const bool inside = WHOLE || k <= d.nz + 1;
     const int s0 = (k - 1) * plane + sa;
-    const int s2 = DOWN ? s0 - plane : inside ? s0 + plane : s0;
-    const float4 ra = STREAM ? ld4_stream(r_own + s0, pol) : ld4(r_own + s0);
-    const float4 rb = STREAM ? ld4_stream(r_own + s0 + Lp, pol) : ld4(r_own + s0 + Lp);
-    const float4 ea = lde(e_own + s0), eb = lde(e_own + s0 + Lp);
-    const float4 osa = lde(e_oth + s0 - Lp), onb = lde(e_oth + s0 + north);
-    const float4 ona = lde(e_oth + s2), onn = lde(e_oth + s2 + Lp);
+    const int s2 = inside ? s0 + plane : s0;
+    const float4 ra = ld4(r_own + s0), rb = ld4(r_own + s0 + Lp);
+    const float4 ea = ld4(e_own + s0), eb = ld4(e_own + s0 + Lp);
+    const float4 osa = ld4(e_oth + s0 - Lp), onb = ld4(e_oth + s0 + north);
+    const float4 ona = ld4(e_oth + s2), onn = ld4(e_oth + s2 + Lp);
     float la = __shfl_up_sync(0xffffffffu, oca.w, 1), ra_ = __shfl_down_sync(0xffffffffu, oca.x, 1);
     float lb = __shfl_up_sync(0xffffffffu, ocb.w, 1), rb_ = __shfl_down_sync(0xffffffffu, ocb.x, 1);
     if (lane == 0) {
@@ -270,16 +222,15 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
     if (first) la = lb = 0.f;    // the row's ghost entries; the neighbouring lane is on another row
     if (last) ra_ = rb_ = 0.f;
     const float4 z = g.acz4[WHOLE ? k - 1 : min(k, d.nz + 1) - 1];
-    const float4 ba = DOWN ? ona : opa, ta = DOWN ? opa : ona, bb = DOWN ? onn : opb, tb = DOWN ? opb : onn;
     const float xa[6] = {la, oca.x, oca.y, oca.z, oca.w, ra_};
     const float xb[6] = {lb, ocb.x, ocb.y, ocb.z, ocb.w, rb_};
     const float rva[4] = {ra.x, ra.y, ra.z, ra.w}, rvb[4] = {rb.x, rb.y, rb.z, rb.w};
     const float sva[4] = {osa.x, osa.y, osa.z, osa.w}, nva[4] = {ocb.x, ocb.y, ocb.z, ocb.w};
     const float svb[4] = {oca.x, oca.y, oca.z, oca.w}, nvb[4] = {onb.x, onb.y, onb.z, onb.w};
-    const float bva[4] = {ba.x, ba.y, ba.z, ba.w}, tva[4] = {ta.x, ta.y, ta.z, ta.w};
-    const float bvb[4] = {bb.x, bb.y, bb.z, bb.w}, tvb[4] = {tb.x, tb.y, tb.z, tb.w};
+    const float bva[4] = {opa.x, opa.y, opa.z, opa.w}, tva[4] = {ona.x, ona.y, ona.z, ona.w};
+    const float bvb[4] = {opb.x, opb.y, opb.z, opb.w}, tvb[4] = {onn.x, onn.y, onn.z, onn.w};
     float eva[4] = {ea.x, ea.y, ea.z, ea.w}, evb[4] = {eb.x, eb.y, eb.z, eb.w};
-    if (odd.value == DOWN) {   // an even plane: slabs start at even planes and hold an even number
+    if (!odd.value) {   // an even plane: slabs start at even planes and hold an even number
       update4<COLOR != 0>(rva, eva, xa, sva, nva, bva, tva, p0, p1, p2, ya0, ya1, ya2, z.x, z.y, z.z, omega, om1);
       update4<COLOR == 0>(rvb, evb, xb, svb, nvb, bvb, tvb, q0, q1, q2, yb0, yb1, yb2, z.x, z.y, z.z, omega, om1);
     } else {
@@ -287,13 +238,8 @@ __global__ void __launch_bounds__(32 * kRows2, 4) k_sor32p2(Dims d, Grid1D g, co
       update4<COLOR != 0>(rvb, evb, xb, svb, nvb, bvb, tvb, p0, p1, p2, yb0, yb1, yb2, z.x, z.y, z.z, omega, om1);
     }
     if (mine && inside) {
-      if (STREAM) {
-        st4_keep(e_own + s0, make_float4(eva[0], eva[1], eva[2], eva[3]), keep);
-        if (rowb) st4_keep(e_own + s0 + Lp, make_float4(evb[0], evb[1], evb[2], evb[3]), keep);
-      } else {
-        *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
-        if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
-      }
+      *reinterpret_cast<float4*>(e_own + s0) = make_float4(eva[0], eva[1], eva[2], eva[3]);
+      if (rowb) *reinterpret_cast<float4*>(e_own + s0 + Lp) = make_float4(evb[0], evb[1], evb[2], evb[3]);
     }
     opa = oca;
     oca = ona;
@@ -634,15 +580,16 @@ void launch_sor32_packed(ib3d_ctx* c, int color, float omega, float om1) {
   }
 }
 
-// Where the four packed arrays exceed 96 MB, L2 no longer holds them with what else a pass
-// touches, and the passes stream the right-hand side and alternate in direction: at
-// 272x192x192 (85 MB) that costs 14 % (22.1 against 19.3 us per sweep), at 288x208x208
-// (106 MB) it gains 5 % (31.7 against 33.4), at 256^3 (145 MB) 18 %.
+// Up to here the four packed arrays stay in L2 from pass to pass; beyond, the sweeps go through the
+// grid in parts (us per sweep, whole and in parts: 272x192x192, 85 MB, 20.3 and 21.9;
+// 288x208x208, 106 MB, 28.9 and 26.4).
 constexpr size_t kResidentMaxBytes = (size_t)96 << 20;
 
-// Up to here the passes keep half of the corrections' lines in L2, beyond an eighth (figures at
-// k_sor32p2: the line lies between 384x288x256, 236 MB, and 448x320x256, 303 MB).
-constexpr size_t kHalfMaxBytes = (size_t)256 << 20;
+// A part's bytes, at most, and sweeps per group: 384x256x256 took 52.3, 47.7 and 51.7 us per sweep
+// with 64, 80 and 96 MB, and 50.3, 47.7 and 51.9 with groups of 4, 8 and 16.
+constexpr size_t kPartBytes = (size_t)80 << 20;
+constexpr int kGroup = 8;
+constexpr int kLaunchPlanes = 4;
 
 // Planes per slab: the fewest that let every block of the pass run at once (four per SM),
 // because a second, partly filled wave costs a whole one (us per sweep at 272x192x192: 8
@@ -650,24 +597,27 @@ constexpr size_t kHalfMaxBytes = (size_t)256 << 20;
 // at 256^3: 8 planes 36.8, 14 planes 33.5), and a thread's planes run one after the other.
 // Beyond 24 planes the slabs of one wave get so long that several waves of 8 planes are
 // as good or better (400x320x300: 96.7 against 106).
-static int slab_planes(const ib3d_ctx* c, unsigned bx) {
+static int slab_planes(const ib3d_ctx* c, unsigned bx, int nz) {
   const unsigned slots = 4u * (unsigned)c->nsm;
-  const int nz = c->d.nz;
   if (bx == 0 || bx > slots) return 8;
   int P = (nz + (int)(slots / bx) - 1) / (int)(slots / bx);
   P += P & 1;
   return P <= 24 ? std::max(P, 2) : 8;
 }
 
-// One colour pass of the two-row kernel.
-static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1) {
-  const Dims& d = c->d;
+// Blocks of one slab of the two-row kernel.
+static unsigned slab_blocks(const Dims& d) {
   const unsigned groups = (unsigned)row_groups(d.nx) * (unsigned)((d.ny + 1) >> 1);
-  const unsigned bx = (groups + 32 * kRows2 - 1) / (32 * kRows2);
-  const int P = slab_planes(c, bx);
-  const size_t packed = 4 * sizeof(float) * (size_t)c->packed_lp * (size_t)d.NY2 * (size_t)d.NZ2;
+  return (groups + 32 * kRows2 - 1) / (32 * kRows2);
+}
+
+// One colour pass of the two-row kernel over planes ka .. kb - 1.
+static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1, int ka, int kb) {
+  const Dims& d = c->d;
+  const unsigned bx = slab_blocks(d);
+  const int n = kb - ka, P = slab_planes(c, bx, n);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(bx, (unsigned)((d.nz + P - 1) / P));
+  cfg.gridDim = dim3(bx, (unsigned)((n + P - 1) / P));
   cfg.blockDim = dim3(32 * kRows2);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = c->st;
@@ -676,31 +626,105 @@ static void launch_pass2(ib3d_ctx* c, int color, float omega, float om1) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const float* r = c->rp[color];
-  float* e = c->ep[color];
-  const float* o = c->ep[1 - color];
-  const int Lp = c->packed_lp;
-  const bool whole = groups % (32 * kRows2) == 0 && d.ny % 2 == 0 && P % kUnroll2 == 0 && d.nz % P == 0;
-  const bool stream = packed > kResidentMaxBytes;
-  decltype(&k_sor32p2<0, false, false, false>) kern;
-  if (color == 0)
-    kern = stream ? (whole ? k_sor32p2<0, true, false, true> : k_sor32p2<0, true, false, false>)
-                  : (whole ? k_sor32p2<0, false, false, true> : k_sor32p2<0, false, false, false>);
-  else
-    kern = stream ? (whole ? k_sor32p2<1, true, true, true> : k_sor32p2<1, true, true, false>)
-                  : (whole ? k_sor32p2<1, false, false, true> : k_sor32p2<1, false, false, false>);
-  cudaLaunchKernelEx(&cfg, kern, d, c->g, r, e, o, Lp, omega, om1, P, packed <= kHalfMaxBytes);
+  const unsigned groups = (unsigned)row_groups(d.nx) * (unsigned)((d.ny + 1) >> 1);
+  const bool whole = groups % (32 * kRows2) == 0 && d.ny % 2 == 0 && P % kUnroll2 == 0 && n % P == 0;
+  const auto kern = color == 0 ? (whole ? k_sor32p2<0, true> : k_sor32p2<0, false>)
+                               : (whole ? k_sor32p2<1, true> : k_sor32p2<1, false>);
+  cudaLaunchKernelEx(&cfg, kern, d, c->g, c->rp[color], c->ep[color], c->ep[1 - color], c->packed_lp, omega, om1, P,
+                     ka, kb);
 }
 
-// One red-black sweep with the colour-packed two-pass kernels.
-void launch_sor32_sweep(ib3d_ctx* c, float omega, float om1) {
-  if (c->prm.sweep_kernel == 0) {
-    launch_pass2(c, 0, omega, om1);
-    launch_pass2(c, 1, omega, om1);
-  } else {
-    launch_sor32_packed(c, 0, omega, om1);
-    launch_sor32_packed(c, 1, omega, om1);
+// How the sweeps of this grid go through it (SweepParts), planned on first use. The parts
+// are those of least cost among the splits that L2 holds, a launch costing what its
+// threads' march of planes costs, all waves, and kLaunchPlanes planes more for its start
+// and drain (2.5 us against 0.6 us a plane). Parts of full waves whatever their number
+// took 34.7 us per sweep at 256^3 (three parts), 30.5 with this rule (two).
+static const SweepParts& sweep_parts(ib3d_ctx* c) {
+  SweepParts& best = c->parts;
+  if (best.n) return best;
+  const Dims& d = c->d;
+  const size_t per_plane = 4 * sizeof(float) * (size_t)c->packed_lp * (size_t)d.NY2;
+  if (per_plane * (size_t)d.NZ2 <= kResidentMaxBytes) return best = {1, 0, d.nz, 1};
+  const int room = std::max(2, (int)(kPartBytes / per_plane) & ~1);
+  const int group = std::max(1, std::min(kGroup, room / 8));
+  const unsigned bx = slab_blocks(d);
+  const unsigned slots = 4u * (unsigned)c->nsm;
+  // planes that a thread of a pass over n planes marches through, all waves
+  auto march = [&](int n) {
+    if (n <= 0) return kLaunchPlanes;
+    const int P = slab_planes(c, bx, n);
+    const unsigned blocks = bx * (unsigned)((n + P - 1) / P);
+    return P * (int)((blocks + slots - 1) / slots) + kLaunchPlanes;
+  };
+  long long least = 0;
+  int most = d.nz + 2;
+  for (int n = 2; n <= most; ++n) {   // the fewest parts that L2 holds, or one more
+    bool fit = false;
+    for (int planes = room; planes >= 2; planes -= 2) {
+      const int ends = d.nz - (n - 2) * planes, first = (ends / 2 + 1) & ~1;
+      if (ends < 0) continue;
+      if (first + 2 * group > room) break;
+      fit = true;
+      long long cost = 0;
+      for (int shift = -2 * group; shift <= 2 * group; shift += 2)
+        cost += (n - 2) * march(planes) + march(first + shift) + march(ends - first - shift);
+      if (best.n == 0 || cost < least) {
+        best = {n, first, planes, group};
+        least = cost;
+      }
+      if (n == 2) break;   // no inner part
+    }
+    if (fit) most = std::min(most, n + 1);
   }
+  return best;
+}
+
+// nsweep red-black sweeps at (w[q].x, w[q].y). A grid beyond L2 is taken in parts: all passes of
+// a group of sweeps run on one part, whose planes then come from L2, before the next part
+// begins. Each pass of a part covers the planes of the pass before moved back by two, so that
+// it finds its neighbour planes as a pass over the whole grid would: at plane k the last
+// pass has reached k + 1, and the next one, in the part before, has stopped below k - 1. (One plane would
+// do; two keep a range's first plane even, which fixes the row phases.) The groups
+// take the parts upwards and downwards in turn, each starting where the last one ended.
+// Same bits as whole passes. Whole passes move 16 B per cell and sweep between DRAM and L2, which bounds them
+// (384x256x256: 55.5 us per sweep with the right-hand side loaded to leave L2 first, half of the
+// corrections marked to stay and passes in alternating directions); a group of sweeps in parts moves the
+// arrays about once: 47.1 us, and 126.5 -> 99.4 at 512x384x256, 31.7 -> 30.5 at 256^3. Returns
+// the launches.
+static int sweep_group(ib3d_ctx* c, int nsweep, const float2* w, bool up, const SweepParts& sp) {
+  const int nz = c->d.nz;
+  int launches = 0;
+  for (int t = 0; t < sp.n; ++t) {
+    const int part = up ? t : sp.n - 1 - t;
+    for (int p = 0; p < 2 * nsweep; ++p) {
+      const int shift = up ? 2 * (nsweep - p) : 2 * (p - nsweep);
+      auto bound = [&](int b) {
+        return b == 0 ? 0 : b == sp.n ? nz : std::min(std::max(sp.first + (b - 1) * sp.planes + shift, 0), nz);
+      };
+      const int ka = bound(part), kb = bound(part + 1);
+      if (ka >= kb) continue;
+      launch_pass2(c, p & 1, w[p >> 1].x, w[p >> 1].y, ka, kb);
+      ++launches;
+    }
+  }
+  return launches;
+}
+
+// n red-black sweeps with the colour-packed two-pass kernels, sweep q at (w[q].x, w[q].y).
+// Returns the launches.
+int launch_sor32_sweeps(ib3d_ctx* c, int n, const float2* w) {
+  int launches = 0;
+  if (c->prm.sweep_kernel == 0) {
+    const SweepParts& sp = sweep_parts(c);
+    bool up = true;
+    for (int q = 0; q < n; q += sp.group, up = !up) launches += sweep_group(c, std::min(sp.group, n - q), w + q, up, sp);
+  } else {
+    for (int q = 0; q < n; ++q, launches += 2) {
+      launch_sor32_packed(c, 0, w[q].x, w[q].y);
+      launch_sor32_packed(c, 1, w[q].x, w[q].y);
+    }
+  }
+  return launches;
 }
 
 // Sweeps per replay of the captured sweep graph: the host issues one graph launch
@@ -724,7 +748,9 @@ static bool ensure_sweep_graph(ib3d_ctx* c, float omega, float om1) {
     cudaGetLastError();
     return false;
   }
-  for (int q = 0; q < kGraphSweeps; ++q) launch_sor32_sweep(c, omega, om1);
+  float2 w[kGraphSweeps];
+  for (float2& x : w) x = make_float2(omega, om1);
+  c->sweep_launches = launch_sor32_sweeps(c, kGraphSweeps, w);
   cudaGraph_t graph = nullptr;
   const cudaError_t e = cudaStreamEndCapture(c->st, &graph);
   bool ok = e == cudaSuccess && graph != nullptr &&
@@ -743,16 +769,21 @@ static bool ensure_sweep_graph(ib3d_ctx* c, float omega, float om1) {
 }
 
 // n red-black sweeps at (omega, om1) with the colour-packed kernels: whole groups of
-// kGraphSweeps as replays of the captured graph, the rest launched directly.
-void run_sor32_sweeps(ib3d_ctx* c, int n, float omega, float om1) {
+// kGraphSweeps as replays of the captured graph, the rest launched directly. Returns the
+// kernel launches.
+int run_sor32_sweeps(ib3d_ctx* c, int n, float omega, float om1) {
+  int launches = 0;
   if (n >= kGraphSweeps && !c->sweep_graph_failed) {
     if (ensure_sweep_graph(c, omega, om1)) {
-      for (; n >= kGraphSweeps; n -= kGraphSweeps) cudaGraphLaunch(c->sweep_exec, c->st);
+      for (; n >= kGraphSweeps; n -= kGraphSweeps, launches += c->sweep_launches) cudaGraphLaunch(c->sweep_exec, c->st);
     } else {
       c->sweep_graph_failed = true;
     }
   }
-  for (; n > 0; --n) launch_sor32_sweep(c, omega, om1);
+  float2 w[kGraphSweeps];
+  for (float2& x : w) x = make_float2(omega, om1);
+  for (; n > 0; n -= kGraphSweeps) launches += launch_sor32_sweeps(c, std::min(n, kGraphSweeps), w);
+  return launches;
 }
 
 // Rows per block and stages of the staged sweep for a row of nq float4 groups: 16 rows

@@ -282,8 +282,8 @@ typedef struct ib3d_timers {
   int64_t outer;      /* defect-correction passes */
   int64_t launches;   /* kernels launched by the library */
   int64_t steps;      /* ib3d_step calls */
-  int64_t launches32; /* launches of the FP32 sweep kernel (one per colour pass, or one per
-                         group of fused sweeps) */
+  int64_t launches32; /* launches of the FP32 sweep kernels (one per colour pass, or per part of
+                         it beyond L2; one per fused sweep; one per pass of on-chip sweeps) */
 } ib3d_timers;
 /* on != 0 clears and starts the timers; on == 0 stops them (counts are kept). */
 int ib3d_timers_enable(ib3d_ctx* ctx, int on);

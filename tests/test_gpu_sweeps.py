@@ -149,3 +149,15 @@ def test_passes_read_the_last_pass_only(ib3d, grids, shape):
         got = _capped(ib3d, grids, shape, 75, b, sweep_kernel=kernel, smooth_sweeps=2, ramp_sweeps=5)
         assert got[0] == want[0]
         assert np.array_equal(got[1], want[1]), kernel
+
+
+# sweeps in parts (grids beyond L2): two parts and more, wide planes (a part is four planes, one sweep
+# a group, more blocks than one wave), parts that end off the grid; odd nz; groups cut short
+@pytest.mark.parametrize("shape,sweeps", [((1500, 1100, 9), 7), ((384, 256, 255), 43), ((512, 400, 151), 36),
+                                          ((300, 290, 301), 17)])
+def test_sweeps_in_parts_match_whole_passes(ib3d, grids, shape, sweeps):
+    b = _rhs(shape)
+    want = _capped(ib3d, grids, shape, sweeps, b, sweep_kernel=3, smooth_sweeps=2, ramp_sweeps=5)
+    got = _capped(ib3d, grids, shape, sweeps, b, sweep_kernel=0, smooth_sweeps=2, ramp_sweeps=5)
+    assert got[0] == want[0] == sweeps
+    assert np.array_equal(got[1], want[1])
