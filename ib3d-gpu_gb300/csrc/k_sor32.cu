@@ -688,8 +688,8 @@ static const SweepParts& sweep_parts(ib3d_ctx* c) {
 // take the parts upwards and downwards in turn, each starting where the last one ended.
 // Same bits as whole passes. Whole passes move 16 B per cell and sweep between DRAM and L2, which bounds them
 // (384x256x256: 55.5 us per sweep with the right-hand side loaded to leave L2 first, half of the
-// corrections marked to stay and passes in alternating directions); a group of sweeps in parts moves the
-// arrays about once: 47.1 us, and 126.5 -> 99.4 at 512x384x256, 31.7 -> 30.5 at 256^3. Returns
+// corrections marked to stay and passes in alternating directions); a group of sweeps in parts moves 45 MB a sweep
+// instead of 272: 47.1 us, and 126.5 -> 99.4 at 512x384x256, 31.7 -> 30.5 at 256^3. Returns
 // the launches.
 static int sweep_group(ib3d_ctx* c, int nsweep, const float2* w, bool up, const SweepParts& sp) {
   const int nz = c->d.nz;
