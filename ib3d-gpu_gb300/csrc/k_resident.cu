@@ -504,6 +504,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident64(Resident64 A) {
       }
       res = warp_max_bits(res);
       if ((t & 31) == 0 && res != 0) atomicMax(A.errs + sweep, res);
+      __syncthreads();   // the next red pass overwrites the values that the residual has read
     }
   }
   for (int it = t; it < items; it += nt) {

@@ -161,3 +161,28 @@ def test_sweeps_in_parts_match_whole_passes(ib3d, grids, shape, sweeps):
     got = _capped(ib3d, grids, shape, sweeps, b, sweep_kernel=0, smooth_sweeps=2, ramp_sweeps=5)
     assert got[0] == want[0] == sweeps
     assert np.array_equal(got[1], want[1])
+
+
+# several cells of a colour per thread, so that the warps of a block finish the residual of a
+# check apart: a red pass that began before all had read its cells would change the recorded
+# measure. Residuals at every sweep and at every third, to the cap (the goal out of reach) and
+# to the goal; the fast form against itself.
+@pytest.mark.parametrize("shape", [(96, 64, 64), (100, 75, 51)])
+@pytest.mark.parametrize("every,eps,cap", [(1, 1e-30, 48), (3, 1e-30, 50), (1, 0.01, 2000), (3, 0.01, 2000)])
+def test_fp64_on_chip_residuals_are_of_one_state(ib3d, grids, oracle_mod, shape, every, eps, cap):
+    x, y, z = (grids.tanh_axis(n) for n in shape)
+    b = _rhs(shape)
+    o = oracle_mod.Oracle(x, y, z, 100.0, 1.0, omega=1.7, eps=eps, criterion=1, max_sweeps=cap, check_every=every)
+    o.no_body()
+    o.set_field("b", b)
+    r = o.redblack_sor(allow_noconv=True)
+    p = ib3d.default_params(re=100.0, deltat=1.0, omega=1.7, eps=eps, max_sweeps=cap)
+    p.criterion, p.check_every = 1, every
+    with ib3d.Solver(x, y, z, p) as s:
+        s.set_field("b", b)
+        for _ in range(8):
+            g = s.redblack_sor(allow_noconv=True)
+            assert (g["sweeps"], g["final_err"]) == (r["sweeps"], r["final_err"])
+        s.set_params(precision=ib3d.PREC_FP64_FAST)
+        fast = {(f["sweeps"], f["final_err"]) for f in (s.redblack_sor(allow_noconv=True) for _ in range(8))}
+        assert len(fast) == 1, fast
