@@ -361,7 +361,8 @@ struct PhaseScope {
     if (_e != cudaSuccess) return ib3d::cuda_fail((c), _e, #expr);    \
   } while (0)
 
-// ---- device helpers ----
+// ---- device helpers (a host compiler that reads this file for its types has no use for them) ----
+#ifdef __CUDACC__
 namespace ib3d {
 // max that keeps a NaN (fmax would drop it), so that a NaN in a convergence
 // scalar reaches the host check instead of reading as "converged".
@@ -474,3 +475,4 @@ __device__ __forceinline__ float sor32_update(float e, float num, float diag, fl
   return fmaf(om1, e, (omega * num) * rcp_approx(diag));
 }
 }  // namespace ib3d
+#endif  // __CUDACC__

@@ -42,6 +42,12 @@ constexpr int kPollLimit = 1 << 20;       // about half a second
 constexpr int kMaxThreads = 512;
 constexpr size_t kSmemCap = 227 * 1024 - 1024;
 
+// The limit belongs to the kernel, not to a context: always the largest plan's, so that no
+// thread's launch meets another's smaller one.
+cudaError_t allow_smem(const void* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
+}
+
 __device__ __forceinline__ void st_pair(u64* p, u64 a, u64 b) {
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" :: "l"(p), "l"(a), "l"(b) : "memory");
 }
@@ -565,7 +571,7 @@ namespace {
 template <int NH>
 cudaError_t go32(const ResidentPlan& pl, Resident32& a, cudaStream_t st) {
   const void* k = (const void*)k_resident32<NH>;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+  const cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(k, dim3((unsigned)(pl.gy * pl.gz)), dim3((unsigned)pl.nt), args, pl.smem, st);
@@ -608,7 +614,7 @@ ResidentPlan plan_resident64(int nx, int ny, int nz, int nsm, bool exact) {
 cudaError_t launch_resident64(const ResidentPlan& pl, Resident64 a, bool exact, cudaStream_t st) {
   a.gy = pl.gy; a.gz = pl.gz; a.by = pl.by; a.bz = pl.bz;
   const void* k = exact ? (const void*)k_resident64<true> : (const void*)k_resident64<false>;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+  const cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(k, dim3((unsigned)(pl.gy * pl.gz)), dim3((unsigned)pl.nt), args, pl.smem, st);

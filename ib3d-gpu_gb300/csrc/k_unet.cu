@@ -772,6 +772,8 @@ __global__ void k_cast_conv_weights(int N, int K, const float* __restrict__ w, b
 
 // ------------------------------------------------------------ launch helpers
 
+// The most dynamic shared memory of a launch, and every kernel's limit: the limit belongs to the
+// kernel, so one set to a launch's own size could have another thread's launch refused.
 constexpr size_t kSmemMax = 227 * 1024 - 512;
 constexpr int kSms = 152;
 
@@ -795,7 +797,7 @@ void launch_conv3(cudaStream_t st, const Vol& vol, Act X, int K, const bf16* W, 
     cudaMemsetAsync(err, 1, sizeof(int), st);
     return;
   }
-  cudaFuncSetAttribute(k_conv3<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_conv3<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
   k_conv3<N><<<(unsigned)blocks(R), kConvThreads, smem, st>>>(seq, X, K, W, bias, relu, sign, Y, R, NX, NB, err);
 }
 
@@ -846,7 +848,7 @@ void wgrad(cudaStream_t st, const Vol& vol, Act dZ, int N, Act X, int K, float* 
     wgrad_cuda_cores(st, vol, dZ, N, X, K, dW);
     return;
   }
-  cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w.smem);
+  cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
   k_wgrad_tc<<<dim3((unsigned)w.gx, (unsigned)w.gy), kConvThreads, w.smem, st>>>(seq, dZ, N, X, K, work, w.nz, w.pairs,
                                                                                  w.stages, err);
   const int n = N * 27 * K;

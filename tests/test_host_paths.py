@@ -1,0 +1,61 @@
+"""Host code that a GPU test cannot reach -- allocations that fail, launches of several threads
+that interleave -- on a CUDA runtime that runs no kernel (fake_cuda.cpp)."""
+from __future__ import annotations
+
+import ctypes as C
+import pathlib
+import subprocess
+
+import numpy as np
+import pytest
+
+
+@pytest.fixture(scope="session")
+def fake_path(ib3d, tmp_path_factory):
+    pkg = pathlib.Path(ib3d.__file__).resolve().parent
+    from ib3d_gpu_gb300 import buildlib
+    objs = [pkg / "_build" / (pathlib.Path(s).stem + ".o") for s in buildlib.SOURCES]
+    newest = max(f.stat().st_mtime for f in buildlib.CSRC.iterdir())
+    if not all(o.exists() and o.stat().st_mtime >= newest for o in objs):
+        ib3d.build()
+    out = tmp_path_factory.mktemp("fake") / "libib3d_fake.so"
+    include = pathlib.Path(buildlib.nvcc()).resolve().parent.parent / "include"
+    subprocess.run(["g++", "-shared", "-fPIC", "-std=c++17", "-O1", "-Wl,-Bsymbolic", "-Wl,--no-undefined", "-I",
+                    str(include), "-I", str(buildlib.CSRC), "-o", str(out),
+                    str(pathlib.Path(__file__).resolve().parent / "fake_cuda.cpp"), *map(str, objs)], check=True)
+    return out
+
+
+@pytest.fixture
+def fake(ib3d, fake_path, monkeypatch):
+    """The package on the library linked with the fake runtime."""
+    monkeypatch.setattr(ib3d, "_lib", None)
+    monkeypatch.setattr(ib3d, "LIB_PATH", fake_path)
+    L = ib3d.lib()
+    L.fake_launches.restype = C.c_char_p
+    L.fake_launches()
+    return L
+
+
+def _solver(ib3d, grids, shape, precision=0, **kw):
+    p = ib3d.default_params(deltat=1.0, omega=1.7, eps=1e-6, max_sweeps=1000, precision=precision, criterion=1, **kw)
+    return ib3d.Solver(*(grids.tanh_axis(n) for n in shape), p)
+
+
+def test_shared_memory_limits_never_fall(ib3d, grids, fake):
+    """A kernel's limit of dynamic shared memory holds for all contexts and threads: a launch that
+    lowered it could have another thread's refused between its own two calls."""
+    before = fake.fake_lowered(), fake.fake_refused()
+    for shape in ((96, 64, 64), (24, 24, 24), (100, 75, 51), (5, 4, 4)):
+        for precision in (ib3d.PREC_FP64, ib3d.PREC_FP32DC, ib3d.PREC_FP64_FAST):
+            with _solver(ib3d, grids, shape, precision) as s:
+                s.redblack_sor()
+    net = ib3d.Net(seed=1)
+    for size in (32, 4):
+        x = np.zeros((1, size, size, size, 4), np.float32)
+        net.loss_grad(x, x[..., 0])
+    net.close()
+    names = fake.fake_launches().decode()
+    for kernel in ("k_resident32", "k_resident64", "k_conv3", "k_wgrad_tc"):
+        assert kernel in names
+    assert (fake.fake_lowered(), fake.fake_refused()) == before
