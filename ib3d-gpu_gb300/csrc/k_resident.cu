@@ -621,23 +621,38 @@ cudaError_t launch_resident64(const ResidentPlan& pl, Resident64 a, bool exact, 
 }
 
 // The exchange buffer of a context, at least `words` long, zeroed when it is new (pass
-// numbers start at 1).
+// numbers start at 1). The forms share it, so the old one stays until there is a larger one.
 static bool ensure_exchange(ib3d_ctx* c, size_t words) {
   if (words <= c->xch_words) return true;
-  cudaStreamSynchronize(c->st);
-  cudaFree(c->xch);
-  c->xch = nullptr;
-  c->xch_words = 0;
-  if (cudaMalloc(&c->xch, words * sizeof(u64)) != cudaSuccess ||
-      cudaMemsetAsync(c->xch, 0, words * sizeof(u64), c->st) != cudaSuccess) {
+  u64* p = nullptr;
+  if (cudaMalloc(&p, words * sizeof(u64)) != cudaSuccess ||
+      cudaMemsetAsync(p, 0, words * sizeof(u64), c->st) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(c->xch);
-    c->xch = nullptr;
+    cudaFree(p);
     return false;
   }
+  cudaStreamSynchronize(c->st);
+  cudaFree(c->xch);
+  c->xch = p;
   c->xch_words = words;
   c->xch_seq = 0;
   return true;
+}
+
+// The second array of the FP64 batches and their recorded measures: all of them, or none.
+constexpr int kBatch = 256;   // sweeps of an FP64 batch, at most
+static bool ensure_batches(ib3d_ctx* c) {
+  if (c->pc2) return true;
+  if (cudaMalloc(&c->pc2, (size_t)c->d.n3 * sizeof(double)) == cudaSuccess &&
+      cudaMalloc(&c->d_errs, (kBatch + 1) * sizeof(u64)) == cudaSuccess &&
+      cudaMallocHost(&c->h_errs, (kBatch + 1) * sizeof(u64)) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  cudaFree(c->pc2);
+  cudaFree(c->d_errs);
+  c->pc2 = nullptr;
+  c->d_errs = c->h_errs = nullptr;   // the last one of the three, so never there when one has failed
+  return false;
 }
 
 // One pass of the defect correction on chip: n FP32 sweeps on the packed right-hand side
@@ -708,7 +723,6 @@ static bool plain_diagonal(const ib3d_ctx* c) {
 // which the stopping test is met runs again from its input up to that sweep; the batches
 // grow to 256 sweeps and shrink as the measured rate says that the end is near.
 bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc) {
-  constexpr int kBatch = 256;
   ResidentPlan& pl = exact ? c->res64 : c->res64f;
   bool& planned = exact ? c->res64_planned : c->res64f_planned;
   if (!planned) {
@@ -716,14 +730,7 @@ bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc) {
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
     if (coop) pl = plan_resident64(c->d.nx, c->d.ny, c->d.nz, c->nsm, exact);
-    const size_t bytes = (size_t)c->d.n3 * sizeof(double);
-    if (pl.ok && !ensure_exchange(c, pl.xch_words)) pl.ok = false;
-    if (pl.ok && !c->pc2 &&
-        (cudaMalloc(&c->pc2, bytes) != cudaSuccess || cudaMalloc(&c->d_errs, (kBatch + 1) * sizeof(u64)) != cudaSuccess ||
-         cudaMallocHost(&c->h_errs, (kBatch + 1) * sizeof(u64)) != cudaSuccess)) {
-      cudaGetLastError();
-      pl.ok = false;
-    }
+    if (pl.ok && (!ensure_exchange(c, pl.xch_words) || !ensure_batches(c))) pl.ok = false;
   }
   if (!pl.ok || (exact && !plain_diagonal(c))) return false;
   const ib3d_params& P = c->prm;

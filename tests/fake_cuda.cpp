@@ -71,13 +71,18 @@ cudaError_t cudaMalloc(void** p, size_t n) { return allocate(p, n); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return allocate(p, n); }
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+  if (!d || !s) return cudaErrorInvalidValue;
   memcpy(d, s, n);
   return cudaSuccess;
 }
-cudaError_t cudaMemset(void* d, int v, size_t n) { memset(d, v, n); return cudaSuccess; }
-cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) { return cudaMemcpy(d, s, n, k); }
+cudaError_t cudaMemset(void* d, int v, size_t n) {
+  if (!d) return cudaErrorInvalidValue;
+  memset(d, v, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return cudaMemset(d, v, n); }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v) {
   if (limits.count(f) && v < limits[f]) ++lowered;
   limits[f] = v;

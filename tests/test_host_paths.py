@@ -59,3 +59,26 @@ def test_shared_memory_limits_never_fall(ib3d, grids, fake):
     for kernel in ("k_resident32", "k_resident64", "k_conv3", "k_wgrad_tc"):
         assert kernel in names
     assert (fake.fake_lowered(), fake.fake_refused()) == before
+
+
+@pytest.mark.parametrize("nth", [1, 2, 3, 4])
+def test_failed_allocation_of_one_form_leaves_the_others_sound(ib3d, grids, fake, nth):
+    """The on-chip forms share the exchange buffer, the two FP64 forms the second array and the
+    recorded measures. The n-th allocation of the first FP64 solve fails: that form launches per
+    pass, the others run on chip with every buffer they take."""
+    before = fake.fake_null_exchange()
+    with _solver(ib3d, grids, (21, 18, 16), ib3d.PREC_FP32DC) as s:
+        def solve(precision, kernel):
+            s.set_params(precision=precision)
+            s.redblack_sor()
+            assert kernel in fake.fake_launches().decode()
+
+        solve(ib3d.PREC_FP32DC, "k_resident32")
+        fake.fake_fail_in(nth)
+        solve(ib3d.PREC_FP64, "k_sor64")
+        assert fake.fake_pending_failure() == 0
+        solve(ib3d.PREC_FP32DC, "k_resident32")
+        solve(ib3d.PREC_FP64_FAST, "k_resident64")
+        solve(ib3d.PREC_FP64, "k_sor64")
+        solve(ib3d.PREC_FP32DC, "k_resident32")
+    assert fake.fake_null_exchange() == before
