@@ -39,6 +39,12 @@ struct Dims {
 // k_sor32.cu: (nx+1)/2 entries a row and colour, rounded up to whole groups).
 __host__ __device__ __forceinline__ int row_groups(int nx) { return (((nx + 1) >> 1) + 3) >> 2; }
 
+// The item of thread t of a block where four threads share an item. (The thread's own number,
+// divided by four, would wrap in 32 bits from 2^30 items on.)
+__host__ __device__ __forceinline__ unsigned quad_item(unsigned block, unsigned threads, unsigned t) {
+  return block * (threads >> 2) + (t >> 2);
+}
+
 // 1-D device tables; every pointer is 1-based (element 0 unused) unless noted.
 struct Grid1D {
   const double *x1, *y1, *z1, *dx, *dy, *dz;

@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kBlock) k_tagging(Dims d, Grid1D g, const doub
   __shared__ float qd[kQueue][kBlock];
   const int t = threadIdx.x, s = t & 3;  // four threads per cell, thread s its elements s, s + 4, ...
   const unsigned quad = (t & 31) & ~3u;
-  const unsigned tid = (blockIdx.x * blockDim.x + t) >> 2;
+  const unsigned tid = quad_item(blockIdx.x, blockDim.x, t);
   const unsigned ncell = list ? (unsigned)nlist : (unsigned)bni * (unsigned)bnj * (unsigned)bnk;
   const bool active = tid < ncell;
   const unsigned cid = active ? tid : 0;   // idle threads follow along on cell 0 and store nothing

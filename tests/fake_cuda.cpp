@@ -59,6 +59,7 @@ int fake_lowered() { return lowered; }           // limits set below an earlier 
 int fake_refused() { return refused; }           // launches above their kernel's limit
 int fake_null_exchange() { return null_exchange; }
 void fake_give_up(int on) { give_up = on; }      // on-chip sweeps report a wait that ran out
+unsigned fake_quad_item(unsigned block, unsigned threads, unsigned t) { return ib3d::quad_item(block, threads, t); }
 const char* fake_launches() {                    // kernels launched since the last call
   joined.clear();
   for (const auto& s : log_) joined += s + "\n";

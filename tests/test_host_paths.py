@@ -33,6 +33,7 @@ def fake(ib3d, fake_path, monkeypatch):
     monkeypatch.setattr(ib3d, "LIB_PATH", fake_path)
     L = ib3d.lib()
     L.fake_launches.restype = C.c_char_p
+    L.fake_quad_item.restype = C.c_uint
     L.fake_launches()
     return L
 
@@ -82,3 +83,12 @@ def test_failed_allocation_of_one_form_leaves_the_others_sound(ib3d, grids, fake
         solve(ib3d.PREC_FP64, "k_sor64")
         solve(ib3d.PREC_FP32DC, "k_resident32")
     assert fake.fake_null_exchange() == before
+
+
+# the first cells, the ones around 2^30 and the last cell of the largest box
+@pytest.mark.parametrize("cell", [0, 63, 64, 2 ** 30 - 1, 2 ** 30, 2 ** 30 + 12345, 2 ** 31 - 1])
+def test_four_threads_a_cell_reach_every_cell_of_a_large_box(fake, cell):
+    """k_tagging's numbering of cells, with its 256 threads a block."""
+    block = cell // 64
+    for lane in range(4):
+        assert fake.fake_quad_item(block, 256, 4 * (cell % 64) + lane) == cell
