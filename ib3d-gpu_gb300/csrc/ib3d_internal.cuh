@@ -124,6 +124,9 @@ struct SweepParts {
   int n, first, planes, group;
 };
 
+// Loads after which a block's wait for its neighbours' rows gives up: about half a second.
+constexpr int kPollLimit = 1 << 20;
+
 // How a grid's rows are split over the blocks of a resident kernel: gy x gz blocks of at
 // most by x bz rows (full x extent), nt threads (zl: FP32, planes a thread marches
 // through), smem bytes of shared memory, and the
@@ -207,6 +210,7 @@ struct ib3d_ctx {
   unsigned long long* xch = nullptr;
   size_t xch_words = 0;
   unsigned xch_seq = 0;
+  int polls = ib3d::kPollLimit;
   unsigned char* cell = nullptr;
   int* ibmap = nullptr;
   ib3d::SolveCtl* ctl = nullptr;

@@ -18,10 +18,13 @@
 // p + 1 from every neighbour, which that neighbour published after all its threads had
 // read pass p (one block barrier ends each pass).
 //
-// The blocks wait on one another, so the launch is cooperative (all blocks resident). A
-// poll gives up after a bounded number of loads, or when another block has: the block then
-// sets the error flag and every block returns without storing a result; nothing is in
-// flight by then. The kernels run on one stream at a time per exchange buffer.
+// The blocks wait on one another, so the launch is cooperative (all blocks resident, and started
+// together: a solve beside a kernel that held 100 SMs for 1.5 s began when it had ended). A
+// wait gives up after a bounded number of polls, or when another block has given up: the block
+// sets the error flag and returns without storing. A block whose last waits had already ended
+// stores its rows all the same, so the array that the launch writes is then part old, part new,
+// and the solve ends with an error. The words left behind carry numbers that no later launch
+// waits for. The kernels run on one stream at a time per exchange buffer.
 //
 // Compiled with -fmad=false: the FP64 kernel keeps the reference's rounding.
 #include <algorithm>
@@ -38,7 +41,6 @@ namespace {
 typedef unsigned long long u64;
 
 constexpr int kHalo = 4;                  // received items per thread, at most
-constexpr int kPollLimit = 1 << 20;       // about half a second
 constexpr int kMaxThreads = 512;
 constexpr size_t kSmemCap = 227 * 1024 - 1024;
 
@@ -259,6 +261,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident32(Resident32 A) {
 #pragma unroll
         for (int n = 0; n < NH; ++n) pend |= hdst[n] >= 0 ? 1u << n : 0u;
         for (int it = 0; pend != 0; ++it) {
+          if (it >= A.polls || ((it & 255) == 255 && ld_flag(A.err) != 0)) {
+            fail = true;
+            break;
+          }
           u64 v[NH][4];
 #pragma unroll
           for (int n = 0; n < NH; ++n)
@@ -277,10 +283,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident32(Resident32 A) {
                 pend &= ~(1u << n);
               }
             }
-          if (pend != 0 && (it & 255) == 255 && (it > kPollLimit || ld_flag(A.err) != 0)) {
-            fail = true;
-            break;
-          }
         }
       }
       if (__syncthreads_or(fail)) {
@@ -454,6 +456,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident64(Resident64 A) {
 #pragma unroll
       for (int n = 0; n < kHalo; ++n) pend |= hdst[n] >= 0 ? 1u << n : 0u;
       for (int it = 0; pend != 0; ++it) {
+        if (it >= A.polls || ((it & 255) == 255 && ld_flag(A.err) != 0)) {
+          fail = true;
+          break;
+        }
         u64 v[kHalo][2];
 #pragma unroll
         for (int n = 0; n < kHalo; ++n)
@@ -464,10 +470,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident64(Resident64 A) {
             Ec[hdst[n]] = __longlong_as_double((long long)((v[n][1] << 32) | (v[n][0] & 0xffffffffull)));
             pend &= ~(1u << n);
           }
-        if (pend != 0 && (it & 255) == 255 && (it > kPollLimit || ld_flag(A.err) != 0)) {
-          fail = true;
-          break;
-        }
       }
       if (__syncthreads_or(fail)) {
         if (t == 0) atomicExch(A.err, 1);
@@ -690,6 +692,7 @@ bool run_resident32(ib3d_ctx* c, int n, int nsmooth, int nramp, double wi, float
   a.om = om;
   a.om1 = om1;
   a.err = &c->ctl->stage_err;
+  a.polls = c->polls;
   if (launch_resident32(c->res32, a, c->st) != cudaSuccess) {
     cudaGetLastError();
     c->res32.ok = false;
@@ -752,6 +755,7 @@ bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc) {
   a.om1 = 1.0 - P.omega;
   a.errs = c->d_errs;
   a.err = reinterpret_cast<int*>(c->d_errs + kBatch);
+  a.polls = c->polls;
   rc = IB3D_ERR_CUDA;
   auto failed = [&](const char* what) {
     c->err = what;

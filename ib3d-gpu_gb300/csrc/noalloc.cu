@@ -250,6 +250,7 @@ int run_noalloc(const ResidentPlan* plan, int64_t nx, int64_t ny, int64_t nz, co
     res.om = (float)omega;
     res.om1 = (float)(1.0 - omega);
     res.err = &ctl->stage_err;
+    res.polls = kPollLimit;
     // the rows' entries past their last cell stay NaN; the pass numbers start over
     if (cudaMemsetAsync(r32, 0xff, 2 * half * sizeof(float), st) != cudaSuccess) return IB3D_ERR_CUDA;
     if (cudaMemsetAsync(res.xch, 0, plan->xch_words * 8, st) != cudaSuccess) return IB3D_ERR_CUDA;

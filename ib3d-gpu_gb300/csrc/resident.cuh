@@ -23,6 +23,7 @@ struct Resident32 {
   double wi;
   float om, om1;
   int* err;                             // set when a wait gave up
+  int polls;                            // loads after which a wait gives up
 };
 cudaError_t launch_resident32(const ResidentPlan& pl, Resident32 a, cudaStream_t st);
 
@@ -42,7 +43,8 @@ struct Resident64 {
   long long sweep0;                     // sweeps of the solve before this launch
   double omega, om1;
   unsigned long long* errs;             // [nsweeps] largest update or residual (bit pattern)
-  int* err;
+  int* err;                             // as in Resident32
+  int polls;
 };
 cudaError_t launch_resident64(const ResidentPlan& pl, Resident64 a, bool exact, cudaStream_t st);
 

@@ -33,7 +33,8 @@ extern "C" {
 
 #define IB3D_OK 0
 #define IB3D_ERR_ARG (-1)       /* bad argument / call order */
-#define IB3D_ERR_CUDA (-2)      /* CUDA runtime error or missing device */
+#define IB3D_ERR_CUDA (-2)      /* CUDA runtime error or missing device, or a bounded wait inside a kernel
+                                   that gave up; after a solve that returns it pc is undefined */
 #define IB3D_ERR_MESH (-3)      /* bad triangle index or degenerate mesh */
 #define IB3D_ERR_PROBE (-4)     /* a ghost-point or drag probe left the grid */
 #define IB3D_ERR_NOCONV (-5)    /* SOR hit max_sweeps; fields stay valid */
@@ -377,7 +378,8 @@ int ib3d_attach_net(ib3d_ctx* ctx, ib3d_net* net);
  * FP64 residual L-inf drops below eps (IB3D_ERR_NOCONV after max_sweeps). acx/acy/acz
  * are the (n,3) column-major Poisson coefficients of coefficientMatrix
  * (subCoefficientMatrix.f90:1-59); cell, b and pc are (nx+2,ny+2,nz+2) arrays in the
- * reference's layout (cell as uint8). stream is a cudaStream_t or NULL.
+ * reference's layout (cell as uint8). stream is a cudaStream_t or NULL. After
+ * IB3D_ERR_CUDA pc is undefined: part of a pass may have been added to it.
  *
  * Limit: (nx+2)*(ny+2)*(nz+2) <= 2^21 cells (two 8 MiB FP32 arrays); larger grids
  * (and any extent above 2^21) return IB3D_ERR_TOO_LARGE before any CUDA call. The

@@ -186,3 +186,44 @@ def test_fp64_on_chip_residuals_are_of_one_state(ib3d, grids, oracle_mod, shape,
         s.set_params(precision=ib3d.PREC_FP64_FAST)
         fast = {(f["sweeps"], f["final_err"]) for f in (s.redblack_sor(allow_noconv=True) for _ in range(8))}
         assert len(fast) == 1, fast
+
+
+@pytest.fixture(scope="module")
+def set_polls(ib3d, tmp_path_factory):
+    """Sets the loads after which a context's waits for neighbouring rows give up."""
+    import ctypes as C
+    import pathlib
+    import subprocess
+    from ib3d_gpu_gb300 import buildlib
+    d = tmp_path_factory.mktemp("polls")
+    (d / "polls.cpp").write_text('#include "ib3d_internal.cuh"\n'
+                                 'extern "C" int set_polls(ib3d_ctx* c, int n) { const int o = c->polls; c->polls = n; return o; }\n')
+    include = pathlib.Path(buildlib.nvcc()).resolve().parent.parent / "include"
+    subprocess.run(["g++", "-shared", "-fPIC", "-std=c++17", "-I", str(include), "-I", str(buildlib.CSRC), "-o",
+                    str(d / "polls.so"), str(d / "polls.cpp")], check=True)
+    f = C.CDLL(str(d / "polls.so")).set_polls
+    f.argtypes, f.restype = [C.c_void_p, C.c_int], C.c_int
+    return f
+
+
+# blocks split both ways; the error is reported, and the next solve on the same exchange buffer
+# has the bits of a solve that never failed
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("criterion", [0, 1])
+def test_wait_that_gives_up_ends_the_solve_with_an_error(ib3d, grids, set_polls, precision, criterion):
+    shape = (40, 33, 31)
+    x, y, z = (grids.tanh_axis(n) for n in shape)
+    p = ib3d.default_params(re=100.0, deltat=1.0, omega=1.7, eps=1e-4, max_sweeps=5000)
+    p.precision, p.criterion, p.inner_sweeps = precision, 1 if precision == 1 else criterion, 32
+    with ib3d.Solver(x, y, z, p) as s:
+        s.set_field("b", _rhs(shape))
+        want = s.redblack_sor(), s.get_field("pc")
+        usual = set_polls(s._h, 0)
+        for _ in range(2):
+            with pytest.raises(ib3d.IB3DError) as e:
+                s.redblack_sor()
+            assert e.value.code == ib3d.ERR_CUDA and "gave up" in str(e.value)
+        set_polls(s._h, usual)
+        got = s.redblack_sor(), s.get_field("pc")
+    assert (got[0]["sweeps"], got[0]["final_err"]) == (want[0]["sweeps"], want[0]["final_err"])
+    assert np.array_equal(got[1], want[1])
