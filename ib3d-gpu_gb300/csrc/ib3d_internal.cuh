@@ -190,9 +190,10 @@ struct ib3d_ctx {
   // sweep reads ep[] and writes epn[], then the pairs swap
   float* epn[2] = {nullptr, nullptr};
   // CUDA graph of kGraphSweeps FP32 sweeps of the colour-packed kernels (k_sor32.cu),
-  // with the tables, relaxation and kernel choice it was captured with
+  // with the tables, corrections, relaxation and kernel choice it was captured with
   cudaGraphExec_t sweep_exec = nullptr;
   ib3d::Grid1D sweep_g{};
+  const float* sweep_ep[2] = {nullptr, nullptr};
   float sweep_w = 0.f, sweep_w1 = 0.f;
   int sweep_kern = -1, sweep_launches = 0;
   ib3d::SweepParts parts{0, 0, 0, 0};

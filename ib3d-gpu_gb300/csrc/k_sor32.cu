@@ -733,12 +733,12 @@ int launch_sor32_sweeps(ib3d_ctx* c, int n, const float2* w) {
 constexpr int kGraphSweeps = 32;
 
 // Captures kGraphSweeps sweeps at (omega, om1) as a CUDA graph on the context's
-// stream, unless the cached one was captured with the same tables, relaxation and
-// kernel choice. Returns false when capture or instantiation fails (the caller then
+// stream, unless the cached one was captured with the same tables, arrays (fused sweeps
+// swap them), relaxation and kernel choice. Returns false when capture or instantiation fails (the caller then
 // launches the sweeps one by one).
 static bool ensure_sweep_graph(ib3d_ctx* c, float omega, float om1) {
   if (c->sweep_exec && c->sweep_w == omega && c->sweep_w1 == om1 && c->sweep_kern == c->prm.sweep_kernel &&
-      std::memcmp(&c->sweep_g, &c->g, sizeof(Grid1D)) == 0)
+      c->sweep_ep[0] == c->ep[0] && c->sweep_ep[1] == c->ep[1] && std::memcmp(&c->sweep_g, &c->g, sizeof(Grid1D)) == 0)
     return true;
   if (c->sweep_exec) {
     cudaGraphExecDestroy(c->sweep_exec);
@@ -764,6 +764,8 @@ static bool ensure_sweep_graph(ib3d_ctx* c, float omega, float om1) {
   c->sweep_w = omega;
   c->sweep_w1 = om1;
   c->sweep_kern = c->prm.sweep_kernel;
+  c->sweep_ep[0] = c->ep[0];
+  c->sweep_ep[1] = c->ep[1];
   c->sweep_g = c->g;
   return true;
 }

@@ -227,3 +227,22 @@ def test_wait_that_gives_up_ends_the_solve_with_an_error(ib3d, grids, set_polls,
         got = s.redblack_sor(), s.get_field("pc")
     assert (got[0]["sweeps"], got[0]["final_err"]) == (want[0]["sweeps"], want[0]["final_err"])
     assert np.array_equal(got[1], want[1])
+
+
+# kernel 0 beyond the on-chip sizes, and the forms that never run on chip
+@pytest.mark.parametrize("kernel,shape", [(3, (40, 33, 31)), (4, (40, 33, 31)), (0, (256, 192, 192))])
+def test_captured_sweeps_follow_the_arrays_that_fused_sweeps_swap(ib3d, grids, kernel, shape):
+    """An odd number of fused sweeps leaves the corrections in the other pair of arrays; the
+    sweeps captured before must not be replayed on the first pair."""
+    x, y, z = (grids.tanh_axis(n) for n in shape)
+    p = ib3d.default_params(re=100.0, deltat=1.0, omega=1.85, eps=1e-30, max_sweeps=75)
+    p.precision, p.criterion, p.inner_sweeps, p.sweep_kernel = ib3d.PREC_FP32DC, 1, 35, kernel
+    with ib3d.Solver(x, y, z, p) as s:
+        s.set_field("b", _rhs(shape))
+        s.redblack_sor(allow_noconv=True)
+        want = s.get_field("pc")
+        s.set_params(sweep_kernel=2, max_sweeps=35)
+        s.redblack_sor(allow_noconv=True)
+        s.set_params(sweep_kernel=kernel, max_sweeps=75)
+        s.redblack_sor(allow_noconv=True)
+        assert np.array_equal(s.get_field("pc"), want)
