@@ -729,14 +729,12 @@ __global__ void __launch_bounds__(256) k_head_bwd(long long M, Act in, const flo
 __global__ void __launch_bounds__(256) k_mse(long long M, const float* __restrict__ out, const float* __restrict__ t,
                                              float* __restrict__ g, double* loss) {
   __shared__ double s[8];
-  double a = 0.0;
-  float f = 0.f;   // a few voxels in FP32, the threads' and blocks' sums in FP64
+  double a = 0.0;   // FP32 squares, added in FP64: a thread's voxels grow with the batch
   for (long long m = (long long)blockIdx.x * 256 + threadIdx.x; m < M; m += (long long)gridDim.x * 256) {
     const float d = out[m] - t[m];
     g[m] = 2.f * d / (float)M;
-    f += d * d;
+    a += (double)(d * d);
   }
-  a = (double)f;
   for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = a;
   __syncthreads();

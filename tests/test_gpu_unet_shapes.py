@@ -49,3 +49,24 @@ def test_strips_give_the_bits_of_whole_rows(ib3d):
     a, b = np.s_[52:84], np.s_[32:64]
     assert np.array_equal(whole[:, a, a, a], crop[:, b, b, b])
     net.close()
+
+
+# several voxels a thread; the smallest; a batch
+@pytest.mark.parametrize("batch,size", [(1, 4), (1, 108), (3, 64)])
+def test_loss_adds_voxels_in_fp64(ib3d, batch, size):
+    """A zero head gives an output of 0, so a constant target t leaves one FP32 square, t * t rounded,
+    a voxel: their mean is that square. The FP64 additions of at most 150 terms a thread, 5 + 8 a
+    block and one a block into the total (1,024 blocks at most), and the quotients, are off by less
+    than 2,000 * 2^-53 of it."""
+    net = ib3d.Net(seed=3)
+    _, head = layout()
+    p = net.get_params()
+    p[head:head + 17] = 0.0
+    net.set_params(p)
+    x = np.random.default_rng(0).standard_normal((batch, size, size, size, 4)).astype(np.float32)
+    t = np.float32(0.7)
+    loss, _, out = net.loss_grad(x, np.full(x.shape[:4], t, np.float32))
+    net.close()
+    assert not out.any()
+    square = float(t * t)
+    assert abs(loss - square) <= 2000 * 2.0 ** -53 * square
