@@ -636,6 +636,7 @@ int ib3d_set_mesh(ib3d_ctx* c, int64_t nnodes, const double* xn, const double* y
     c->d_nodes = nullptr; c->d_tri = nullptr; c->d_surf = nullptr; c->d_scache = nullptr; c->d_contrib = nullptr;
     c->nodes_cap = c->elems_cap = 0;
     c->nnodes = c->nelems = 0;
+    c->searched = c->retag_ok = c->have_scache = false;   // should an allocation fail, no kernel runs on what is left
     IB3D_CUDA(c, cudaMalloc(&c->d_nodes, (size_t)3 * nnodes * sizeof(double)));
     IB3D_CUDA(c, cudaMalloc(&c->d_tri, (size_t)3 * nelems * sizeof(int)));
     IB3D_CUDA(c, cudaMalloc(&c->d_scache, (size_t)15 * nelems * sizeof(int)));
@@ -692,7 +693,10 @@ int ib3d_search(ib3d_ctx* c, const int64_t box[6], int64_t counts[5]) {
   for (int q = 0; q < 6; ++q) c->box[q] = box[q];
   c->retag_ok = false;
   int rc = run_search(c);
-  if (rc) return rc;
+  if (rc) {
+    if (rc != IB3D_ERR_PROBE) c->searched = false;   // arrays of the earlier search may be gone
+    return rc;
+  }
   c->searched = true;
   c->retag_ok = true;
   if (counts)
@@ -706,7 +710,10 @@ int ib3d_selective_retag(ib3d_ctx* c, int64_t counts[5]) {
     return fail(c, IB3D_ERR_ARG, "ib3d_selective_retag: needs the IB cells of an earlier search of this mesh");
   c->retag_ok = false;
   int rc = run_selective_retag(c);
-  if (rc) return rc;
+  if (rc) {
+    if (rc != IB3D_ERR_PROBE) c->searched = false;
+    return rc;
+  }
   c->searched = true;
   c->retag_ok = c->nib > 0;
   if (counts)

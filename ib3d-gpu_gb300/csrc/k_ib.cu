@@ -1098,8 +1098,9 @@ int ensure_scan(ib3d_ctx* c, size_t n) {
   if (n + 9 > c->scan_cap) {
     cudaFree(c->d_scan);
     c->d_scan = nullptr;
+    c->scan_cap = 0;
+    IB3D_CUDA(c, cudaMalloc(&c->d_scan, sizeof(long long) * (n + 64)));
     c->scan_cap = n + 64;
-    IB3D_CUDA(c, cudaMalloc(&c->d_scan, sizeof(long long) * c->scan_cap));
   }
   return IB3D_OK;
 }
@@ -1185,9 +1186,11 @@ int run_selective_retag(ib3d_ctx* c) {
     cudaFree(c->d_retag_list);
     c->d_retag_mask = nullptr;
     c->d_retag_list = nullptr;
-    c->retag_cap = (size_t)nbox + (size_t)nbox / 4;
-    IB3D_CUDA(c, cudaMalloc(&c->d_retag_mask, c->retag_cap));
-    IB3D_CUDA(c, cudaMalloc(&c->d_retag_list, 3 * sizeof(int) * c->retag_cap));
+    c->retag_cap = 0;
+    const size_t n = (size_t)nbox + (size_t)nbox / 4;
+    IB3D_CUDA(c, cudaMalloc(&c->d_retag_mask, n));
+    IB3D_CUDA(c, cudaMalloc(&c->d_retag_list, 3 * sizeof(int) * n));
+    c->retag_cap = n;
   }
   IB3D_CUDA(c, cudaMemsetAsync(c->d_retag_mask, 0, nbox, c->st));
   k_mark_neighbourhoods<<<nblk(216ll * nib), kBlock, 0, c->st>>>(c->d_iblist, nib, bi0, bj0, bk0, bni, bnj, bnk,
@@ -1220,6 +1223,8 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
   const Dims& d = c->d;
   const unsigned nbox = (unsigned)bni * bnj * bnk;
   const int ne = (int)c->nelems;
+  const unsigned nb = nblk(nbox);
+  if (int rc = ensure_scan(c, nb)) return rc;
   IB3D_CUDA(c, cudaMemsetAsync(c->ibmap, 0xff, sizeof(int) * (size_t)d.n3, c->st));
   // counts
   unsigned long long* dcount = reinterpret_cast<unsigned long long*>(c->d_scan);
@@ -1233,8 +1238,6 @@ int finish_search(ib3d_ctx* c, int bi0, int bj0, int bk0, int bni, int bnj, int 
   const int nib = c->nib;
   // compaction of the IB cells
   if (int rc = ensure_ib(c, (size_t)nib)) return rc;
-  const unsigned nb = nblk(nbox);
-  if (int rc = ensure_scan(c, nb)) return rc;
   long long* boff = c->d_scan + 8;
   k_ib_blockcount<<<nb, kBlock, 0, c->st>>>(d, c->cell, bi0, bj0, bk0, bni, bnj, nbox, boff);
   k_exclusive_scan<<<1, 1024, 0, c->st>>>(boff, (int)nb, c->d_scan);

@@ -92,3 +92,47 @@ def test_four_threads_a_cell_reach_every_cell_of_a_large_box(fake, cell):
     block = cell // 64
     for lane in range(4):
         assert fake.fake_quad_item(block, 256, 4 * (cell % 64) + lane) == cell
+
+
+def _forcing_is_refused(ib3d, s):
+    for call in (s.velocity_forcing, s.pressure_forcing, lambda: s.stress(True), lambda: s.step(True)):
+        with pytest.raises(ib3d.IB3DError) as e:
+            call()
+        assert e.value.code == ib3d.ERR_ARG
+
+
+@pytest.mark.parametrize("nth", [1, 4, 7])
+def test_failed_mesh_ends_the_earlier_search(ib3d, grids, fake, nth):
+    """A larger mesh whose arrays cannot be allocated leaves none: what was searched for the
+    earlier mesh must not be run on them. The next mesh that fits is searched as ever."""
+    cs = grids.case("tiny")
+    with ib3d.Solver(cs.x, cs.y, cs.z, ib3d.default_params()) as s:
+        s.set_mesh(*grids.icosphere(1, 0.5))
+        s.search(cs.box)
+        s.velocity_forcing()
+        fake.fake_fail_in(nth)
+        with pytest.raises(ib3d.IB3DError) as e:
+            s.set_mesh(*grids.icosphere(2, 0.5))
+        assert e.value.code == ib3d.ERR_CUDA
+        _forcing_is_refused(ib3d, s)
+        s.set_mesh(*grids.icosphere(2, 0.5))
+        s.search(cs.box)
+        s.velocity_forcing()
+
+
+@pytest.mark.parametrize("nth", [1, 2])
+def test_failed_search_ends_the_earlier_search(ib3d, grids, fake, nth):
+    """The same for a search whose larger box finds no room for its cells' nearest elements, or for
+    its scan."""
+    z = np.arange(161) * 0.05
+    small = [10, 20, 10, 20, 10, 20]
+    with ib3d.Solver(z, z, z, ib3d.default_params()) as s:
+        s.set_mesh(*grids.icosphere(1, 0.5))
+        s.search(small)
+        fake.fake_fail_in(nth)
+        with pytest.raises(ib3d.IB3DError) as e:
+            s.search([1, s.nx + 2, 1, s.ny + 2, 1, s.nz + 2])
+        assert e.value.code == ib3d.ERR_CUDA and fake.fake_pending_failure() == 0
+        _forcing_is_refused(ib3d, s)
+        s.search(small)
+        s.velocity_forcing()
