@@ -262,20 +262,10 @@ int alloc_fields(ib3d_ctx* c) {
   }
   if (cudaMalloc(&c->e32, n3 * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMalloc(&c->r32, n3 * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
-  // colour-packed arrays of the FP32 inner solve; the sweep kernels use 32-bit offsets, and
-  // an odd nx whose packed rows exceed them (a row of few cells is mostly padding) keeps
-  // the padded layout
   c->packed_lp = packed_row_length(c->d.nx);
   const size_t np = (size_t)c->packed_lp * (size_t)c->d.NY2 * (size_t)c->d.NZ2;
-  if (np >= ((size_t)1 << 31) && c->d.nx % 2 == 0) return IB3D_ERR_TOO_LARGE;
-  if (np < ((size_t)1 << 31)) {
-    for (int q = 0; q < 2; ++q) {
-      if (cudaMalloc(&c->ep[q], np * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
-      if (cudaMalloc(&c->rp[q], np * sizeof(float)) != cudaSuccess) return IB3D_ERR_MEMORY;
-      cudaMemsetAsync(c->ep[q], 0, np * sizeof(float), c->st);
-      cudaMemsetAsync(c->rp[q], 0xff, np * sizeof(float), c->st);   // all-ones bits: NaN
-    }
-  }
+  const bool odd = c->d.nx % 2 != 0;
+  if (np >= ((size_t)1 << 31) && !odd) return IB3D_ERR_TOO_LARGE;   // the sweep kernels use 32-bit offsets
   if (cudaMalloc(&c->cell, n3) != cudaSuccess) return IB3D_ERR_MEMORY;
   if (cudaMalloc(&c->ibmap, n3 * sizeof(int)) != cudaSuccess) return IB3D_ERR_MEMORY;
   cudaMemsetAsync(c->e32, 0, n3 * sizeof(float), c->st);
@@ -295,6 +285,26 @@ int alloc_fields(ib3d_ctx* c) {
   c->scan_cap = 64;
   if (cudaMalloc(&c->d_scan, c->scan_cap * sizeof(long long)) != cudaSuccess) return IB3D_ERR_MEMORY;
   cudaMemsetAsync(c->ctl, 0, sizeof(SolveCtl), c->st);
+  // colour-packed arrays of the FP32 inner solve, after what every grid needs: an odd nx whose
+  // packed rows exceed the kernels' offsets (a row of few cells is mostly padding), or whose
+  // arrays find no room, keeps the padded layout
+  if (np >= ((size_t)1 << 31)) return IB3D_OK;
+  float** packed[] = {&c->ep[0], &c->rp[0], &c->ep[1], &c->rp[1]};
+  for (float** q : packed)
+    if (cudaMalloc(q, np * sizeof(float)) != cudaSuccess) {
+      *q = nullptr;
+      if (!odd) return IB3D_ERR_MEMORY;
+      cudaGetLastError();
+      for (float** r : packed) {
+        cudaFree(*r);
+        *r = nullptr;
+      }
+      return IB3D_OK;
+    }
+  for (int q = 0; q < 2; ++q) {
+    cudaMemsetAsync(c->ep[q], 0, np * sizeof(float), c->st);
+    cudaMemsetAsync(c->rp[q], 0xff, np * sizeof(float), c->st);   // all-ones bits: NaN
+  }
   return IB3D_OK;
 }
 

@@ -136,3 +136,33 @@ def test_failed_search_ends_the_earlier_search(ib3d, grids, fake, nth):
         _forcing_is_refused(ib3d, s)
         s.search(small)
         s.velocity_forcing()
+
+
+@pytest.mark.parametrize("nth", [1, 2, 3, 4])
+def test_odd_rows_fall_back_to_the_padded_layout(ib3d, grids, fake, nth):
+    """A grid of odd nx needs no packed arrays: where one of the four finds no room, the context is
+    created without them and solves in the padded layout. An even nx is refused, as ever."""
+    import re
+    axes = lambda *n: [grids.tanh_axis(k) for k in n]
+    kw = dict(precision=ib3d.PREC_FP32DC, criterion=1, inner_sweeps=32, max_sweeps=100)
+    packed = []   # the allocations that may fail
+    for k in range(1, 60):
+        fake.fake_fail_in(k)
+        try:
+            ib3d.Solver(*axes(21, 18, 16), **kw).close()
+            if fake.fake_pending_failure() == 0:
+                packed.append(k)
+        except ib3d.IB3DError as e:
+            assert e.code == ib3d.ERR_MEMORY
+    assert len(packed) == 4, packed
+    fake.fake_fail_in(packed[nth - 1])
+    with ib3d.Solver(*axes(21, 18, 16), **kw) as s:
+        assert fake.fake_pending_failure() == 0
+        fake.fake_launches()
+        s.redblack_sor()
+        names = fake.fake_launches().decode()
+        assert re.search(r"k_sor32ILi0", names) and "k_resident32" not in names
+    fake.fake_fail_in(packed[nth - 1])
+    with pytest.raises(ib3d.IB3DError) as e:
+        ib3d.Solver(*axes(20, 18, 16), **kw)
+    assert e.value.code == ib3d.ERR_MEMORY
