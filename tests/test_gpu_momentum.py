@@ -68,3 +68,34 @@ def test_contracted_predictor_agrees_to_rounding(ib3d, grids, shape, ab):
         assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
         assert np.any(got != 0.0)
     s.close()
+
+
+@pytest.mark.parametrize("ab", [0, 1])
+@pytest.mark.parametrize("kind", ["sizes", "infinite"])
+def test_predictor_keeps_the_signs_of_zeros(ib3d, grids, oracle_mod, kind, ab):
+    """Bit patterns, with one for all NaNs: fields of signed zeros almost everywhere, so that
+    predicted values are zeros of both signs too."""
+    x, y, z = (grids.tanh_axis(n) for n in (33, 12, 9))
+    s = ib3d.Solver(x, y, z, ib3d.default_params(re=100.0, deltat=0.01, momentum=ab))
+    o = oracle_mod.Oracle(x, y, z, 100.0, 0.01, momentum=ab)
+    o.no_body()
+    rng = np.random.default_rng(7)
+    for k, f in enumerate(("u", "v", "w", "p", "ut", "vt", "wt")):
+        a = _field(s.shape, kind, 40 + k)
+        a = np.where(rng.integers(0, 40, s.shape) == 0, a, np.copysign(0.0, rng.standard_normal(s.shape)))
+        a[:, :, :5] = np.copysign(0.0, -1.0)   # a region of negative zeros alone
+        a = np.asfortranarray(a)
+        s.set_field(f, a)
+        o.set_field(f, a)
+
+    def bits(a):
+        return np.where(np.isnan(a), np.uint64(0x7FF8000000000000), a.view(np.uint64))
+    for _ in range(2):
+        for m in (s, o):
+            (m.ns_momentum_ab if ab else m.ns_momentum)()
+        for f in ("ut", "vt", "wt"):
+            got, want = s.get_field(f), o.get_field(f)
+            np.testing.assert_array_equal(bits(got), bits(want), f)
+    inner = want[1:-1, 1:-1, 1:-1]
+    assert np.any((inner == 0) & np.signbit(inner)) or np.any((inner == 0) & ~np.signbit(inner))
+    s.close()

@@ -246,3 +246,59 @@ def test_captured_sweeps_follow_the_arrays_that_fused_sweeps_swap(ib3d, grids, k
         s.set_params(sweep_kernel=kernel, max_sweeps=75)
         s.redblack_sor(allow_noconv=True)
         assert np.array_equal(s.get_field("pc"), want)
+
+
+def _sweeps_by_hand(a, b, pc, fluid, omega, sweeps):
+    """The reference's red-black sweeps in numpy, each operation rounded as the kernels round it:
+    pc, the last sweep's largest update, the residual's largest value."""
+    i = np.s_[1:-1]
+    ax, ay, az = ([v[:, q].reshape(s) for q in range(3)] for v, s in zip(a, ((-1, 1, 1), (1, -1, 1), (1, 1, -1))))
+    diag = ax[1] + ay[1] + az[1]
+    odd = np.indices(fluid.shape).sum(0) % 2 == 1     # 0-based interior indices: i + j + k is odd for the same cells
+    pc = pc.copy(order="F")
+
+    def num():
+        n = b[i, i, i] - ax[0] * pc[:-2, i, i] - ax[2] * pc[2:, i, i]
+        n = n - ay[0] * pc[i, :-2, i] - ay[2] * pc[i, 2:, i]
+        return n - az[0] * pc[i, i, :-2] - az[2] * pc[i, i, 2:]
+    for _ in range(sweeps):
+        largest = 0.0
+        for colour in (odd, ~odd):
+            c = pc[i, i, i]
+            new = np.where(fluid & colour, (1.0 - omega) * c + omega * (num() / diag), c)
+            largest = max(largest, np.abs(new - c).max())
+            pc[i, i, i] = new
+    return pc, largest, np.abs(num() - diag * pc[i, i, i])[fluid].max()
+
+
+# solid and immersed-boundary cells across the blocks' edges in y and z, and a start from a given
+# pc whose ghost, solid and fluid cells are all nonzero; one batch, two, three (the result in
+# either array)
+@pytest.mark.parametrize("shape", [(37, 18, 25), (64, 47, 40)])
+@pytest.mark.parametrize("criterion,cap", [(0, 13), (0, 40), (1, 13), (1, 70)])
+def test_fp64_on_chip_sweeps_from_a_given_pc_around_a_body(ib3d, grids, oracle_mod, shape, criterion, cap):
+    x, y, z = (grids.tanh_axis(n) for n in shape)
+    nodes, tris = grids.icosphere(2, 0.3)
+    b = _rhs(shape)
+    pc0 = np.asfortranarray(np.random.default_rng(9).standard_normal(b.shape))
+    p = ib3d.default_params(re=100.0, deltat=1.0, omega=1.7, eps=1e-30, max_sweeps=cap)
+    p.criterion, p.warm_start = criterion, ib3d.WARM_PREV
+    with ib3d.Solver(x, y, z, p) as s:
+        s.set_mesh(nodes + 0.5, tris)
+        counts = s.search([1, s.nx + 2, 1, s.ny + 2, 1, s.nz + 2])
+        assert counts["solid"] > 0 and counts["ib"] > 0
+        cell = s.get_search()["cell"]
+        s.set_field("b", b)
+        s.set_field("pc", pc0)
+        g, got = s.redblack_sor(allow_noconv=True), s.get_field("pc")
+        s.set_params(precision=ib3d.PREC_FP64_FAST)
+        s.set_field("pc", pc0)
+        f, fast = s.redblack_sor(allow_noconv=True), s.get_field("pc")
+    o = oracle_mod.Oracle(x, y, z, 100.0, 1.0)
+    want, update, residual = _sweeps_by_hand([np.asarray(o.acoef(q)) for q in range(3)], b, pc0,
+                                             cell[1:-1, 1:-1, 1:-1] == 0, 1.7, cap)
+    assert (g["sweeps"], g["final_err"]) == (cap, residual if criterion else update)
+    assert np.array_equal(got, want)
+    # the contracted form: the same cells, within rounding amplified by the sweeps
+    assert f["sweeps"] == cap and np.array_equal(fast[cell != 0], pc0[cell != 0])
+    assert np.max(np.abs(fast - want)) <= 1e-13 * cap * np.max(np.abs(want))
