@@ -212,6 +212,7 @@ struct ib3d_ctx {
   size_t xch_words = 0;
   unsigned xch_seq = 0;
   int polls = ib3d::kPollLimit;
+  unsigned poll_skew = 0;   // a test sets it, so that waits run out
   unsigned char* cell = nullptr;
   int* ibmap = nullptr;
   ib3d::SolveCtl* ctl = nullptr;

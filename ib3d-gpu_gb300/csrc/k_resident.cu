@@ -261,10 +261,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident32(Resident32 A) {
 #pragma unroll
         for (int n = 0; n < NH; ++n) pend |= hdst[n] >= 0 ? 1u << n : 0u;
         for (int it = 0; pend != 0; ++it) {
-          if (it >= A.polls || ((it & 255) == 255 && ld_flag(A.err) != 0)) {
-            fail = true;
-            break;
-          }
           u64 v[NH][4];
 #pragma unroll
           for (int n = 0; n < NH; ++n)
@@ -275,14 +271,18 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident32(Resident32 A) {
 #pragma unroll
           for (int n = 0; n < NH; ++n)
             if (pend >> n & 1) {
-              if ((unsigned)(v[n][0] >> 32) == seq && (unsigned)(v[n][1] >> 32) == seq &&
-                  (unsigned)(v[n][2] >> 32) == seq && (unsigned)(v[n][3] >> 32) == seq) {
+              if ((unsigned)(v[n][0] >> 32) == seq + A.skew && (unsigned)(v[n][1] >> 32) == seq + A.skew &&
+                  (unsigned)(v[n][2] >> 32) == seq + A.skew && (unsigned)(v[n][3] >> 32) == seq + A.skew) {
                 *reinterpret_cast<float4*>(E + c * all + hdst[n]) =
                     make_float4(__uint_as_float((unsigned)v[n][0]), __uint_as_float((unsigned)v[n][1]),
                                 __uint_as_float((unsigned)v[n][2]), __uint_as_float((unsigned)v[n][3]));
                 pend &= ~(1u << n);
               }
             }
+          if (pend != 0 && (it & 255) == 255 && (it > A.polls || ld_flag(A.err) != 0)) {
+            fail = true;
+            break;
+          }
         }
       }
       if (__syncthreads_or(fail)) {
@@ -456,20 +456,20 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_resident64(Resident64 A) {
 #pragma unroll
       for (int n = 0; n < kHalo; ++n) pend |= hdst[n] >= 0 ? 1u << n : 0u;
       for (int it = 0; pend != 0; ++it) {
-        if (it >= A.polls || ((it & 255) == 255 && ld_flag(A.err) != 0)) {
-          fail = true;
-          break;
-        }
         u64 v[kHalo][2];
 #pragma unroll
         for (int n = 0; n < kHalo; ++n)
           if (pend >> n & 1) ld_pair(hsrc[n] + c * cstride, v[n][0], v[n][1]);
 #pragma unroll
         for (int n = 0; n < kHalo; ++n)
-          if ((pend >> n & 1) && (unsigned)(v[n][0] >> 32) == seq && (unsigned)(v[n][1] >> 32) == seq) {
+          if ((pend >> n & 1) && (unsigned)(v[n][0] >> 32) == seq + A.skew && (unsigned)(v[n][1] >> 32) == seq + A.skew) {
             Ec[hdst[n]] = __longlong_as_double((long long)((v[n][1] << 32) | (v[n][0] & 0xffffffffull)));
             pend &= ~(1u << n);
           }
+        if (pend != 0 && (it & 255) == 255 && (it > A.polls || ld_flag(A.err) != 0)) {
+          fail = true;
+          break;
+        }
       }
       if (__syncthreads_or(fail)) {
         if (t == 0) atomicExch(A.err, 1);
@@ -693,6 +693,7 @@ bool run_resident32(ib3d_ctx* c, int n, int nsmooth, int nramp, double wi, float
   a.om1 = om1;
   a.err = &c->ctl->stage_err;
   a.polls = c->polls;
+  a.skew = c->poll_skew;
   if (launch_resident32(c->res32, a, c->st) != cudaSuccess) {
     cudaGetLastError();
     c->res32.ok = false;
@@ -756,6 +757,7 @@ bool run_resident64(ib3d_ctx* c, ib3d_solve_stats* st, bool exact, int& rc) {
   a.errs = c->d_errs;
   a.err = reinterpret_cast<int*>(c->d_errs + kBatch);
   a.polls = c->polls;
+  a.skew = c->poll_skew;
   rc = IB3D_ERR_CUDA;
   auto failed = [&](const char* what) {
     c->err = what;

@@ -23,7 +23,8 @@ struct Resident32 {
   double wi;
   float om, om1;
   int* err;                             // set when a wait gave up
-  int polls;                            // loads after which a wait gives up
+  int polls;                            // loads after which a wait gives up, checked every 256
+  unsigned skew;                        // added to the numbers waited for: 0, or no wait ends
 };
 cudaError_t launch_resident32(const ResidentPlan& pl, Resident32 a, cudaStream_t st);
 
@@ -45,6 +46,7 @@ struct Resident64 {
   unsigned long long* errs;             // [nsweeps] largest update or residual (bit pattern)
   int* err;                             // as in Resident32
   int polls;
+  unsigned skew;
 };
 cudaError_t launch_resident64(const ResidentPlan& pl, Resident64 a, bool exact, cudaStream_t st);
 

@@ -190,23 +190,26 @@ def test_fp64_on_chip_residuals_are_of_one_state(ib3d, grids, oracle_mod, shape,
 
 @pytest.fixture(scope="module")
 def set_polls(ib3d, tmp_path_factory):
-    """Sets the loads after which a context's waits for neighbouring rows give up."""
+    """Sets the loads after which a context's waits for neighbouring rows give up, and what is added
+    to the numbers that they wait for."""
     import ctypes as C
     import pathlib
     import subprocess
     from ib3d_gpu_gb300 import buildlib
     d = tmp_path_factory.mktemp("polls")
     (d / "polls.cpp").write_text('#include "ib3d_internal.cuh"\n'
-                                 'extern "C" int set_polls(ib3d_ctx* c, int n) { const int o = c->polls; c->polls = n; return o; }\n')
+                                 'extern "C" int set_polls(ib3d_ctx* c, int n, unsigned skew) {\n'
+                                 '  const int o = c->polls;\n  c->polls = n;\n  c->poll_skew = skew;\n  return o;\n}\n')
     include = pathlib.Path(buildlib.nvcc()).resolve().parent.parent / "include"
     subprocess.run(["g++", "-shared", "-fPIC", "-std=c++17", "-I", str(include), "-I", str(buildlib.CSRC), "-o",
                     str(d / "polls.so"), str(d / "polls.cpp")], check=True)
     f = C.CDLL(str(d / "polls.so")).set_polls
-    f.argtypes, f.restype = [C.c_void_p, C.c_int], C.c_int
+    f.argtypes, f.restype = [C.c_void_p, C.c_int, C.c_uint], C.c_int
     return f
 
 
-# blocks split both ways; the error is reported, and the next solve on the same exchange buffer
+# blocks split both ways; the words waited for carry numbers that are 2^31 passes away, so every
+# wait runs out at its limit of 256 polls. The error is reported, and the next solve on the same exchange buffer
 # has the bits of a solve that never failed
 @pytest.mark.parametrize("precision", [0, 1, 2])
 @pytest.mark.parametrize("criterion", [0, 1])
@@ -218,12 +221,12 @@ def test_wait_that_gives_up_ends_the_solve_with_an_error(ib3d, grids, set_polls,
     with ib3d.Solver(x, y, z, p) as s:
         s.set_field("b", _rhs(shape))
         want = s.redblack_sor(), s.get_field("pc")
-        usual = set_polls(s._h, 0)
+        usual = set_polls(s._h, 0, 1 << 31)
         for _ in range(2):
             with pytest.raises(ib3d.IB3DError) as e:
                 s.redblack_sor()
             assert e.value.code == ib3d.ERR_CUDA and "gave up" in str(e.value)
-        set_polls(s._h, usual)
+        set_polls(s._h, usual, 0)
         got = s.redblack_sor(), s.get_field("pc")
     assert (got[0]["sweeps"], got[0]["final_err"]) == (want[0]["sweeps"], want[0]["final_err"])
     assert np.array_equal(got[1], want[1])
