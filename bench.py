@@ -61,11 +61,11 @@ BYTES_SOR32_SWEEP = 13.0
 BYTES_SOR64_SWEEP = 25.0
 # DRAM bytes (read + written) per grid cell and sweep of the FP32 sweep kernel
 # (k_sor32p2) at 256x192x192, from one ncu capture of four launches inside the sweep
-# loop (warm: caches as the previous launch left them; 9,702,144 B in all) and of two
-# launches after a cache flush (cold; 60,701,696 B each on average). Other workloads
+# loop (warm: caches as the previous launch left them; 12,405,504 B in all) and of two
+# launches after a cache flush (cold; 60,693,760 B each on average). Other workloads
 # scale them by their cell count.
-DRAM_BYTES_PER_CELL_SWEEP32 = 2 * 9702144.0 / 4 / 9437184.0
-DRAM_BYTES_PER_CELL_SWEEP32_COLD = 2 * 60701696.0 / 9437184.0
+DRAM_BYTES_PER_CELL_SWEEP32 = 2 * 12405504.0 / 4 / 9437184.0
+DRAM_BYTES_PER_CELL_SWEEP32_COLD = 2 * 60693760.0 / 9437184.0
 
 
 def package():

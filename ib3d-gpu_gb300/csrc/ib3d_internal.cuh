@@ -474,7 +474,7 @@ __device__ __forceinline__ void finish_block(SolveCtl* ctl, unsigned long long* 
 // The FP32 SOR update shared by every FP32 sweep kernel: e <- (1-omega) e +
 // omega num / diag, the quotient as a product with the hardware's approximate
 // reciprocal (rcp.approx.ftz.f32, one instruction) instead of the IEEE division's
-// sequence. diag is the sum of three positive Poisson diagonal entries, a normal
+// sequence. diag is the sum of three Poisson diagonal entries of one sign, a normal
 // number far from the range limits, so the reciprocal needs no range handling. The
 // FP32 sweeps only precondition the FP64 defect correction, whose FP64 residual
 // decides convergence, so the quotient's last-bit rounding does not reach the result.

@@ -82,8 +82,9 @@ typedef struct ib3d_params {
   int32_t warm_start;   /* IB3D_WARM_* */
   int32_t check_every;  /* sweeps between residual checks (IB3D_CRIT_RESIDUAL); >= 1 */
   int32_t inner_sweeps; /* FP32 sweeps per defect-correction pass (IB3D_PREC_FP32DC) */
-  int32_t sweep_kernel; /* FP32 sweep kernel: 0 colour-packed arrays, one launch per colour pass,
-                           two rows per thread; 1 the padded field layout; 2 colour-packed arrays, the red and black
+  int32_t sweep_kernel; /* FP32 sweep kernel: 0 colour-packed arrays, a whole pass of sweeps in one
+                           launch where the grid fits on chip, else one launch per colour pass
+                           (or per part of it, beyond L2), two rows per thread; 1 the padded field layout; 2 colour-packed arrays, the red and black
                            passes fused into one z-wavefront launch per sweep (even nx <= 512); 3
                            and 4 colour-packed arrays, one row per thread, the loads without (3)
                            or behind (4) branches. All give the same results. */

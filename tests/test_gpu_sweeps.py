@@ -27,7 +27,7 @@ def _capped(ib3d, grids, shape, sweeps, b, **kw):
 # sizes whose sweeps run on chip (blocks split both ways, along one axis, with several planes
 # a thread) and beyond; odd nx (the second colour's rows end in the ghost cell), odd ny (a row pair's second row is
 # the ghost row), nz no multiple of a slab; the last two exceed what the blocks hold on chip,
-# and the last one streams its right-hand side and alternates the direction of its passes
+# and the last one L2, where the sweeps go through parts
 @pytest.mark.parametrize("kernel,shape", [(0, (129, 21, 19)), (0, (37, 18, 45)), (0, (5, 4, 4)), (0, (7, 5, 301)),
                                           (0, (9, 203, 6)), (0, (126, 130, 97)), (3, (129, 21, 19)),
                                           (4, (67, 9, 11)), (0, (1201, 41, 78)), (0, (271, 225, 202))])
@@ -57,7 +57,7 @@ def _rhs(shape, seed=5):
 
 # blocks of two rows, of several, split along one axis only; odd extents; the test met inside a
 # batch (of 16, 32, ... sweeps), at its end, and not at all; residuals checked at every sweep
-# and between; a start from a given pc whose ghost and boundary values count
+# and between; a given pc, which the zero start replaces
 @pytest.mark.parametrize("shape,criterion,every,eps,cap", [
     ((21, 9, 8), 0, 1, 1e-7, 100000), ((37, 18, 25), 1, 3, 1e-6, 100000), ((8, 41, 5), 1, 1, 1e-6, 100000),
     ((7, 5, 61), 0, 1, 1e-30, 77), ((16, 12, 12), 1, 8, 1e-30, 48), ((16, 12, 12), 1, 5, 1e-30, 33),
@@ -138,8 +138,8 @@ def test_noalloc_solve_meets_the_residual(ib3d, grids, oracle_mod, shape):
     assert np.all(q[cell != 0] == 0.0)
 
 
-# launch-per-pass sweeps: whole tiles (256 x 192 x 192; streamed: 512 x 128 x 304), odd ny and nz
-# (the march starts or ends on the ghost plane, up and down), enough passes in a row
+# launch-per-pass sweeps: whole tiles (256 x 192 x 192; in parts: 512 x 128 x 304), odd ny and nz
+# (the march ends on the ghost plane), enough passes in a row
 # that a value left over from an earlier pass would show
 @pytest.mark.parametrize("shape", [(256, 192, 192), (256, 193, 193), (250, 191, 191), (512, 128, 304), (271, 225, 201)])
 def test_passes_read_the_last_pass_only(ib3d, grids, shape):
